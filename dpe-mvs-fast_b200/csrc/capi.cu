@@ -338,17 +338,24 @@ void set_carveout(const void *func, int percent) {
 }
 dim3 shape_grid(int W, int H, dim3 b) { return dim3((W + b.x - 1) / b.x, (H + b.y - 1) / b.y); }
 
-void launch_strong_update(int staging, bool gn, dim3 grid, size_t smem, cudaStream_t s, const Launch args, int it,
-                          int parity, int carveout) {
+// Dynamic shared bytes above the 48 KB that need no opt-in (many sources).
+template <class K> cudaError_t allow_smem(K *kernel, size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+cudaError_t launch_strong_update(int staging, bool gn, dim3 grid, size_t smem, cudaStream_t s, const Launch args, int it,
+                                 int parity, int carveout) {
+  cudaError_t attr = cudaSuccess;
   with_stage(staging, [&](auto st) {
-    if (gn) {
-      set_carveout((const void *)k_strong_update<decltype(st)::value, true>, carveout);
-      k_strong_update<decltype(st)::value, true><<<grid, kCoopThreads, smem, s>>>(args, it, parity);
-    } else {
-      set_carveout((const void *)k_strong_update<decltype(st)::value, false>, carveout);
-      k_strong_update<decltype(st)::value, false><<<grid, kCoopThreads, smem, s>>>(args, it, parity);
-    }
+    auto go = [&](auto *kernel) {
+      if ((attr = allow_smem(kernel, smem)) != cudaSuccess) return;
+      set_carveout((const void *)kernel, carveout);
+      kernel<<<grid, kCoopThreads, smem, s>>>(args, it, parity);
+    };
+    if (gn) go(k_strong_update<decltype(st)::value, true>);
+    else go(k_strong_update<decltype(st)::value, false>);
   });
+  return attr;
 }
 
 // WEAK pixels of one red/black colour, (x + y) & 1 == parity.
@@ -519,7 +526,7 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
     PM_LAUNCHED("k_pad_image", s);
   }
   // FP32 staging: when every source texel is exact in BF16 (8-bit images, the finest pyramid
-  // level), the cost kernels sample BF16 pairs instead: the same values, half the gather bytes.
+  // level), the cost kernels sample BF16 quads instead: the same values, one load per tap.
   int staging = ctx->opt.staging;
   if (staging == DPE_STAGE_FP32 && N > 1) {
     unsigned *flag = get((unsigned *)0, "bf16_flag", 1);
@@ -536,16 +543,18 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
   }
   ps->staging = staging;
   a.stage = staging;
-  uint32_t *img_pairs = staging != DPE_STAGE_FP32 ? get((uint32_t *)0, "img_pairs", PL * N) : nullptr;
-  if (staging != DPE_STAGE_FP32 && !img_pairs) return DPE_ERR_OUT_OF_MEMORY;
+  uint2 *img_quads = staging != DPE_STAGE_FP32 ? get((uint2 *)0, "img_quads", PL * N) : nullptr;
+  if (staging != DPE_STAGE_FP32 && !img_quads) return DPE_ERR_OUT_OF_MEMORY;
   for (int i = 1; i < N; ++i) {
     if (staging != DPE_STAGE_FP32) {
-      a.pair[i] = img_pairs + PL * i;
+      uint2 *quads = img_quads + PL * i;
+      const unsigned blocks = (unsigned)((PL + 255) / 256);
+      a.quad[i] = quads;
       if (staging == DPE_STAGE_BF16)
-        k_stage_pairs<true><<<(unsigned)((PL + 255) / 256), 256, 0, s>>>(img_pad + PL * i, img_pairs + PL * i, (long long)PL);
+        k_stage_quads<true><<<blocks, 256, 0, s>>>(img_pad + PL * i, quads, (long long)PL, W + 2);
       else
-        k_stage_pairs<false><<<(unsigned)((PL + 255) / 256), 256, 0, s>>>(img_pad + PL * i, img_pairs + PL * i, (long long)PL);
-      PM_LAUNCHED("k_stage_pairs", s);
+        k_stage_quads<false><<<blocks, 256, 0, s>>>(img_pad + PL * i, quads, (long long)PL, W + 2);
+      PM_LAUNCHED("k_stage_quads", s);
     }
   }
   return DPE_OK;
@@ -568,7 +577,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   cudaStream_t s = ctx->stream;
   Arena &A = ctx->arena;
   const dpe_params &P = ps[0].a.P;
-  // one staging for the sequence: BF16 pairs only when every problem has them
+  // one staging for the sequence: BF16 quads only when every problem has them
   int staging = ps[0].staging;
   for (int b = 1; b < n; ++b)
     if (ps[b].staging != staging) staging = ctx->opt.staging;
@@ -659,9 +668,11 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
           DPE_TRY(cudaMemcpyAsync(a.plane_snap, a.plane, ps[b].L * sizeof(float4), cudaMemcpyDeviceToDevice, s));
           DPE_TRY(cudaMemcpyAsync(a.cost_snap, a.cost, ps[b].L * 4, cudaMemcpyDeviceToDevice, s));
         }
+      cudaError_t attr = cudaSuccess;
       DPE_TIMED(ctx, KID_STRONG_UPDATE, s, carved(KID_STRONG_UPDATE, [&](int cv) {
-                  launch_strong_update(staging, gn, g.cg, g.coop_smem, s, g.coop, it, parity, cv);
+                  attr = launch_strong_update(staging, gn, g.cg, g.coop_smem, s, g.coop, it, parity, cv);
                 }));
+      DPE_TRY(attr);
       PM_LAUNCHED("k_strong_update", s);
     }
     DPE_TIMED(ctx, KID_RANSAC, s,
@@ -697,9 +708,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   {
     cudaError_t attr = cudaSuccess;
     with_stage(staging, [&](auto st) {
-      if (g.lr_smem > 48 * 1024)
-        attr = cudaFuncSetAttribute(k_local_refine<decltype(st)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)g.lr_smem);
+      attr = allow_smem(k_local_refine<decltype(st)::value>, g.lr_smem);
     });
     DPE_TRY(attr);
   }

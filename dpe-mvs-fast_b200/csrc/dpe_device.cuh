@@ -22,38 +22,19 @@ constexpr int kMaxSrc = DPE_MAX_IMAGES - 1;
 constexpr int kNeighbours = DPE_NEIGHBOUR_NUM;
 constexpr int kMaxWin = 6;  // taps per window side for radius 5 / step 2 (DPE.cu:728-737)
 // Minimum resident blocks per multiprocessor requested for the strong-window cost kernels
-// (__launch_bounds__): bounds their registers, trading spills against occupancy.  Measured on
-// the 10-view 1600x1200 schedule: the cooperative strong update runs fastest at 8 blocks of 128
-// (64 registers; 2 % faster than 6 blocks at 80), the sweep kernels unconstrained.
+// (__launch_bounds__): bounds their registers, trading spills against occupancy.  Measured on a
+// 1600x1200 view, first call with 10 sources / geometric call with 9 (ms): strong update at 8 blocks
+// 77.9 / 74.2, at 6 64.8 / 61.2, at 5 (96 registers, no spills) 62.7 / 62.1, at 4 59.1 / 61.8, the
+// latter slower at 160x120 (0.59 against 0.52); DepthToWeak at 8, 6 and 5 blocks 50.7, 49.7 and 51.1.
 #ifndef DPE_COST_MIN_BLOCKS
 #define DPE_COST_MIN_BLOCKS 1
 #endif
 #ifndef DPE_STRONG_MIN_BLOCKS
-#define DPE_STRONG_MIN_BLOCKS 8
+#define DPE_STRONG_MIN_BLOCKS 5
 #endif
-// the same bound for the cooperative DepthToWeak sweep (measured: 8 blocks, 64 registers, 4 %
-// faster than unbounded; the cooperative LocalRefine, with its larger shared-memory block, runs
-// fastest unbounded and uses DPE_COST_MIN_BLOCKS)
 #ifndef DPE_SWEEP_MIN_BLOCKS
-#define DPE_SWEEP_MIN_BLOCKS 8
+#define DPE_SWEEP_MIN_BLOCKS 6
 #endif
-// Unrolling of a window column's taps (the reference window, radius 5 / step 2, has 6 per column)
-// in the kernels that sweep one plane family over all sources (DepthToWeak, LocalRefine, the
-// random initialisation).  Measured on the 10-view 1600x1200 schedule with the packed tap
-// arithmetic: the whole column (6) makes DepthToWeak 6 % and LocalRefine 7 % faster than 3, and 2
-// is slower than 3.
-#ifndef DPE_SWEEP_UNROLL
-#define DPE_SWEEP_UNROLL 6
-#endif
-constexpr int kSweepUnroll = DPE_SWEEP_UNROLL;
-// taps of a window column unrolled in the strong update's cost evaluations (0: rolled loop).
-// Measured on the 10-view 1600x1200 schedule with the packed tap arithmetic: unrolling by 2 makes
-// the cooperative strong update 5 % faster (the next tap's gathers issue before this tap's blend);
-// by 3 or 6 it was 35-40 % slower with the scalar taps (registers, under the 8-block bound).
-#ifndef DPE_STRONG_UNROLL
-#define DPE_STRONG_UNROLL 2
-#endif
-constexpr int kStrongUnroll = DPE_STRONG_UNROLL;
 
 // All per-call read-only data (cameras, relative poses, params, buffer pointers).  It lives in a
 // small device buffer written once per call; kernels receive its address.
@@ -64,12 +45,14 @@ struct PMArgs {
   // Plane-independent parts of each source's homography H = A - b m^T / w (homography_base):
   // composed in double (window centres are projected in double), and the same rounded to float.
   double dA[kMaxImages][9], db[kMaxImages][3], dm[4];
+  double dsize[kMaxImages][2];  // each source camera's (width, height)
   float hA[kMaxImages][9], hb[kMaxImages][3], hm[4];
   uint32_t key[2];
   const float *img[kMaxImages];  // padded (W+2)*(H+2) float images
-  // Staged source images (dpe_options::staging FP16 / BF16): pair[s][o] holds the padded texels
-  // P[o] and P[o+1] as two 16-bit values in one 32-bit word, so a bilinear footprint is two loads.
-  const uint32_t *pair[kMaxImages];
+  // Staged source images (dpe_options::staging FP16 / BF16): quad[s][o] holds the footprint of padded
+  // offset o, the texels P[o], P[o+1], P[o+pw], P[o+pw+1], as four 16-bit values, so a bilinear
+  // footprint is one 8-byte load.
+  const uint2 *quad[kMaxImages];
   int stage;  // DPE_STAGE_*: storage the cost kernels sample the source images from
   int gn;     // 1: Gauss-Newton plane hypothesis in the strong update (dpe_options::gn_refine)
   const float *dep[kMaxImages];  // W*H depth maps (geom consistency)
@@ -155,6 +138,8 @@ inline void homography_base(const dpe_camera &rc, const dpe_camera &sc, double A
 inline void set_homography_bases(PMArgs &a) {
   for (int s = 1; s < a.N; ++s) {
     homography_base(a.cam[0], a.cam[s], a.dA[s], a.db[s], a.dm);
+    a.dsize[s][0] = a.cam[s].width;
+    a.dsize[s][1] = a.cam[s].height;
     for (int k = 0; k < 9; ++k) a.hA[s][k] = (float)a.dA[s][k];
     for (int k = 0; k < 3; ++k) a.hb[s][k] = (float)a.db[s][k];
   }
@@ -279,6 +264,20 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return make_float2(a.x * b.x, a.y * b.y);
 #endif
 }
+// Sum of two packed products with both roundings kept: p * 1 + q, the 1 read from constant memory so
+// that the compiler can neither fold the multiply away nor fuse a product into the sum.  One FFMA2
+// with the result of two scalar adds (p * 1 is exact).
+#ifdef __CUDACC__
+static __device__ __constant__ float2 c_one2 = {1.0f, 1.0f};
+#endif
+__device__ __forceinline__ float2 addp2(float2 p, float2 q) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  return __ffma2_rn(p, c_one2, q);
+#else
+  return make_float2(p.x + q.x, p.y + q.y);
+#endif
+}
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 // floor_split of both coordinates of a pair.
 __device__ __forceinline__ float2 floor_split2(float2 v, int *ix, int *iy) {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
@@ -320,37 +319,45 @@ struct SrcF32 {
                        img_ld(p, o + pw + 1, n, 105));
   }
 };
-__device__ __forceinline__ uint32_t pair_ld(const uint32_t *p, long long off, long long n, int tag) {
+__device__ __forceinline__ uint2 quad_ld(const uint2 *p, long long off, long long n, int tag) {
 #ifdef DPE_CHECKED
   return *dpe_chk(p, off, n, tag);
 #else
   return __ldg(p + off);
 #endif
 }
-// FP16 pairs: low half P[o], high half P[o+1].
+// FP16 quads: the footprint's upper row in x, its lower row in y, left texels in the low halves.
 struct SrcF16 {
-  const uint32_t *p;
+  const uint2 *p;
   int pw;
   long long n;
   __device__ __forceinline__ float4 fetch(int o) const {
-    const uint32_t t = pair_ld(p, o, n, 108), b = pair_ld(p, o + pw, n, 109);
-    return make_float4(__half2float(__ushort_as_half((unsigned short)(t & 0xFFFFu))),
-                       __half2float(__ushort_as_half((unsigned short)(t >> 16))),
-                       __half2float(__ushort_as_half((unsigned short)(b & 0xFFFFu))),
-                       __half2float(__ushort_as_half((unsigned short)(b >> 16))));
+    const uint2 t = quad_ld(p, (unsigned)o, n, 108);
+    return make_float4(__half2float(__ushort_as_half((unsigned short)(t.x & 0xFFFFu))),
+                       __half2float(__ushort_as_half((unsigned short)(t.x >> 16))),
+                       __half2float(__ushort_as_half((unsigned short)(t.y & 0xFFFFu))),
+                       __half2float(__ushort_as_half((unsigned short)(t.y >> 16))));
   }
 };
-// BF16 pairs: a bfloat16 is the top half of an FP32 word, so widening is a shift.
+// BF16 quads: a bfloat16 is the top half of an FP32 word, so widening is a shift.
 struct SrcBF16 {
-  const uint32_t *p;
+  const uint2 *p;
   int pw;
   long long n;
   __device__ __forceinline__ float4 fetch(int o) const {
-    const uint32_t t = pair_ld(p, o, n, 110), b = pair_ld(p, o + pw, n, 111);
-    return make_float4(__uint_as_float(t << 16), __uint_as_float(t & 0xFFFF0000u), __uint_as_float(b << 16),
-                       __uint_as_float(b & 0xFFFF0000u));
+    const uint2 t = quad_ld(p, (unsigned)o, n, 110);
+    return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16),
+                       __uint_as_float(t.y & 0xFFFF0000u));
   }
 };
+// The footprints of two taps as pairs: v00 holds both taps' upper left texels, and so on.
+struct Foot2 {
+  float2 v00, v10, v01, v11;
+};
+template <class Src> __device__ __forceinline__ Foot2 fetch2(const Src &src, int o0, int o1) {
+  const float4 a = src.fetch(o0), b = src.fetch(o1);
+  return Foot2{make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), make_float2(a.w, b.w)};
+}
 // kClamp = false: the caller knows -1 <= x <= W-1 and -1 <= y <= H-1, where the clamp is the
 // identity.
 template <class Src, bool kClamp = true>
@@ -373,10 +380,10 @@ __device__ __forceinline__ SrcF32 src_f32(const PMArgs &a, int s) {
   return SrcF32{a.img[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
 }
 __device__ __forceinline__ SrcF16 src_f16(const PMArgs &a, int s) {
-  return SrcF16{a.pair[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
+  return SrcF16{a.quad[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
 }
 __device__ __forceinline__ SrcBF16 src_bf16(const PMArgs &a, int s) {
-  return SrcBF16{a.pair[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
+  return SrcBF16{a.quad[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
 }
 // The sampler of a staging (DPE_STAGE_*), chosen at compile time: each cost kernel is built once
 // per staging, so a kernel carries only its own tap loop.
@@ -521,25 +528,37 @@ __device__ __forceinline__ float bilateral_weight(float dx, float dy, float pix,
 // local memory, which L1 serves well here.  (A block-shared copy measured slower: 36 KB of static
 // shared memory per block cuts the resident blocks and the L1 left for the image gathers.)
 constexpr int kWinTaps = kMaxWin * kMaxWin;
+// Taps are stored in pairs, (w0, w1, w0 (r0 - c), w1 (r1 - c)): one 16-byte load gives two taps in the
+// form the packed arithmetic takes.
+constexpr int kWinPairs = (kWinTaps + 1) / 2;
+__device__ __forceinline__ void win_store(float4 *t, int k, float w, float wr) {
+  float *f = reinterpret_cast<float *>(&G(t, k >> 1, kWinPairs, 320)) + (k & 1);
+  f[0] = w;
+  f[2] = wr;
+}
+__device__ __forceinline__ float2 win_tap(const float4 *t, int k) {
+  const float *f = reinterpret_cast<const float *>(&G(t, k >> 1, kWinPairs, 322)) + (k & 1);
+  return make_float2(f[0], f[2]);
+}
 struct RefWindow {
-  float2 t_[kWinTaps];  // per tap (w, w * (r - c)): one 8-byte load per tap
+  float4 t_[kWinPairs];
   float center, inv_wsum, mean_r, var_r;
   unsigned long long *cnt;  // this kernel's strong-evaluation counter (counting runs only)
-  __device__ __forceinline__ float2 tap(int k) const { return G(t_, k, kWinTaps, 322); }
+  __device__ __forceinline__ float2 tap(int k) const { return win_tap(t_, k); }
+  __device__ __forceinline__ float4 tap2(int p) const { return G(t_, p, kWinPairs, 323); }
   __device__ __forceinline__ float w(int k) const { return tap(k).x; }
-  __device__ __forceinline__ float wr(int k) const { return tap(k).y; }
 };
 #define DPE_REF_WINDOW(rw) ::dpe::RefWindow rw
 // The same window held once per pixel in shared memory, read by every thread that evaluates a
 // hypothesis of that pixel (the cooperative strong update).  The threads of one pixel read the
 // same tap together, so a warp's read is one broadcast per pixel.
 struct SmemWindow {
-  const float2 *t_;
+  const float4 *t_;
   float center, inv_wsum, mean_r, var_r;
   unsigned long long *cnt;
-  __device__ __forceinline__ float2 tap(int k) const { return t_[k]; }
-  __device__ __forceinline__ float w(int k) const { return t_[k].x; }
-  __device__ __forceinline__ float wr(int k) const { return t_[k].y; }
+  __device__ __forceinline__ float2 tap(int k) const { return win_tap(t_, k); }
+  __device__ __forceinline__ float4 tap2(int p) const { return t_[p]; }
+  __device__ __forceinline__ float w(int k) const { return tap(k).x; }
 };
 
 __device__ __forceinline__ void build_ref_window(const PMArgs &a, int px, int py, RefWindow &rw, int kid) {
@@ -553,7 +572,7 @@ __device__ __forceinline__ void build_ref_window(const PMArgs &a, int px, int py
       const float rp = texel(a, 0, px + i, py + j);
       const float w = bilateral_weight((float)i, (float)j, rp, center, a.P.sigma_spatial, a.P.sigma_color);
       const float rc = rp - center;
-      G(rw.t_, k, kWinTaps, 320) = make_float2(w, w * rc);
+      win_store(rw.t_, k, w, w * rc);
       sw += w; swr += w * rc; swrr += w * rc * rc;
       ++k;
     }
@@ -593,45 +612,92 @@ struct WinProj {
   float2 g14;   // the dy coefficients (H01 - uc H21, H11 - vc H21)
   float zc;     // projective depth of the centre
   float h6, h7; // H20, H21
-  float2 lo, hi;  // the texture clamp [-1, W-1] x [-1, H-1] relative to (U0, V0)
 };
-// Fills wp for plane pl at pixel (px, py) of source s; false when the centre does not project
-// inside the source (the cost is then 2, DPE.cu:709-712).
-__device__ __forceinline__ bool window_projection(const PMArgs &a, int s, float4 pl, int px, int py, WinProj &wp) {
-  const double *A = a.dA[s], *b = a.db[s];
-  const double m0 = (double)pl.x * a.dm[0], m1 = (double)pl.y * a.dm[1];
+// The plane's part of the projection, the same for every source: the first two entries of m = Kr^-T n,
+// 1 / w and m . p0 / w.
+struct PlaneProj {
+  double m0, m1, iw, q;
+};
+__device__ __forceinline__ PlaneProj plane_projection(const PMArgs &a, float4 pl, int px, int py) {
+  PlaneProj p;
+  p.m0 = (double)pl.x * a.dm[0];
+  p.m1 = (double)pl.y * a.dm[1];
   const double m2 = (double)pl.x * a.dm[2] + (double)pl.y * a.dm[3] + (double)pl.z;
-  const double iw = 1.0 / (double)pl.w;
+  p.iw = 1.0 / (double)pl.w;
+  p.q = (p.m0 * (double)px + p.m1 * (double)py + m2) * p.iw;
+  return p;
+}
+// The pixel's part of the projection into one source, the same for every plane: A (px, py, 1).
+struct PixelProj {
+  double x, y, z;
+};
+__device__ __forceinline__ PixelProj pixel_projection(const PMArgs &a, int s, int px, int py) {
+  const double *A = a.dA[s];
   const double x = (double)px, y = (double)py;
-  const double q = (m0 * x + m1 * y + m2) * iw;  // m . p0 / w
-  const double X = A[0] * x + A[1] * y + A[2] - b[0] * q;
-  const double Y = A[3] * x + A[4] * y + A[5] - b[1] * q;
-  const double Z = A[6] * x + A[7] * y + A[8] - b[2] * q;
+  return PixelProj{A[0] * x + A[1] * y + A[2], A[3] * x + A[4] * y + A[5], A[6] * x + A[7] * y + A[8]};
+}
+// floor(x) as a double and an int for 0 <= x < 2^31.  On the device one round-down add of 1.5 * 2^52
+// (floor_split's construction): rounds and conversions of doubles run at 16 per clock and SM.
+__device__ __forceinline__ double floor_split(double x, int *ix) {
+#ifdef __CUDA_ARCH__
+  const double f = __dadd_rd(x, 6755399441055744.0);
+  *ix = __double2loint(f);
+  return f - 6755399441055744.0;
+#else
+  const double f = floor(x);
+  *ix = (int)f;
+  return f;
+#endif
+}
+// Fills wp for a plane at a pixel and source s; false when the centre does not project inside the
+// source (the cost is then 2, DPE.cu:709-712).
+__device__ __forceinline__ bool window_projection(const PMArgs &a, int s, const PlaneProj &p, const PixelProj &c,
+                                                  WinProj &wp) {
+  const double *A = a.dA[s], *b = a.db[s];
+  const double X = c.x - b[0] * p.q;
+  const double Y = c.y - b[1] * p.q;
+  const double Z = c.z - b[2] * p.q;
   const double iz = 1.0 / Z;
   const double uc = X * iz, vc = Y * iz;
-  const dpe_camera &sc = a.cam[s];
-  if (!(uc >= 0.0 && uc < (double)sc.width && vc >= 0.0 && vc < (double)sc.height)) return false;
-  const double U = floor(uc), V = floor(vc);
-  wp.U0 = (int)U;
-  wp.V0 = (int)V;
+  const double *size = a.dsize[s];
+  if (!(uc >= 0.0 && uc < size[0] && vc >= 0.0 && vc < size[1])) return false;
+  const double U = floor_split(uc, &wp.U0), V = floor_split(vc, &wp.V0);
   wp.fuv = make_float2((float)(uc - U), (float)(vc - V));
   wp.zc = (float)Z;
-  const double bw0 = b[0] * iw, bw1 = b[1] * iw, bw2 = b[2] * iw;
-  const double h6 = A[6] - bw2 * m0, h7 = A[7] - bw2 * m1;
-  wp.g03 = make_float2((float)((A[0] - bw0 * m0) - uc * h6), (float)((A[3] - bw1 * m0) - vc * h6));
-  wp.g14 = make_float2((float)((A[1] - bw0 * m1) - uc * h7), (float)((A[4] - bw1 * m1) - vc * h7));
+  const double bw0 = b[0] * p.iw, bw1 = b[1] * p.iw, bw2 = b[2] * p.iw;
+  const double h6 = A[6] - bw2 * p.m0, h7 = A[7] - bw2 * p.m1;
+  wp.g03 = make_float2((float)((A[0] - bw0 * p.m0) - uc * h6), (float)((A[3] - bw1 * p.m0) - vc * h6));
+  wp.g14 = make_float2((float)((A[1] - bw0 * p.m1) - uc * h7), (float)((A[4] - bw1 * p.m1) - vc * h7));
   wp.h6 = (float)h6;
   wp.h7 = (float)h7;
-  wp.lo = make_float2((float)(-1 - wp.U0), (float)(-1 - wp.V0));
-  wp.hi = make_float2((float)(a.W - 1 - wp.U0), (float)(a.H - 1 - wp.V0));
   return true;
+}
+__device__ __forceinline__ bool window_projection(const PMArgs &a, int s, float4 pl, int px, int py, WinProj &wp) {
+  return window_projection(a, s, plane_projection(a, pl, px, py), pixel_projection(a, s, px, py), wp);
+}
+// The texture clamp [-1, W-1] x [-1, H-1] relative to (U0, V0).
+struct WinClamp {
+  float2 lo, hi;
+};
+__device__ __forceinline__ WinClamp window_clamp(const PMArgs &a, const WinProj &wp) {
+  return WinClamp{make_float2((float)(-1 - wp.U0), (float)(-1 - wp.V0)),
+                  make_float2((float)(a.W - 1 - wp.U0), (float)(a.H - 1 - wp.V0))};
+}
+// True when no tap (|dx|, |dy| <= r) can reach the clamp: the numerators are bounded by r times the sum
+// of their coefficients' magnitudes and the depth from below by |zc| minus the same for Z, so an offset
+// is at most their quotient; 1 % of slack covers the roundings.  The fraction is in [0, 1].
+__device__ __forceinline__ bool window_inside(const PMArgs &a, const WinProj &wp, float r) {
+  const float den = 0.99f * (fabsf(wp.zc) - r * (fabsf(wp.h6) + fabsf(wp.h7)));
+  const int mx = min(wp.U0, a.W - 2 - wp.U0), my = min(wp.V0, a.H - 2 - wp.V0);
+  return den > 1e-30f && den < 1e30f && r * (fabsf(wp.g03.x) + fabsf(wp.g14.x)) <= den * (float)mx &&
+         r * (fabsf(wp.g03.y) + fabsf(wp.g14.y)) <= den * (float)my;
 }
 // bilinear_s at (U0 + x, V0 + y): the clamp to [-1, W-1] x [-1, H-1] and the split into texel and
 // weight are taken on the offsets, which equals them on the absolute coordinates.  The x and y
 // halves and the two rows of the blend run as packed pairs (the same operations as bilinear_s).
-template <class Src, bool kClamp = true>
-__device__ __forceinline__ float bilinear_w(const Src &src, const WinProj &wp, float2 p) {
-  const float2 c = kClamp ? make_float2(fminf(fmaxf(p.x, wp.lo.x), wp.hi.x), fminf(fmaxf(p.y, wp.lo.y), wp.hi.y)) : p;
+template <class Src>
+__device__ __forceinline__ float bilinear_w(const Src &src, const WinProj &wp, const WinClamp &wc, float2 p) {
+  const float2 c = make_float2(fminf(fmaxf(p.x, wc.lo.x), wc.hi.x), fminf(fmaxf(p.y, wc.lo.y), wc.hi.y));
   int ix, iy;
   const float2 f = floor_split2(c, &ix, &iy);
   const float2 a = sub2(c, f);                            // (ax, ay)
@@ -646,71 +712,133 @@ __device__ __forceinline__ float bilinear_w(const Src &src, const WinProj &wp, f
 // One tap of the strong window: sample the source at the projected tap and accumulate the
 // hypothesis-dependent moments (sums of w*s, w*s^2, w*(r-c)*s over s = sample - c); acc holds
 // (sum w*s, sum w*(r-c)*s).  cxy and cz carry the tap column's dx terms.
-template <bool kClamp, class Src, class RW>
-__device__ __forceinline__ void strong_tap(const WinProj &wp, const Src &src, const RW &rw, float2 cxy, float cz,
-                                           float dy, int k, float2 &acc, float &s_ss) {
+template <class Src, class RW>
+__device__ __forceinline__ void strong_tap(const WinProj &wp, const WinClamp &wc, const Src &src, const RW &rw,
+                                           float2 cxy, float cz, float dy, int k, float2 &acc, float &s_ss) {
   const float2 gy = mul2(wp.g14, make_float2(dy, dy));
   const float Z = wp.h7 * dy + cz;
   const float iz = tap_rcp(Z);
   const float2 t = mul2(make_float2(gy.x + cxy.x, gy.y + cxy.y), make_float2(iz, iz));  // (X, Y) / Z
-  const float sv = bilinear_w<Src, kClamp>(src, wp, make_float2(wp.fuv.x + t.x, wp.fuv.y + t.y)) - rw.center;
+  const float sv = bilinear_w<Src>(src, wp, wc, make_float2(wp.fuv.x + t.x, wp.fuv.y + t.y)) - rw.center;
   const float2 m = mul2(rw.tap(k), make_float2(sv, sv));  // (w s, w (r - c) s)
   const float q = m.x * sv;
   acc.x += m.x;
   acc.y += m.y;
   s_ss += q;
 }
+#ifdef __CUDA_ARCH__
+// Two taps of a window column at once, rows dy0 and dy1: strong_tap's operations on both, each
+// result the same bits, every sum in the same order.  gx, gy, gz: the taps' dy terms (g14.x dy, g14.y
+// dy, h7 dy); cx, cy, cz: the column's dx terms; p: the taps' pair in the reference window.
+template <bool kClamp, class Src, class RW>
+__device__ __forceinline__ void strong_tap2(const WinProj &wp, const WinClamp &wc, const Src &src, const RW &rw, float2 gx, float2 gy,
+                                            float2 gz, float cx, float cy, float cz, unsigned base, int p, float &s_s,
+                                            float &s_ss, float &s_rs) {
+  const float2 X = addp2(gx, dup2(cx)), Y = addp2(gy, dup2(cy)), Z = addp2(gz, dup2(cz));
+  const float2 iz = make_float2(tap_rcp(Z.x), tap_rcp(Z.y));
+  float2 u = addp2(mul2(X, iz), dup2(wp.fuv.x)), v = addp2(mul2(Y, iz), dup2(wp.fuv.y));
+  if (kClamp) {
+    u = make_float2(fminf(fmaxf(u.x, wc.lo.x), wc.hi.x), fminf(fmaxf(u.y, wc.lo.x), wc.hi.x));
+    v = make_float2(fminf(fmaxf(v.x, wc.lo.y), wc.hi.y), fminf(fmaxf(v.y, wc.lo.y), wc.hi.y));
+  }
+  const float2 bias = dup2(12582912.0f);
+  const float2 fu = __fadd2_rd(u, bias), fv = __fadd2_rd(v, bias);  // 1.5 * 2^23 + floor (floor_split)
+  const float2 au = sub2(u, sub2(fu, bias)), av = sub2(v, sub2(fv, bias));
+  const float2 ou = sub2(dup2(1.0f), au), ov = sub2(dup2(1.0f), av);
+  // the texel index straight from the biased floors: base holds the window's origin minus the biases
+  const unsigned pw = (unsigned)src.pw;
+  const Foot2 t = fetch2(src, (int)(__float_as_uint(fv.x) * pw + __float_as_uint(fu.x) + base),
+                         (int)(__float_as_uint(fv.y) * pw + __float_as_uint(fu.y) + base));
+  const float2 top = addp2(mul2(ou, t.v00), mul2(au, t.v10)), bot = addp2(mul2(ou, t.v01), mul2(au, t.v11));
+  const float2 sv = sub2(addp2(mul2(ov, top), mul2(av, bot)), dup2(rw.center));
+  const float4 w = rw.tap2(p);
+  const float2 ws = mul2(make_float2(w.x, w.y), sv), rs = mul2(make_float2(w.z, w.w), sv), q = mul2(ws, sv);
+  s_s += ws.x; s_s += ws.y;
+  s_rs += rs.x; s_rs += rs.y;
+  s_ss += q.x; s_ss += q.y;
+}
+#endif
 // ComputeBilateralNCCOld (DPE.cu:696-782) with the reference window precomputed; the window loop
 // for one source sampler, columns dx outer and rows dy inner as the reference window's taps.
-template <bool kClamp, class Src, int kUnroll, class RW>
-__device__ __forceinline__ void strong_window(const PMArgs &a, const WinProj &wp, const Src &src, const RW &rw,
-                                              float &s_s, float &s_ss, float &s_rs) {
+template <class Src, class RW>
+__device__ __forceinline__ void strong_window_any(const PMArgs &a, const WinProj &wp, const Src &src, const RW &rw,
+                                                  float &s_s, float &s_ss, float &s_rs) {
   const int r = a.P.strong_radius, inc = a.P.strong_increment;
+  const WinClamp wc = window_clamp(a, wp);
   float2 acc = make_float2(s_s, s_rs);
   // Tap offsets are small whole numbers, so stepping them by float adds gives the same floats as
   // converting each integer, without a conversion per tap.
-  if (kUnroll > 0 && r == 5 && inc == 2) {
-    for (int ii = 0; ii < 6; ++ii) {
-      const float dx = (float)(2 * ii - 5);
-      const float2 cxy = mul2(wp.g03, make_float2(dx, dx));
-      const float cz = wp.h6 * dx + wp.zc;
-#pragma unroll(kUnroll > 0 ? kUnroll : 1)
-      for (int jj = 0; jj < 6; ++jj)
-        strong_tap<kClamp>(wp, src, rw, cxy, cz, (float)(2 * jj - 5), 6 * ii + jj, acc, s_ss);
-    }
-  } else {
-    int k = 0;
-    const float finc = (float)inc, d0 = (float)(-r);
-    float dx = d0;
-    for (int i = -r; i <= r; i += inc, dx += finc) {
-      const float2 cxy = mul2(wp.g03, make_float2(dx, dx));
-      const float cz = wp.h6 * dx + wp.zc;
-      float dy = d0;
-      for (int j = -r; j <= r; j += inc, dy += finc)
-        strong_tap<kClamp>(wp, src, rw, cxy, cz, dy, k++, acc, s_ss);
-    }
+  int k = 0;
+  const float finc = (float)inc, d0 = (float)(-r);
+  float dx = d0;
+  for (int i = -r; i <= r; i += inc, dx += finc) {
+    const float2 cxy = mul2(wp.g03, make_float2(dx, dx));
+    const float cz = wp.h6 * dx + wp.zc;
+    float dy = d0;
+    for (int j = -r; j <= r; j += inc, dy += finc) strong_tap(wp, wc, src, rw, cxy, cz, dy, k++, acc, s_ss);
   }
   s_s = acc.x;
   s_rs = acc.y;
 }
-template <class Src, int kUnroll, class RW>
+#ifdef __CUDA_ARCH__
+// The 6 x 6 window (radius 5, step 2), two taps at a time.
+template <bool kClamp, class Src, class RW>
+__device__ __forceinline__ void strong_window6(const PMArgs &a, const WinProj &wp, const Src &src, const RW &rw,
+                                               float &s_s, float &s_ss, float &s_rs) {
+  WinClamp wc;
+  if (kClamp) wc = window_clamp(a, wp);
+  // the dy terms of the six rows, the same for every column
+  float2 gx[3], gy[3], gz[3];
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const float2 dy = make_float2((float)(4 * p - 5), (float)(4 * p - 3));
+    gx[p] = mul2(dup2(wp.g14.x), dy);
+    gy[p] = mul2(dup2(wp.g14.y), dy);
+    gz[p] = mul2(dup2(wp.h7), dy);
+  }
+  // (V0 + iy + 1) * pw + (U0 + ix + 1) with iy, ix = biased floor - 0x4B400000, modulo 2^32
+  const unsigned base = ((unsigned)wp.V0 + 1u - 0x4B400000u) * (unsigned)src.pw + ((unsigned)wp.U0 + 1u - 0x4B400000u);
+  float dx = -5.0f;
+#pragma unroll 1
+  for (int ii = 0; ii < 18; ii += 3, dx += 2.0f) {
+    const float cx = wp.g03.x * dx, cy = wp.g03.y * dx, cz = wp.h6 * dx + wp.zc;
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      strong_tap2<kClamp>(wp, wc, src, rw, gx[p], gy[p], gz[p], cx, cy, cz, base, ii + p, s_s, s_ss, s_rs);
+  }
+}
+#endif
+template <class Src, bool kPairs, class RW>
 __device__ __forceinline__ float ncc_strong_src(const PMArgs &a, const WinProj &wp, const Src &src, const RW &rw) {
   float s_s = 0.f, s_ss = 0.f, s_rs = 0.f;
-  // (a clamp-free copy of the loop for windows that project inside the source measured slower:
-  // the second copy costs registers under the strong update's occupancy bound)
-  strong_window<true, Src, kUnroll>(a, wp, src, rw, s_s, s_ss, s_rs);
+#ifdef __CUDA_ARCH__
+  if (kPairs && a.P.strong_radius == 5 && a.P.strong_increment == 2) {
+    // one path per warp: the clamped taps are right for every window, and running both would cost more
+    if (__all_sync(__activemask(), window_inside(a, wp, 5.0f))) strong_window6<false>(a, wp, src, rw, s_s, s_ss, s_rs);
+    else strong_window6<true>(a, wp, src, rw, s_s, s_ss, s_rs);
+  } else
+#endif
+    strong_window_any(a, wp, src, rw, s_s, s_ss, s_rs);
   const float m_s = s_s * rw.inv_wsum;
   const float var_s = s_ss * rw.inv_wsum - m_s * m_s;
   if (rw.var_r < 1e-5f || var_s < 1e-5f) return 2.0f;
   const float cov = s_rs * rw.inv_wsum - rw.mean_r * m_s;
   return fmaxf(0.0f, fminf(2.0f, 1.0f - cov / sqrtf(rw.var_r * var_s)));
 }
-template <int kStage = DPE_STAGE_FP32, int kUnroll = 0, class RW>
+template <int kStage, bool kPairs, class RW>
+__device__ __forceinline__ float ncc_strong_proj(const PMArgs &a, int px, int py, int s, const PlaneProj &pp,
+                                                 const RW &rw) {
+  WinProj wp;
+  if (!window_projection(a, s, pp, pixel_projection(a, s, px, py), wp)) return 2.0f;
+  if (rw.cnt) atomicAdd(rw.cnt, 1ull);
+  return ncc_strong_src<decltype(SrcOf<kStage>::make(a, s)), kPairs, RW>(a, wp, SrcOf<kStage>::make(a, s), rw);
+}
+template <int kStage = DPE_STAGE_FP32, bool kPairs = false, class RW>
 __device__ __forceinline__ float ncc_strong(const PMArgs &a, int px, int py, int s, float4 pl, const RW &rw) {
   WinProj wp;
   if (!window_projection(a, s, pl, px, py, wp)) return 2.0f;
   if (rw.cnt) atomicAdd(rw.cnt, 1ull);
-  return ncc_strong_src<decltype(SrcOf<kStage>::make(a, s)), kUnroll, RW>(a, wp, SrcOf<kStage>::make(a, s), rw);
+  return ncc_strong_src<decltype(SrcOf<kStage>::make(a, s)), kPairs, RW>(a, wp, SrcOf<kStage>::make(a, s), rw);
 }
 
 // ------------------------------------------------------------------ strong NCC adjoint
@@ -732,7 +860,7 @@ __device__ __forceinline__ float ncc_strong_adjoint(const PMArgs &a, int px, int
   const int r = a.P.strong_radius, inc = a.P.strong_increment;
   // pass 1: ncc_strong's own window loop
   float s_s = 0.f, s_ss = 0.f, s_rs = 0.f;
-  strong_window<true, SrcF32, 0>(a, wp, src_f32(a, s), rw, s_s, s_ss, s_rs);
+  strong_window_any(a, wp, src_f32(a, s), rw, s_s, s_ss, s_rs);
   const float m_s = s_s * rw.inv_wsum;
   const float var_s = s_ss * rw.inv_wsum - m_s * m_s;
   if (rw.var_r < 1e-5f || var_s < 1e-5f) return 2.0f;
@@ -744,6 +872,7 @@ __device__ __forceinline__ float ncc_strong_adjoint(const PMArgs &a, int px, int
   // dC/ds_k = w_k / sum(w) * (-(r_k - mean_r) / sq + cov * (s_k - m_s) / (var_s * sq))
   const float ka = -rw.inv_wsum / sq, kb = rw.inv_wsum * cov / (var_s * sq);
   float gH[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const WinClamp wc = window_clamp(a, wp);
   const int W = a.W, Hh = a.H, pw = a.pad_w;
   const float *__restrict__ img = a.img[s];
   int k = 0;
@@ -755,7 +884,7 @@ __device__ __forceinline__ float ncc_strong_adjoint(const PMArgs &a, int px, int
       const float X = wp.g14.x * dy + cx, Y = wp.g14.y * dy + cy, Z = wp.h7 * dy + cz;
       const float iz = tap_rcp(Z);
       const float uo = wp.fuv.x + X * iz, vo = wp.fuv.y + Y * iz;  // offsets from (U0, V0)
-      const float xc = fminf(fmaxf(uo, wp.lo.x), wp.hi.x), yc = fminf(fmaxf(vo, wp.lo.y), wp.hi.y);
+      const float xc = fminf(fmaxf(uo, wc.lo.x), wc.hi.x), yc = fminf(fmaxf(vo, wc.lo.y), wc.hi.y);
       int ix, iy;
       const float fx = floor_split(xc, &ix), fy = floor_split(yc, &iy);
       const float ax = xc - fx, ay = yc - fy;
@@ -766,8 +895,8 @@ __device__ __forceinline__ float ncc_strong_adjoint(const PMArgs &a, int px, int
       const float rc = texel(a, 0, px + i, py + j) - rw.center;  // r_k - c
       const float dc = rw.w(k) * (ka * (rc - rw.mean_r) + kb * (sv - m_s));
       // slope of the sample; zero along a clamped coordinate
-      const float dsx = (uo > wp.lo.x && uo < wp.hi.x) ? (1.0f - ay) * (v10 - v00) + ay * (v11 - v01) : 0.0f;
-      const float dsy = (vo > wp.lo.y && vo < wp.hi.y) ? (1.0f - ax) * (v01 - v00) + ax * (v11 - v10) : 0.0f;
+      const float dsx = (uo > wc.lo.x && uo < wc.hi.x) ? (1.0f - ay) * (v10 - v00) + ay * (v11 - v01) : 0.0f;
+      const float dsy = (vo > wc.lo.y && vo < wc.hi.y) ? (1.0f - ax) * (v01 - v00) + ax * (v11 - v10) : 0.0f;
       // u = X' / Z' with X' = H0. p, Z' = H2. p: du/dH0j = p_j / Z', du/dH2j = -u p_j / Z'
       const float u = (float)wp.U0 + uo, v = (float)wp.V0 + vo;
       const float gu = dc * dsx * iz, gv = dc * dsy * iz;
@@ -801,10 +930,10 @@ __device__ __forceinline__ float ncc_strong_adjoint(const PMArgs &a, int px, int
 }
 
 // Strong costs of plane pl against every source: out[j] = cost against source j + 1.
-template <int kStage, int kUnroll = 0, class RW>
+template <int kStage, bool kPairs = false, class RW>
 __device__ __forceinline__ void ncc_all_sources(const PMArgs &a, int px, int py, float4 pl, const RW &rw,
                                                 float *out) {
-  for (int j = 0; j < a.N - 1; ++j) out[j] = ncc_strong<kStage, kUnroll>(a, px, py, j + 1, pl, rw);
+  for (int j = 0; j < a.N - 1; ++j) out[j] = ncc_strong<kStage, kPairs>(a, px, py, j + 1, pl, rw);
 }
 // Sum over the listed sources act[0..na) (ascending) of vw[j] * cost(j), in list order.
 template <int kStage, class RW, class A>

@@ -77,22 +77,18 @@ __global__ void k_pad_image(const float *__restrict__ src, float *__restrict__ d
   dst[(size_t)(y + 1) * (W + 2) + (x + 1)] = src[(size_t)sy * W + sx];
 }
 
-// Staged copy of one padded source image (PMArgs::pair): word o packs P[o] (low 16 bits) and
-// P[o+1] (high 16 bits) as FP16 or BF16, rounded to nearest-even.  The last word repeats P[o].
+// Staged copy of one padded source image (PMArgs::quad): word o packs the footprint P[o], P[o+1],
+// P[o+pw], P[o+pw+1] as FP16 or BF16, rounded to nearest-even.  Words past the last footprint repeat
+// the last texel.
 template <bool kBF16>
-__global__ void k_stage_pairs(const float *__restrict__ pad, uint32_t *__restrict__ out, long long n) {
+__global__ void k_stage_quads(const float *__restrict__ pad, uint2 *__restrict__ out, long long n, int pw) {
   const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n) return;
-  const float lo = pad[o], hi = pad[o + 1 < n ? o + 1 : o];
-  uint32_t a, b;
-  if (kBF16) {
-    a = __bfloat16_as_ushort(__float2bfloat16_rn(lo));
-    b = __bfloat16_as_ushort(__float2bfloat16_rn(hi));
-  } else {
-    a = __half_as_ushort(__float2half_rn(lo));
-    b = __half_as_ushort(__float2half_rn(hi));
-  }
-  out[o] = a | (b << 16);
+  auto bits = [&](long long k) -> uint32_t {
+    const float v = pad[k < n ? k : n - 1];
+    return kBF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+  };
+  out[o] = make_uint2(bits(o) | bits(o + 1) << 16, bits(o + pw) | bits(o + pw + 1) << 16);
 }
 
 // Sets *flag when any of the n floats is not exact in BF16 (a float is exact when its low 16
@@ -551,7 +547,7 @@ __global__ void __launch_bounds__(128, DPE_COST_MIN_BLOCKS) k_random_init(const 
     a.plane[center] = pl;
     float cv[kMaxSrc], srt[kMaxSrc];
     int valid = 0;
-    ncc_all_sources<kStage, kSweepUnroll>(a, px, py, pl, rw, cv);
+    ncc_all_sources<kStage, true>(a, px, py, pl, rw, cv);
     for (int i = 0; i < n; ++i) {
       const float v = cv[i];
       srt[i] = v;
@@ -581,7 +577,7 @@ __global__ void __launch_bounds__(128, DPE_COST_MIN_BLOCKS) k_random_init(const 
     float cost = 0.0f;
     for (int i = 1; i < a.N; ++i) {
       if (isSet(views, i - 1)) {
-        const float v = ncc_strong<kStage, kSweepUnroll>(a, px, py, i, pl, rw);
+        const float v = ncc_strong<kStage, true>(a, px, py, i, pl, rw);
         if (v < 2.0f) { cnt++; cost += v; }
         else unSetBit(&views, i - 1);
       }
@@ -712,75 +708,95 @@ __device__ __forceinline__ bool gn_solve(const PMArgs &a, int px, int py, float4
 // ------------------------------------------------------------------ strong update (DPE.cu:1218-1670, 1069-1122)
 // Block-cooperative: a block holds kCoopPix pixels of one colour (consecutive x on one row of the
 // half grid) and kCoopLanes threads per pixel.  The pixel's reference window and its candidate
-// cost matrix live once in shared memory; the threads of a pixel evaluate its hypotheses side by
-// side (lane d: candidate d; then the sampled sources of the current plane and of the five
-// refinement planes), and one thread per pixel takes every decision in the reference's order, so
-// the random draws and the order of each weighted sum are those of one thread doing it all.
+// cost matrix live once in shared memory.  The four pixels of a warp put the (plane, source) pairs
+// they need a cost for into one list, and the warp's 32 threads evaluate the list side by side; the
+// threads of a pixel split its other work, and one thread per pixel takes every decision in the
+// reference's order, so the random draws and the order of each weighted sum are those of one thread
+// doing it all.  Everything a pixel needs stays within its warp, so phases end with a warp barrier; the
+// block barriers around an evaluation only keep the block's warps in the same code, which they fetch
+// together (without them the kernel waits on instruction fetch: 62.4 against 55.8 ms below).
 //
-// Phases, separated by block barriers:
-//   0  window taps (lanes split the taps)
-//   1  window sums (lane 0); candidate search (lane d: direction d)
-//   2  candidate costs (lane d: candidate d)
-//   3  view-selection probabilities per source and the 15 uniform draws (lanes split them)
-//   4  view sampling from the draws, in order (lane 0)
-//   5  candidates' weighted costs (lane d) and the current plane's costs (lanes split sources)
-//   6  best candidate, acceptance, refinement planes (lane 0)
-//   7  refinement costs (lanes split plane x source)
-//   8  refinement decisions, outputs (lane 0)
-//   9-11  with the Gauss-Newton hypothesis only: its normal equations (lanes split the sources,
-//         shuffle sums), its costs (lanes split the sources), its decision and the outputs (lane 0)
+// What bounds it: instruction issue and register reads of the tap loop (strong_tap2) and, with
+// several inlined copies of it, instruction fetch.  Hence one evaluation loop (strong_eval) that
+// every stage runs its list through, and lists without what cannot matter:
+//   * candidates with the same plane share one cost row (the cost depends on the plane only), and the
+//     current plane takes the row of a candidate that equals it;
+//   * a refinement plane whose depth is out of range is never taken, and one whose sum over its first
+//     sources already reaches the cost to beat neither: costs are not negative and rounded sums and
+//     quotients of such terms are monotone, so the full sum cannot fall below it.
+// Both leave every decision, and so every result bit, as it was.
+// Six launches on a 1600x1200 view: first call with 10 sources 69.1 -> 55.8 ms, geometric call with 9
+// and a fifth of the pixels WEAK 77.6 -> 55.3 ms; on a 801x603 level image 19.9 -> 12.6 ms.
+//
+// Stages (each: evaluate the list, then the work that follows from the costs and the next list):
+//   start  window taps, candidate search, the list of distinct candidates x all sources
+//   0      edge form's choice between the two searches; view-selection probabilities, the 15 draws,
+//          the sampled sources; candidates' weighted costs; list: current plane x sampled sources
+//   1      best candidate, acceptance, refinement planes; list: the planes x their heaviest sources
+//   2      list: the planes still in play x their other sampled sources
+//   3      refinement decisions, outputs
+//   3, 4   with the Gauss-Newton hypothesis only: its normal equations (shuffle sums) and list; its
+//          decision and the outputs
 constexpr int kCoopPix = 16, kCoopLanes = 8, kCoopThreads = kCoopPix * kCoopLanes;
+constexpr int kWarpPix = 32 / kCoopLanes;  // pixels of one warp
+constexpr int kRows = 17;                  // cost rows of a pixel: 16 candidates, the current plane
+constexpr int kCurRow = 16;
+constexpr int kListCap = kWarpPix * 5 * 15;  // longest list: 5 planes x 15 sources per pixel
 
-// The strong NCC as the cooperative strong update calls it, inlined at each call site (measured:
-// one shared out-of-line copy, which would ease the instruction cache, is 10 % slower).
-template <int kStage>
-__device__ __forceinline__ float coop_ncc(const PMArgs &a, int px, int py, int s, float4 pl, const SmemWindow &rw) {
-  return ncc_strong<kStage, kStrongUnroll>(a, px, py, s, pl, rw);
-}
-template <int kStage>
-__device__ __forceinline__ void coop_ncc_all(const PMArgs &a, int px, int py, float4 pl, const SmemWindow &rw, float *out) {
-  for (int j = 0; j < a.N - 1; ++j) out[j] = coop_ncc<kStage>(a, px, py, j + 1, pl, rw);
-}
+// A plane as the cost evaluation takes it (PlaneProj without the products that its normal gives).
+struct HypProj {
+  double iw, q;
+  float nx, ny;
+};
 
 // Decision state of one pixel, in shared memory.
 struct CoopPixel {
-  float2 win[kWinTaps];  // (w, w * (r - c)) per tap
+  float4 win[kWinPairs];  // the taps in pairs (win_store)
+  HypProj rec[kRows];     // candidates (0-7 the first search, 8-15 the edge form's second), current
   union {
-    float rc[kWinTaps];     // phases 0-1: r - c per tap
-    float probs[kMaxSrc];   // phases 3-4: view-selection probability per source
+    float rc[kWinTaps];   // until the window sums: w (r - c)^2 per tap
+    struct {
+      float probs[kMaxSrc];
+      float pad;
+    };                    // view selection
+    float4 hyp[5];        // from the refinement planes on
   };
-  union {
-    float4 hyp[5];          // phases 6-8: the refinement planes
-    float u[16];            // phases 3-4: the 15 uniform draws of the view sampling
-    float fc[8];            // phases 5-6: the candidates' weighted costs
-  };
-  float4 pl_cur, pl_now;
+  float u[16];            // the uniform draws; then the refinement planes' weighted costs
+  float fc[8];            // the candidates' weighted costs
+  float4 pl_cur, pl_now, n_rand, n_pert;
   float center, inv_wsum, mean_r, var_r;
-  float wn, cost_now, cost_written, depth_now;
-  int pos[8];
-  uint8_t act[32];  // the sampled sources (source index - 1), ascending
-  int na;
+  float wn, cost_now, cost_written, depth_now, depth_rand, depth_pert;
+  int pos[kCurRow];
   uint32_t views_new, temp_sel, rng_ctr;
-  uint8_t flag[8];
+  int cnt;                 // entries of this pixel in its warp's list
+  uint8_t uniq[kCurRow];   // candidate h has a cost row of its own
+  uint8_t dup[kRows];      // the row that holds candidate h's costs (itself, or an equal plane's)
+  uint8_t row[8];          // the row of the candidate kept for direction d
+  uint8_t flag[8];         // direction d has a candidate
+  uint8_t valid[kCurRow];  // the search found candidate h
+  uint8_t samp[16];        // the source each draw selects (255: none)
   uint8_t vw[32];
+  uint8_t act[32];         // the sampled sources (source index - 1), ascending
+  uint8_t alive[8];        // refinement plane h can still be taken
+  uint8_t first, second;   // positions in act of the two heaviest sources
+  uint8_t na;
 };
-// Shared bytes of one block: the pixels' states, then per pixel 8 candidate cost rows and 6
-// hypothesis cost rows of n = N - 1 floats.
+// Shared bytes of one block: the pixels' states, the warps' lists, then per pixel kRows cost rows of
+// n = N - 1 floats.
 __host__ __device__ inline size_t coop_smem_bytes(int n) {
-  return sizeof(CoopPixel) * kCoopPix + sizeof(float) * (size_t)kCoopPix * 14 * n;
+  return sizeof(CoopPixel) * kCoopPix + sizeof(uint16_t) * kListCap * (kCoopThreads / 32) +
+         sizeof(float) * (size_t)kCoopPix * kRows * n;
 }
 
 struct CoopCtx {
   const PMArgs *a;
-  int slot, lane, px, py, center, n;
+  int slot, lane, px, py, center, n, parity;
   bool live;  // a pixel of this colour inside the image, not WEAK
-  CoopPixel *P;
-  float *cost;  // 8 rows of n
-  float *hc;    // 6 rows of n: the current plane, then the five refinement planes
-  __device__ __forceinline__ SmemWindow window() const {
-    return SmemWindow{P->win, P->center, P->inv_wsum, P->mean_r, P->var_r,
-                      a->counters ? a->counters + 2 * KID_STRONG_UPDATE : nullptr};
-  }
+  CoopPixel *P;      // this thread's pixel
+  CoopPixel *W0;     // the first pixel of this thread's warp
+  float *cost;       // this pixel's rows
+  float *cost0;      // the rows of the warp's first pixel
+  uint16_t *list;    // the warp's list: pixel of the warp | row << 2 | source << 7
 };
 
 __device__ __forceinline__ CoopCtx coop_ctx(const Launch &lc, int parity, void *smem) {
@@ -788,6 +804,7 @@ __device__ __forceinline__ CoopCtx coop_ctx(const Launch &lc, int parity, void *
   const PMArgs &a = *B.a;
   CoopCtx c;
   c.a = B.a;
+  c.parity = parity;
   c.slot = (int)threadIdx.x / kCoopLanes;
   c.lane = (int)threadIdx.x % kCoopLanes;
   c.n = a.N - 1;
@@ -797,15 +814,61 @@ __device__ __forceinline__ CoopCtx coop_ctx(const Launch &lc, int parity, void *
   c.live = c.px < a.W && c.py < a.H;
   if (c.live) c.live = G(a.weak, c.center, (long long)a.W * a.H, 201) != DPE_WEAK;
   CoopPixel *base = static_cast<CoopPixel *>(smem);
+  const int warp = (int)threadIdx.x / 32;
   c.P = base + c.slot;
-  float *rows = reinterpret_cast<float *>(base + kCoopPix);
-  c.cost = rows + (size_t)c.slot * 8 * c.n;
-  c.hc = rows + (size_t)kCoopPix * 8 * c.n + (size_t)c.slot * 6 * c.n;
+  c.W0 = base + warp * kWarpPix;
+  uint16_t *lists = reinterpret_cast<uint16_t *>(base + kCoopPix);
+  c.list = lists + (size_t)warp * kListCap;
+  float *rows = reinterpret_cast<float *>(lists + (size_t)kListCap * (kCoopThreads / 32));
+  c.cost = rows + (size_t)c.slot * kRows * c.n;
+  c.cost0 = rows + (size_t)warp * kWarpPix * kRows * c.n;
   return c;
 }
+__device__ __forceinline__ void coop_rec(const CoopCtx &c, int h, float4 pl) {
+  const PlaneProj p = plane_projection(*c.a, pl, c.px, c.py);
+  HypProj &r = c.P->rec[h];
+  r.iw = p.iw; r.q = p.q; r.nx = pl.x; r.ny = pl.y;
+}
+// Entries of the warp's list before this pixel's.
+__device__ __forceinline__ int coop_offset(const CoopCtx &c) {
+  int o = 0;
+  for (int k = 0; k < kWarpPix - 1; ++k)
+    if (k < (c.slot & (kWarpPix - 1))) o += c.W0[k].cnt;
+  return o;
+}
+__device__ __forceinline__ uint16_t coop_entry(const CoopCtx &c, int row, int src) {
+  return (uint16_t)((c.slot & (kWarpPix - 1)) | row << 2 | src << 7);
+}
 
-// Phase 0: the window taps of build_ref_window, split over the lanes.
-__device__ __forceinline__ void strong_p0(const CoopCtx &c) {
+// Evaluates the warp's list: costs of every entry's plane against its source, and against the ns - 1
+// that follow it (stage 0: all sources), sources in the outer order so that the threads of a round
+// read one source image.
+template <int kStage>
+__device__ __forceinline__ void strong_eval(const CoopCtx &c, int ns) {
+  const PMArgs &a = *c.a;
+  int T = 0;
+  for (int k = 0; k < kWarpPix; ++k) T += c.W0[k].cnt;
+  if (T == 0) return;
+  const int px0 = c.px - (c.slot & (kWarpPix - 1)), row2 = c.py - ((c.px + c.parity) & 1);
+  int r = (int)threadIdx.x & 31, j0 = 0;
+  while (true) {
+    while (r >= T) { r -= T; ++j0; }
+    if (j0 >= ns) break;
+    const unsigned e = c.list[r];
+    const int k = e & (kWarpPix - 1), h = (e >> 2) & 31, j = (int)(e >> 7) + j0;
+    const int px = px0 + k, py = row2 + ((px + c.parity) & 1);
+    const CoopPixel &Q = c.W0[k];
+    const HypProj &hp = Q.rec[h];
+    const PlaneProj pp{(double)hp.nx * a.dm[0], (double)hp.ny * a.dm[1], hp.iw, hp.q};
+    const SmemWindow rw{Q.win, Q.center, Q.inv_wsum, Q.mean_r, Q.var_r,
+                        a.counters ? a.counters + 2 * KID_STRONG_UPDATE : nullptr};
+    c.cost0[((size_t)k * kRows + h) * c.n + j] = ncc_strong_proj<kStage, true>(a, px, py, j + 1, pp, rw);
+    r += 32;
+  }
+}
+
+// Window taps of build_ref_window, split over the lanes.
+__device__ __forceinline__ void strong_taps(const CoopCtx &c) {
   if (!c.live) return;
   const PMArgs &a = *c.a;
   const int r = a.P.strong_radius, inc = a.P.strong_increment, side = 2 * r / inc + 1;
@@ -814,9 +877,9 @@ __device__ __forceinline__ void strong_p0(const CoopCtx &c) {
     const int i = -r + (k / side) * inc, j = -r + (k % side) * inc;
     const float rp = texel(a, 0, c.px + i, c.py + j);
     const float w = bilateral_weight((float)i, (float)j, rp, center, a.P.sigma_spatial, a.P.sigma_color);
-    const float rc = rp - center;
-    G(c.P->win, k, kWinTaps, 320) = make_float2(w, w * rc);
-    c.P->rc[k] = rc;
+    const float rc = rp - center, wr = w * rc;
+    win_store(c.P->win, k, w, wr);
+    c.P->rc[k] = wr * rc;
   }
   if (c.lane == 0) c.P->center = center;
 }
@@ -912,93 +975,152 @@ __device__ __forceinline__ int strong_search_edge(const PMArgs &a, int px, int p
   return mc < FLT_MAX ? mp : -1;
 }
 
-// Phase 1: window sums in tap order (lane 0), as build_ref_window accumulates them; every lane
-// searches its candidate direction (the non-edge form; the edge form searches in phase 2).
-__device__ __forceinline__ void strong_p1(const CoopCtx &c) {
+// The edge form's second search for direction d: 11 steps of two pixels (DPE.cu:1302-1333).
+__device__ __forceinline__ int strong_search_edge2(const PMArgs &a, int px, int py, int d, int iter) {
+  [[maybe_unused]] const long long L = (long long)a.W * a.H;
+  const int dx = kDir[d][0], dy = kDir[d][1], min_step = 2;
+  const int sx = cvmax(1, 5 - 2 * iter) * dx, sy = cvmax(1, 5 - 2 * iter) * dy;
+  float mc = FLT_MAX;
+  int mp = -1;
+  int fx = 0, fy = 0;
+  if (d > 4) { if (d % 2) fx = dx; else fy = dy; }
+  for (int s = 0; s < 11; ++s) {
+    const int tx = px + sx + s * min_step * dx + fx, ty = py + sy + s * min_step * dy + fy;
+    if (!(tx >= 0 && ty >= 0 && tx < a.W && ty < a.H)) continue;
+    const int tc = tx + ty * a.W;
+    const float cc = G(a.cost_snap, tc, L, 204);
+    if (mc > cc) { mp = tc; mc = cc; }
+  }
+  return mc < FLT_MAX ? mp : -1;
+}
+
+// Candidate search (lane d: direction d) and the planes' projections; window sums in tap order, as
+// build_ref_window accumulates them (lane 0).
+__device__ __forceinline__ void strong_search(const CoopCtx &c, int iter) {
   if (!c.live) return;
   const PMArgs &a = *c.a;
-  if (c.lane == 0) {
+  [[maybe_unused]] const long long L = (long long)a.W * a.H;
+  CoopPixel &P = *c.P;
+  const int d = c.lane;
+  int pos, pos2 = -1;
+  if (a.P.use_edge) {
+    pos = strong_search_edge(a, c.px, c.py, c.center, d, iter);
+    if (G(a.edge, c.center, L, 203) == 0) pos2 = strong_search_edge2(a, c.px, c.py, d, iter);
+  } else {
+    pos = strong_search_plain(a, c.px, c.py, c.center, d);
+  }
+  P.pos[d] = pos;
+  P.pos[8 + d] = pos2;
+  P.valid[d] = pos >= 0 ? 1 : 0;
+  P.valid[8 + d] = pos2 >= 0 ? 1 : 0;
+  const float4 *planes = a.P.use_edge ? a.plane_snap : a.plane;
+  if (pos >= 0) coop_rec(c, d, G(planes, pos, L, 205));
+  if (pos2 >= 0 && pos2 != pos) coop_rec(c, 8 + d, G(planes, pos2, L, 205));
+  else if (pos2 >= 0) P.rec[8 + d] = P.rec[d];
+  if (d == 0) {
+    const float4 pl = G(a.plane, c.center, L, 212);
+    P.pl_cur = pl;
+    coop_rec(c, kCurRow, pl);
     const int r = a.P.strong_radius, inc = a.P.strong_increment, side = 2 * r / inc + 1;
     float sw = 0.f, swr = 0.f, swrr = 0.f;
     for (int k = 0; k < side * side; ++k) {
-      const float2 t = c.P->win[k];
-      sw += t.x; swr += t.y; swrr += t.y * c.P->rc[k];
+      const float2 t = win_tap(P.win, k);
+      sw += t.x; swr += t.y; swrr += P.rc[k];
     }
-    c.P->inv_wsum = 1.0f / sw;
-    c.P->mean_r = swr * c.P->inv_wsum;
-    c.P->var_r = swrr * c.P->inv_wsum - c.P->mean_r * c.P->mean_r;
+    P.inv_wsum = 1.0f / sw;
+    P.mean_r = swr * P.inv_wsum;
+    P.var_r = swrr * P.inv_wsum - P.mean_r * P.mean_r;
   }
-  if (!a.P.use_edge) c.P->pos[c.lane] = strong_search_plain(a, c.px, c.py, c.center, c.lane);
 }
 
-// Phase 2: candidate d's costs against every source (lane d), with the edge form's second search
-// and its replacement rule (DPE.cu:1302-1366).
-template <int kStage>
-__device__ __forceinline__ void strong_p2(const CoopCtx &c, int iter) {
+__device__ __forceinline__ bool same_rec(const HypProj &x, const HypProj &y) {
+  // by value: +0 and -0 give the same costs, and a NaN plane keeps its own row
+  return x.nx == y.nx && x.ny == y.ny && x.iw == y.iw && x.q == y.q;
+}
+// Which planes need a row of their own: lane d looks at candidates d and 8 + d, lane 0 at the current
+// plane too.
+__device__ __forceinline__ void strong_distinct(const CoopCtx &c) {
+  CoopPixel &P = *c.P;
+  if (!c.live) {
+    if (c.lane == 0) P.cnt = 0;
+    return;
+  }
+  const int last = c.a->P.use_edge ? kCurRow : 8;
+  for (int h = c.lane; h < last; h += 8) {
+    int to = h;
+    if (P.valid[h])
+      for (int e = 0; e < h; ++e)
+        if (P.valid[e] && same_rec(P.rec[e], P.rec[h])) { to = e; break; }
+    P.dup[h] = (uint8_t)to;
+    P.uniq[h] = P.valid[h] && to == h ? 1 : 0;
+  }
+  if (c.lane == kCoopLanes - 1) {
+    int to = kCurRow;
+    for (int e = 0; e < last; ++e)
+      if (P.valid[e] && same_rec(P.rec[e], P.rec[kCurRow])) { to = e; break; }
+    P.dup[kCurRow] = (uint8_t)to;
+  }
+}
+__device__ __forceinline__ void strong_count(const CoopCtx &c) {
+  if (!c.live || c.lane != 0) return;
+  CoopPixel &P = *c.P;
+  const int last = c.a->P.use_edge ? kCurRow : 8;
+  int m = 0;
+  for (int h = 0; h < last; ++h) m += P.uniq[h];
+  P.cnt = m;
+}
+__device__ __forceinline__ void strong_list(const CoopCtx &c) {
   if (!c.live) return;
-  const PMArgs &a = *c.a;
-  const int n = c.n, d = c.lane;
-  [[maybe_unused]] const long long L = (long long)a.W * a.H;
-  float *row = c.cost + d * n;
-  for (int j = 0; j < n; ++j) row[j] = 0.0f;
-  if (d == 0) row[0] = 2.0f;  // `= {2.0f}` initialises only the first element (quirk Q2)
-  const SmemWindow rw = c.window();
-  bool flag = false;
-  int pos = -1;
-  if (a.P.use_edge) {
-    pos = strong_search_edge(a, c.px, c.py, c.center, d, iter);
-    if (pos >= 0) {
-      flag = true;
-      coop_ncc_all<kStage>(a, c.px, c.py, G(a.plane_snap, pos, L, 205), rw, row);
-    }
-    if (G(a.edge, c.center, L, 203) == 0) {
-      const float good_thr = 0.8f * dpe_expf((float)(iter * iter) / (-90.0f));
-      const int dx = kDir[d][0], dy = kDir[d][1], min_step = 2;
-      const int sx = cvmax(1, 5 - 2 * iter) * dx, sy = cvmax(1, 5 - 2 * iter) * dy;
-      const bool had = flag;
-      float mc = FLT_MAX;
-      int mp = -1;
-      int fx = 0, fy = 0;
-      if (d > 4) { if (d % 2) fx = dx; else fy = dy; }
-      for (int s = 0; s < 11; ++s) {
-        const int tx = c.px + sx + s * min_step * dx + fx, ty = c.py + sy + s * min_step * dy + fy;
-        if (!(tx >= 0 && ty >= 0 && tx < a.W && ty < a.H)) continue;
-        const int tc = tx + ty * a.W;
-        const float cc = G(a.cost_snap, tc, L, 204);
-        if (mc > cc) { mp = tc; mc = cc; }
-      }
-      if (mc < FLT_MAX) {
-        flag = true;
-        float tca[kMaxSrc];
-        coop_ncc_all<kStage>(a, c.px, c.py, G(a.plane_snap, mp, L, 205), rw, tca);
-        int g0 = 0, g1 = 0, b0 = 0, b1 = 0;
-        for (int j = 0; j < n; ++j) {
-          if (row[j] < good_thr) g0++;
-          if (row[j] > 1.2f) b0++;
-          if (tca[j] < good_thr) g1++;
-          if (tca[j] > 1.2f) b1++;
-        }
-        if (!had || g1 > g0 || (g1 == g0 && b1 < b0)) {
-          pos = mp;
-          for (int j = 0; j < n; ++j) row[j] = tca[j];
-        }
-      }
-    }
-  } else {
-    pos = c.P->pos[d];
-    if (pos >= 0) {
-      flag = true;
-      coop_ncc_all<kStage>(a, c.px, c.py, G(a.plane, pos, L, 210), rw, row);
-    }
+  const CoopPixel &P = *c.P;
+  const int last = c.a->P.use_edge ? kCurRow : 8;
+  const int off = coop_offset(c);
+  for (int h = c.lane; h < last; h += 8) {
+    if (!P.uniq[h]) continue;
+    int rank = 0;
+    for (int e = 0; e < h; ++e) rank += P.uniq[e];
+    c.list[off + rank] = coop_entry(c, h, 0);
   }
-  c.P->flag[d] = flag ? 1 : 0;
-  c.P->pos[d] = pos;
 }
 
-// Phase 3: the view-selection probability of each source (sample_views' first loop, with the
-// priors of DPE.cu:1551-1563), lane j taking sources j, j + 8, ...; and the 15 uniform draws of
-// the sampling (counter-based, so draw s is the pixel's counter + s), split over the lanes.
-__device__ __forceinline__ void strong_p3(const CoopCtx &c, int iter) {
+// The candidate kept for direction d and its cost row (lane d): the edge form takes the second search
+// where it has more good sources, or as many and fewer bad ones (DPE.cu:1334-1366).  A direction
+// without a candidate keeps the initial costs: 0, and 2 for the first direction's first source,
+// because `= {2.0f}` initialises only the first element (quirk Q2).
+__device__ __forceinline__ void strong_choose(const CoopCtx &c, int iter) {
+  if (!c.live) return;
+  CoopPixel &P = *c.P;
+  const int n = c.n, d = c.lane;
+  const bool v1 = P.valid[d] != 0, v2 = P.valid[8 + d] != 0;
+  int take = d;
+  if (v2) {
+    take = 8 + d;
+    if (v1) {
+      const float good_thr = 0.8f * dpe_expf((float)(iter * iter) / (-90.0f));
+      const float *r0 = c.cost + P.dup[d] * n, *r1 = c.cost + P.dup[8 + d] * n;
+      int g0 = 0, g1 = 0, b0 = 0, b1 = 0;
+      for (int j = 0; j < n; ++j) {
+        if (r0[j] < good_thr) g0++;
+        if (r0[j] > 1.2f) b0++;
+        if (r1[j] < good_thr) g1++;
+        if (r1[j] > 1.2f) b1++;
+      }
+      if (!(g1 > g0 || (g1 == g0 && b1 < b0))) take = d;
+    }
+  }
+  P.flag[d] = v1 || v2 ? 1 : 0;
+  P.row[d] = v1 || v2 ? P.dup[take] : (uint8_t)d;
+  P.pos[d] = v1 || v2 ? P.pos[take] : -1;
+  if (!(v1 || v2)) {
+    float *row = c.cost + d * n;
+    for (int j = 0; j < n; ++j) row[j] = 0.0f;
+    if (d == 0) row[0] = 2.0f;
+  }
+}
+
+// The view-selection probability of each source (sample_views' first loop, with the priors of
+// DPE.cu:1551-1563), lane j taking sources j, j + 8, ...; and the 15 uniform draws of the sampling
+// (counter-based, so draw s is the pixel's counter + s), split over the lanes.
+__device__ __forceinline__ void strong_probs(const CoopCtx &c, int iter) {
   if (!c.live) return;
   const PMArgs &a = *c.a;
   const int W = a.W, n = c.n, center = c.center;
@@ -1024,7 +1146,7 @@ __device__ __forceinline__ void strong_p3(const CoopCtx &c, int iter) {
     int count_false = 0;
     float tmpw = 0;
     for (int d = 0; d < 8; ++d) {
-      const float v = c.cost[d * n + j];
+      const float v = c.cost[P.row[d] * n + j];
       if (v < thr) { tmpw += dpe_expf(v * v / (-0.18f)); count++; }
       if (v > 1.2f) count_false++;
     }
@@ -1033,68 +1155,94 @@ __device__ __forceinline__ void strong_p3(const CoopCtx &c, int iter) {
     else if (count_false < 3) p = base;
     P.probs[j] = p * prior;
   }
-  if (c.lane == 0) {
-    P.rng_ctr = ctr0 + 15;
-    P.pl_cur = G(a.plane, center, L, 212);
-  }
+  if (c.lane == 0) P.rng_ctr = ctr0 + 15;
 }
-
-// Phase 4 (lane 0): the rest of sample_views (normalised cumulative probabilities, the 15
-// samples, the selection mask and weight sum) and the list of sampled sources.
-__device__ __forceinline__ void strong_p4(const CoopCtx &c) {
+// The rest of sample_views: normalised cumulative probabilities (lane 0), the source of each draw (the
+// lanes split the draws), the counts per source (the lanes split the sources), the list of sampled
+// sources and the weight sum (lane 0).
+__device__ __forceinline__ void strong_cumulate(const CoopCtx &c) {
   if (!c.live || c.lane != 0) return;
   const int n = c.n;
   CoopPixel &P = *c.P;
-  for (int i = 0; i < 32; ++i) P.vw[i] = 0;
   float sum = 0.0f;
   for (int i = 0; i < n; ++i) sum += P.probs[i];
   const float inv = 1.0f / sum;
   float cum = 0.0f;
   for (int i = 0; i < n; ++i) { cum += P.probs[i] * inv; P.probs[i] = cum; }
-  for (int s = 0; s < 15; ++s) {
+}
+__device__ __forceinline__ void strong_sample(const CoopCtx &c) {
+  if (!c.live) return;
+  CoopPixel &P = *c.P;
+  for (int s = c.lane; s < 15; s += kCoopLanes) {
     const float r = P.u[s] - FLT_EPSILON;
-    for (int id = 0; id < n; ++id)
-      if (P.probs[id] > r) { P.vw[id] += 1; break; }
+    int id = 0;
+    while (id < c.n && !(P.probs[id] > r)) ++id;
+    P.samp[s] = (uint8_t)(id < c.n ? id : 255);
   }
+}
+__device__ __forceinline__ void strong_weigh(const CoopCtx &c) {
+  if (!c.live) return;
+  CoopPixel &P = *c.P;
+  for (int j = c.lane; j < 32; j += kCoopLanes) {
+    int m = 0;
+    if (j < c.n)
+      for (int s = 0; s < 15; ++s) m += P.samp[s] == j;
+    P.vw[j] = (uint8_t)m;
+  }
+}
+__device__ __forceinline__ void strong_active(const CoopCtx &c) {
+  if (c.lane != 0) return;
+  CoopPixel &P = *c.P;
+  if (!c.live) { P.cnt = 0; return; }
   uint32_t sel = 0;
   float wn = 0;
-  int na = 0;
-  for (int i = 0; i < n; ++i)
-    if (P.vw[i] > 0) { setBit(&sel, i); wn += P.vw[i]; P.act[na++] = i; }
-  P.na = na;
+  int na = 0, w1 = 0, w2 = 0, f1 = 0, f2 = 0;
+  for (int i = 0; i < c.n; ++i) {
+    const int v = P.vw[i];
+    if (v > 0) {
+      setBit(&sel, i);
+      wn += v;
+      if (v > w1) { w2 = w1; f2 = f1; w1 = v; f1 = na; }
+      else if (v > w2) { w2 = v; f2 = na; }
+      P.act[na++] = (uint8_t)i;
+    }
+  }
+  P.na = (uint8_t)na;
+  P.first = (uint8_t)f1;
+  P.second = (uint8_t)f2;
   P.wn = wn;
   P.temp_sel = sel;
+  // the current plane is evaluated unless a candidate's row holds its costs
+  P.cnt = P.dup[kCurRow] == kCurRow ? na : 0;
 }
-
-// Phase 5: candidate d's cost weighted by the samples (lane d), then the current plane's cost
-// against each sampled source (lanes split the sources).
-template <int kStage>
-__device__ __forceinline__ void strong_p5(const CoopCtx &c) {
+// Candidate d's cost weighted by the samples (lane d); the current plane's list.
+__device__ __forceinline__ void strong_weighted(const CoopCtx &c) {
   if (!c.live) return;
   CoopPixel &P = *c.P;
   const int n = c.n, d = c.lane;
+  const float *row = c.cost + P.row[d] * n;
   float fc = 0.0f;
   for (int j = 0; j < n; ++j)
-    if (P.vw[j] > 0) fc += P.vw[j] * c.cost[d * n + j];
+    if (P.vw[j] > 0) fc += P.vw[j] * row[j];
   P.fc[d] = fc / P.wn;
-  const SmemWindow rw = c.window();
-  const int na = P.na;
-  const float4 pl = P.pl_cur;
-  for (int q = c.lane; q < na; q += kCoopLanes)
-    c.hc[q] = coop_ncc<kStage>(*c.a, c.px, c.py, P.act[q] + 1, pl, rw);
+  if (P.cnt > 0) {
+    const int off = coop_offset(c);
+    for (int q = c.lane; q < P.na; q += kCoopLanes) c.list[off + q] = coop_entry(c, kCurRow, P.act[q]);
+  }
 }
 
-// Phase 6 (lane 0): the current cost, the best candidate and its acceptance, and the five
-// refinement planes of PlaneHypothesisRefinementStrong (DPE.cu:1069-1122) with their draws.
-__device__ __forceinline__ void strong_p6(const CoopCtx &c) {
+// The current cost, the best candidate and its acceptance, and the draws of
+// PlaneHypothesisRefinementStrong (DPE.cu:1069-1122) (lane 0).
+__device__ __forceinline__ void strong_accept(const CoopCtx &c) {
   if (!c.live || c.lane != 0) return;
   const PMArgs &a = *c.a;
   const dpe_camera &rc = a.cam[0];
   [[maybe_unused]] const long long L = (long long)a.W * a.H;
   CoopPixel &P = *c.P;
   const int na = P.na;
+  const float *cur = c.cost + P.dup[kCurRow] * c.n;
   float cost_now = 0.0f;
-  for (int q = 0; q < na; ++q) cost_now += P.vw[P.act[q]] * c.hc[q];
+  for (int q = 0; q < na; ++q) cost_now += P.vw[P.act[q]] * cur[P.act[q]];
   cost_now /= P.wn;
   P.cost_written = cost_now;
   const float4 pl_cur = P.pl_cur;
@@ -1113,35 +1261,106 @@ __device__ __forceinline__ void strong_p6(const CoopCtx &c) {
   }
   Rng rng{a.key[0], a.key[1], (uint32_t)c.center, P.rng_ctr};
   const float dmin = a.P.depth_min, dmax = a.P.depth_max;
-  const float depth_rand = rng.uniform() * (dmax - dmin) + dmin;
-  const float4 n_rand = random_normal(rc, c.px, c.py, rng, depth_now);
+  P.depth_rand = rng.uniform() * (dmax - dmin) + dmin;
+  P.n_rand = random_normal(rc, c.px, c.py, rng, depth_now);
   const float lo = (1 - 0.02f) * depth_now, hi = (1 + 0.02f) * depth_now;
-  const float depth_pert = rng.uniform() * (hi - lo) + lo;
-  const float4 n_pert = perturbed_normal(rc, c.px, c.py, pl_now, rng, (float)(0.02f * 3.14159265358979323846));
-  const float depths[5] = {depth_rand, depth_now, depth_rand, depth_now, depth_pert};
-  const float4 normals[5] = {pl_now, n_rand, n_rand, n_pert, pl_now};
-  for (int h = 0; h < 5; ++h) {
-    float4 t = normals[h];
-    t.w = dist_to_origin(rc, c.px, c.py, depths[h], t);
-    P.hyp[h] = t;
-  }
+  P.depth_pert = rng.uniform() * (hi - lo) + lo;
+  P.n_pert = perturbed_normal(rc, c.px, c.py, pl_now, rng, (float)(0.02f * 3.14159265358979323846));
   P.pl_now = pl_now;
   P.depth_now = depth_now;
   P.cost_now = cost_now;
   P.views_new = views_new;
   P.rng_ctr = rng.ctr;
 }
-
-// Phase 7: the refinement planes' costs, (plane, sampled source) pairs split over the lanes.
-template <int kStage>
-__device__ __forceinline__ void strong_p7(const CoopCtx &c) {
+// Refinement plane h (lane h): (random depth, normal now), (depth now, random normal), both random,
+// (depth now, perturbed normal), (perturbed depth, normal now).  Its first sources: the heaviest, and
+// for the perturbed planes, which often win, the next one too.
+__device__ __forceinline__ int refine_first(const CoopPixel &P, int h) {
+  return P.na == 0 ? 0 : (h >= 3 && P.na > 1) ? 2 : 1;
+}
+__device__ __forceinline__ void strong_planes(const CoopCtx &c) {
+  CoopPixel &P = *c.P;
   if (!c.live) return;
-  const SmemWindow rw = c.window();
-  const int na = c.P->na, n = c.n;
-  for (int i = c.lane; i < 5 * na; i += kCoopLanes) {
-    const int h = i / na, q = i - h * na;
-    c.hc[(1 + h) * n + q] = coop_ncc<kStage>(*c.a, c.px, c.py, c.P->act[q] + 1, c.P->hyp[h], rw);
+  const int h = c.lane;
+  if (h >= 5) return;
+  const PMArgs &a = *c.a;
+  const dpe_camera &rc = a.cam[0];
+  float4 t = h == 0 || h == 4 ? P.pl_now : h == 3 ? P.n_pert : P.n_rand;
+  const float depth = h == 0 || h == 2 ? P.depth_rand : h == 4 ? P.depth_pert : P.depth_now;
+  t.w = dist_to_origin(rc, c.px, c.py, depth, t);
+  P.hyp[h] = t;
+  coop_rec(c, h, t);
+  const float db = depth_from_plane(rc, t, c.px, c.py);
+  P.alive[h] = db >= a.P.depth_min && db <= a.P.depth_max && P.na > 0 ? 1 : 0;
+}
+__device__ __forceinline__ void strong_first_count(const CoopCtx &c) {
+  CoopPixel &P = *c.P;
+  if (c.lane != 0) return;
+  int m = 0;
+  if (c.live)
+    for (int h = 0; h < 5; ++h)
+      if (P.alive[h]) m += refine_first(P, h);
+  P.cnt = m;
+}
+__device__ __forceinline__ void strong_first_list(const CoopCtx &c) {
+  if (!c.live || c.lane >= 5) return;
+  const CoopPixel &P = *c.P;
+  const int h = c.lane;
+  if (!P.alive[h]) return;
+  int o = coop_offset(c);
+  for (int e = 0; e < h; ++e)
+    if (P.alive[e]) o += refine_first(P, e);
+  c.list[o] = coop_entry(c, h, P.act[P.first]);
+  if (refine_first(P, h) > 1) c.list[o + 1] = coop_entry(c, h, P.act[P.second]);
+}
+// A plane whose first sources' weighted sum already reaches the cost to beat is out of play (lane h).
+__device__ __forceinline__ void strong_drop(const CoopCtx &c) {
+  if (!c.live || c.lane >= 5) return;
+  CoopPixel &P = *c.P;
+  const int h = c.lane;
+  if (!P.alive[h]) return;
+  const float *row = c.cost + h * c.n;
+  const int s0 = P.act[P.first], s1 = P.act[P.second];
+  float t = 0.0f;
+  if (refine_first(P, h) > 1) {  // in the order of the full sum
+    t += P.vw[min(s0, s1)] * row[min(s0, s1)];
+    t += P.vw[max(s0, s1)] * row[max(s0, s1)];
+  } else {
+    t += P.vw[s0] * row[s0];
   }
+  if (!(t / P.wn < P.cost_now)) P.alive[h] = 0;
+}
+__device__ __forceinline__ void strong_rest_count(const CoopCtx &c) {
+  CoopPixel &P = *c.P;
+  if (c.lane != 0) return;
+  int m = 0;
+  if (c.live)
+    for (int h = 0; h < 5; ++h)
+      if (P.alive[h]) m += P.na - refine_first(P, h);
+  P.cnt = m;
+}
+__device__ __forceinline__ void strong_rest_list(const CoopCtx &c) {
+  if (!c.live || c.lane >= 5) return;
+  const CoopPixel &P = *c.P;
+  const int h = c.lane;
+  if (!P.alive[h]) return;
+  int o = coop_offset(c);
+  for (int e = 0; e < h; ++e)
+    if (P.alive[e]) o += P.na - refine_first(P, e);
+  const bool two = refine_first(P, h) > 1;
+  for (int q = 0; q < P.na; ++q)
+    if (q != P.first && !(two && q == P.second)) c.list[o++] = coop_entry(c, h, P.act[q]);
+}
+// Plane h's weighted cost in list order (lane h).
+__device__ __forceinline__ void strong_refine_sum(const CoopCtx &c) {
+  if (!c.live || c.lane >= 5) return;
+  CoopPixel &P = *c.P;
+  const int h = c.lane, na = P.na;
+  if (!P.alive[h]) return;
+  const float *row = c.cost + h * c.n;
+  float tc = 0.0f;
+  for (int q = 0; q < na; ++q) tc += P.vw[P.act[q]] * row[P.act[q]];
+  P.u[h] = tc / P.wn;
 }
 
 // The pixel's outputs after its last decision.
@@ -1163,40 +1382,32 @@ __device__ __forceinline__ void strong_write(const CoopCtx &c, float4 pl_now, fl
   }
 }
 
-// Phase 8 (lane 0): the refinement decisions in order, then the outputs -- or, with the
-// Gauss-Newton hypothesis, the state phases 9-11 continue from.
-template <int kStage, bool kGN>
-__device__ __forceinline__ void strong_p8(const CoopCtx &c) {
+// The refinement decisions in order (lane 0), then the outputs -- or, with the Gauss-Newton hypothesis,
+// the state its stages continue from.
+template <bool kGN>
+__device__ __forceinline__ void strong_decide(const CoopCtx &c) {
   if (!c.live || c.lane != 0) return;
-  const PMArgs &a = *c.a;
-  const dpe_camera &rc = a.cam[0];
-  const int na = c.P->na, n = c.n;
+  const dpe_camera &rc = c.a->cam[0];
   CoopPixel &P = *c.P;
-  const float dmin = a.P.depth_min, dmax = a.P.depth_max;
-  float depth_now = P.depth_now, cost_now = P.cost_now;
-  float4 pl_now = P.pl_now;
-  for (int h = 0; h < 5; ++h) {
-    const float4 t = P.hyp[h];
-    float tc = 0.0f;
-    for (int q = 0; q < na; ++q) tc += P.vw[P.act[q]] * c.hc[(1 + h) * n + q];
-    tc /= P.wn;
-    const float db = depth_from_plane(rc, t, c.px, c.py);
-    if (db >= dmin && db <= dmax && tc < cost_now) { depth_now = db; pl_now = t; cost_now = tc; }
-  }
+  float cost_now = P.cost_now;
+  int best = -1;
+  for (int h = 0; h < 5; ++h)
+    if (P.alive[h] && P.u[h] < cost_now) { best = h; cost_now = P.u[h]; }
+  const float4 pl_now = best >= 0 ? P.hyp[best] : P.pl_now;
   if (kGN) {
-    P.pl_now = pl_now; P.depth_now = depth_now; P.cost_now = cost_now;
+    if (best >= 0) P.depth_now = depth_from_plane(rc, pl_now, c.px, c.py);
+    P.pl_now = pl_now; P.cost_now = cost_now;
     return;
   }
   strong_write(c, pl_now, cost_now);
 }
 
 #ifdef __CUDA_ARCH__
-// Phases 9-11, the Gauss-Newton hypothesis split over the lanes of a pixel.
-// Phase 9: lane q adds the normal equations of sampled sources q, q + 8, ...; the lanes' sums are
-// added by shuffles inside each 8-lane group (a pixel's lanes are 8 consecutive threads of one
-// warp, and every thread of the block takes part); lane 0 solves and keeps the plane in hyp[0].
-template <int kStage>
-__device__ __forceinline__ void strong_p9_gn(const CoopCtx &c) {
+// The Gauss-Newton hypothesis split over the lanes of a pixel: lane q adds the normal equations of
+// sampled sources q, q + 8, ...; the lanes' sums are added by shuffles inside each 8-lane group (a
+// pixel's lanes are 8 consecutive threads of one warp, and every thread of the block takes part);
+// lane 0 solves, keeps the plane in hyp[0] and lists it against the sampled sources.
+__device__ __forceinline__ void strong_gn(const CoopCtx &c) {
   static_assert(kCoopLanes == 8 && kCoopThreads % 32 == 0, "lane groups must tile whole warps");
   CoopPixel &P = *c.P;
   const bool on = c.live && P.na > 0;
@@ -1205,7 +1416,8 @@ __device__ __forceinline__ void strong_p9_gn(const CoopCtx &c) {
   if (on) {
     const PMArgs &a = *c.a;
     f = gn_frame(a.cam[0], c.px, c.py, P.pl_now, P.depth_now);
-    const SmemWindow rw = c.window();
+    const SmemWindow rw{P.win, P.center, P.inv_wsum, P.mean_r, P.var_r,
+                        a.counters ? a.counters + 2 * KID_STRONG_UPDATE : nullptr};
     for (int q = c.lane; q < P.na; q += kCoopLanes)
       gn_accumulate(a, c.px, c.py, rw, P.pl_now, f, P.act[q], (float)P.vw[P.act[q]], m);
   }
@@ -1213,32 +1425,32 @@ __device__ __forceinline__ void strong_p9_gn(const CoopCtx &c) {
   for (int k = 0; k < 9; ++k)
 #pragma unroll
     for (int off = 1; off < kCoopLanes; off <<= 1) m[k] += __shfl_xor_sync(0xffffffffu, m[k], off, kCoopLanes);
-  if (on && c.lane == 0) {
+  if (c.lane == 0) {
     float4 t;
-    const bool ok = gn_solve(*c.a, c.px, c.py, P.pl_now, f, m, &t);
+    const bool ok = on && gn_solve(*c.a, c.px, c.py, P.pl_now, f, m, &t);
     P.flag[0] = ok ? 1 : 0;
-    if (ok) P.hyp[0] = t;
+    if (ok) {
+      P.hyp[0] = t;
+      coop_rec(c, 0, t);
+    }
+    P.cnt = ok ? P.na : 0;
   }
 }
-// Phase 10: the hypothesis' cost against each sampled source, split over the lanes (hc row 0).
-template <int kStage>
-__device__ __forceinline__ void strong_p10_gn(const CoopCtx &c) {
+__device__ __forceinline__ void strong_gn_list(const CoopCtx &c) {
   if (!c.live) return;
-  const CoopPixel &P = *c.P;
-  if (P.na == 0 || !P.flag[0]) return;
-  const SmemWindow rw = c.window();
-  for (int q = c.lane; q < P.na; q += kCoopLanes) c.hc[q] = coop_ncc<kStage>(*c.a, c.px, c.py, P.act[q] + 1, P.hyp[0], rw);
+  const int off = coop_offset(c);
+  for (int q = c.lane; q < c.P->cnt; q += kCoopLanes) c.list[off + q] = coop_entry(c, 0, c.P->act[q]);
 }
-// Phase 11 (lane 0): the weighted cost in list order, the decision, the outputs.
-__device__ __forceinline__ void strong_p11_gn(const CoopCtx &c) {
+// The weighted cost in list order, the decision, the outputs (lane 0).
+__device__ __forceinline__ void strong_gn_decide(const CoopCtx &c) {
   if (!c.live || c.lane != 0) return;
   const PMArgs &a = *c.a;
   const CoopPixel &P = *c.P;
   float4 pl_now = P.pl_now;
   float cost_now = P.cost_now;
-  if (P.na > 0 && P.flag[0]) {
+  if (P.cnt > 0) {
     float tc = 0.0f;
-    for (int q = 0; q < P.na; ++q) tc += P.vw[P.act[q]] * c.hc[q];
+    for (int q = 0; q < P.na; ++q) tc += P.vw[P.act[q]] * c.cost[P.act[q]];
     tc /= P.wn;
     const float4 t = P.hyp[0];
     const float db = depth_from_plane(a.cam[0], t, c.px, c.py);
@@ -1246,25 +1458,58 @@ __device__ __forceinline__ void strong_p11_gn(const CoopCtx &c) {
   }
   strong_write(c, pl_now, cost_now);
 }
+#define DPE_WARP_BARRIER() __syncwarp()
+#else
+#define DPE_WARP_BARRIER() ((void)0)
 #endif
 
-// One phase for one thread (host builds of this source run the phases in lock-step over a block).
+// The phases between barriers, one thread's part of each (host builds of this source run them in
+// lock-step over a block).
+enum {
+  kPhTaps, kPhSearch, kPhDistinct, kPhCount, kPhList, kPhEval0, kPhChoose, kPhProbs, kPhCumulate, kPhSample, kPhWeigh,
+  kPhActive, kPhWeighted, kPhEval1, kPhAccept, kPhPlanes, kPhFirstCount, kPhFirstList, kPhEval2, kPhDrop, kPhRestCount,
+  kPhRestList, kPhEval3, kPhRefineSum, kPhDecide, kStrongPhases
+};
 template <int kStage, bool kGN>
-__device__ __forceinline__ void strong_update_phase(int phase, const Launch &lc, int iter, int parity, void *smem) {
-  const CoopCtx c = coop_ctx(lc, parity, smem);
+__device__ __forceinline__ void strong_phase(const CoopCtx &c, int phase, int iter) {
   switch (phase) {
-    case 0: strong_p0(c); break;
-    case 1: strong_p1(c); break;
-    case 2: strong_p2<kStage>(c, iter); break;
-    case 3: strong_p3(c, iter); break;
-    case 4: strong_p4(c); break;
-    case 5: strong_p5<kStage>(c); break;
-    case 6: strong_p6(c); break;
-    case 7: strong_p7<kStage>(c); break;
-    default: strong_p8<kStage, kGN>(c); break;
+    case kPhTaps: strong_taps(c); break;
+    case kPhSearch: strong_search(c, iter); break;
+    case kPhDistinct: strong_distinct(c); break;
+    case kPhCount: strong_count(c); break;
+    case kPhList: strong_list(c); break;
+    case kPhChoose: strong_choose(c, iter); break;
+    case kPhProbs: strong_probs(c, iter); break;
+    case kPhCumulate: strong_cumulate(c); break;
+    case kPhSample: strong_sample(c); break;
+    case kPhWeigh: strong_weigh(c); break;
+    case kPhActive: strong_active(c); break;
+    case kPhWeighted: strong_weighted(c); break;
+    case kPhAccept: strong_accept(c); break;
+    case kPhPlanes: strong_planes(c); break;
+    case kPhFirstCount: strong_first_count(c); break;
+    case kPhFirstList: strong_first_list(c); break;
+    case kPhDrop: strong_drop(c); break;
+    case kPhRestCount: strong_rest_count(c); break;
+    case kPhRestList: strong_rest_list(c); break;
+    case kPhRefineSum: strong_refine_sum(c); break;
+    case kPhDecide: strong_decide<kGN>(c); break;
+    case kPhEval0: strong_eval<kStage>(c, c.n); break;
+    default: strong_eval<kStage>(c, 1); break;
   }
 }
-constexpr int kStrongPhases = 9;
+template <int kStage, bool kGN>
+__device__ __forceinline__ void strong_update_phase(int phase, const Launch &lc, int iter, int parity, void *smem) {
+  strong_phase<kStage, kGN>(coop_ctx(lc, parity, smem), phase, iter);
+}
+
+// Phases kFirst..kLast, each followed by a warp barrier.
+template <int kStage, bool kGN, int kFirst, int kLast>
+__device__ __forceinline__ void strong_run(const CoopCtx &c, int iter) {
+  strong_phase<kStage, kGN>(c, kFirst, iter);
+  DPE_WARP_BARRIER();
+  if constexpr (kFirst < kLast) strong_run<kStage, kGN, kFirst + 1, kLast>(c, iter);
+}
 
 // Grid: ((W + 15) / 16, (H + 1) / 2) blocks of kCoopThreads; coop_smem_bytes(N - 1) dynamic shared
 // bytes (the largest N of a batch).
@@ -1272,33 +1517,29 @@ template <int kStage, bool kGN>
 __global__ void __launch_bounds__(kCoopThreads, DPE_STRONG_MIN_BLOCKS) k_strong_update(const Launch lc, int iter, int parity) {
   extern __shared__ float4 coop_smem[];
   const CoopCtx c = coop_ctx(lc, parity, coop_smem);
-  strong_p0(c);
-  __syncthreads();
-  strong_p1(c);
-  __syncthreads();
-  strong_p2<kStage>(c, iter);
-  __syncthreads();
-  strong_p3(c, iter);
-  __syncthreads();
-  strong_p4(c);
-  __syncthreads();
-  strong_p5<kStage>(c);
-  __syncthreads();
-  strong_p6(c);
-  __syncthreads();
-  strong_p7<kStage>(c);
-  __syncthreads();
-  strong_p8<kStage, kGN>(c);
+  strong_run<kStage, kGN, kPhTaps, kPhList>(c, iter);
+#pragma unroll 1
+  for (int stage = 0; stage < (kGN ? 5 : 4); ++stage) {
+    __syncthreads();
+    strong_eval<kStage>(c, stage == 0 ? c.n : 1);
+    __syncthreads();
+    if (stage == 0) strong_run<kStage, kGN, kPhChoose, kPhWeighted>(c, iter);
+    else if (stage == 1) strong_run<kStage, kGN, kPhAccept, kPhFirstList>(c, iter);
+    else if (stage == 2) strong_run<kStage, kGN, kPhDrop, kPhRestList>(c, iter);
+    else if (stage == 3) {
+      strong_run<kStage, kGN, kPhRefineSum, kPhDecide>(c, iter);
 #ifdef __CUDA_ARCH__
-  if constexpr (kGN) {
-    __syncthreads();
-    strong_p9_gn<kStage>(c);
-    __syncthreads();
-    strong_p10_gn<kStage>(c);
-    __syncthreads();
-    strong_p11_gn(c);
-  }
+      if constexpr (kGN) {
+        strong_gn(c);
+        DPE_WARP_BARRIER();
+        strong_gn_list(c);
+        DPE_WARP_BARRIER();
+      }
+    } else {
+      if constexpr (kGN) strong_gn_decide(c);
 #endif
+    }
+  }
 }
 
 
@@ -1762,7 +2003,7 @@ __global__ void k_filter_strong(const Launch lc, int parity) {
 //   phase 2  sample costs (lanes split the samples; LocalRefine also the current plane's sources)
 //   phase 3  the decision (lane 0)
 struct SweepPixel {
-  float2 win[kWinTaps];
+  float4 win[kWinPairs];
   float rc[kWinTaps];
   float4 pl;
   uint4 vw;
@@ -1817,7 +2058,7 @@ __device__ __forceinline__ void sweep_p0(const SweepCtx &c) {
     const float rp = texel(a, 0, c.px + i, c.py + j);
     const float w = bilateral_weight((float)i, (float)j, rp, center, a.P.sigma_spatial, a.P.sigma_color);
     const float rcv = rp - center;
-    G(c.P->win, k, kWinTaps, 320) = make_float2(w, w * rcv);
+    win_store(c.P->win, k, w, w * rcv);
     c.P->rc[k] = rcv;
   }
   if (c.lane == 0) c.P->center = center;
@@ -1833,7 +2074,7 @@ __device__ __forceinline__ void sweep_p1(const SweepCtx &c) {
   const int r = a.P.strong_radius, inc = a.P.strong_increment, side = 2 * r / inc + 1;
   float sw = 0.f, swr = 0.f, swrr = 0.f;
   for (int k = 0; k < side * side; ++k) {
-    const float2 t = P.win[k];
+    const float2 t = win_tap(P.win, k);
     sw += t.x; swr += t.y; swrr += t.y * P.rc[k];
   }
   P.inv_wsum = 1.0f / sw;
@@ -1877,10 +2118,10 @@ __device__ __forceinline__ float sweep_sample(const SweepCtx &c, const SmemWindo
     const int vi = P.act[q];
     const int w = vweight_at(P.vw, vi);
     if (kLocal) {
-      cost += ncc_strong<kStage, kSweepUnroll>(a, c.px, c.py, vi + 1, t, rw) * w;
+      cost += ncc_strong<kStage, true>(a, c.px, c.py, vi + 1, t, rw) * w;
       if (a.P.geom_consistency) cost += a.P.geom_factor * geom_cost(a, c.px, c.py, vi + 1, t) * w;
     } else {
-      float tc = ncc_strong<kStage, kSweepUnroll>(a, c.px, c.py, vi + 1, t, rw);
+      float tc = ncc_strong<kStage, true>(a, c.px, c.py, vi + 1, t, rw);
       if (a.P.geom_consistency) tc += a.P.geom_factor * geom_cost(a, c.px, c.py, vi + 1, t);
       cost += tc * w;
     }
@@ -1971,7 +2212,7 @@ __device__ __forceinline__ void lr_p2(const SweepCtx &c) {
     float4 t = P.pl;
     t.w = dist_to_origin(a.cam[0], c.px, c.py, pdep, t);
     const int si = P.act[q] + 1;
-    const float ncc = ncc_strong<kStage, kSweepUnroll>(a, c.px, c.py, si, t, rw);
+    const float ncc = ncc_strong<kStage, true>(a, c.px, c.py, si, t, rw);
     c.items[h * n + q] = make_float2(ncc, geom ? geom_cost(a, c.px, c.py, si, t) : 0.0f);
   }
 }

@@ -417,12 +417,12 @@ int dpe_view_scores(dpe_ctx *ctx, const dpe_sparse_model *m, double *scores_out)
 enum { DPE_STAGE_FP32 = 0, DPE_STAGE_FP16 = 1, DPE_STAGE_BF16 = 2 };
 typedef struct dpe_options {
   /* Storage of the source images the cost kernels sample (DPE_STAGE_*).  FP16 / BF16 keep each
-   * padded texel and its right neighbour in one 32-bit word; the bilinear interpolation, the
-   * moments and the NCC stay FP32, as do the reference image and the window weights.  Images of
-   * 8-bit integers are exact in both (the finest pyramid level); interpolated pyramid levels are
-   * rounded.  Default DPE_STAGE_FP32: sources sampled as FP32 values, from BF16 pairs when every
-   * source texel of the call is exact in BF16 (checked on the device), which gives the same
-   * results with half the gather bytes. */
+   * padded texel's 2x2 footprint as four 16-bit values, one load per bilinear sample; the
+   * interpolation, the moments and the NCC stay FP32, as do the reference image and the
+   * window weights.  Images of 8-bit integers are exact in both (the finest pyramid level);
+   * interpolated pyramid levels are rounded.  Default DPE_STAGE_FP32: sources sampled as FP32
+   * values, from BF16 footprints when every source texel of the call is exact in BF16 (checked on
+   * the device), which gives the same results with a quarter of the loads. */
   int staging;
   /* 1: every strong-update iteration adds one Gauss-Newton plane hypothesis, built from the
    * adjoint of the strong NCC (dpe_ncc_grad) over the pixel's sampled sources, and keeps it when
