@@ -492,6 +492,18 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
     } else {
       a.edge = p->edge; a.edge_low = p->edge_low_res;
     }
+    // Walks of a line stop after max_step steps (line_map): where no edge is that near, none is met.
+    const int radius = (int)round(std::max(a.lowW, a.lowH) / 60.0);
+    if (a.P.use_limit && a.P.use_APD && a.P.high_res_img && radius > 0) {
+      uint8_t *rows = get((uint8_t *)0, "edge_clear_rows", LL), *clear = get((uint8_t *)0, "edge_clear", LL);
+      if (!rows || !clear) return DPE_ERR_OUT_OF_MEMORY;
+      const dim3 gr((a.lowW + 31) / 32, (a.lowH + 7) / 8), bl(32, 8);
+      k_edge_clear_rows<<<gr, bl, 0, s>>>(a.edge_low, a.lowW, a.lowH, radius, rows);
+      PM_LAUNCHED("k_edge_clear_rows", s);
+      k_edge_clear_cols<<<gr, bl, 0, s>>>(rows, a.lowW, a.lowH, radius, clear);
+      PM_LAUNCHED("k_edge_clear_cols", s);
+      a.edge_dist = clear;
+    }
   }
   if (a.P.use_label) {
     if (host) {
@@ -563,11 +575,11 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
 // Grids of one kernel sequence: for one problem the 2D pixel grids; for a batch one 1D grid per
 // kind over all problems, with the prefix tables the kernels resolve their problem from.
 struct SequenceGrids {
-  Launch full, half, prep, eval, coop, sweep;
+  Launch full, half, prep, eval, coop, sweep, gneigh;
   dim3 fg, hg, cg, sg;
   size_t coop_smem = 0;  // dynamic shared bytes of the strong update (largest source count)
   size_t lr_smem = 0;    // dynamic shared bytes of LocalRefine (largest source count)
-  unsigned gp = 0, ge = 0;
+  unsigned gp = 0, ge = 0, gn = 0;
   const dim3 fb = kFullBlock, hb = kHalfBlock;
 };
 
@@ -632,15 +644,16 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   DPE_TIMED(ctx, KID_GEN_EDGE_INFORM, s,
             shaped(KID_GEN_EDGE_INFORM, [&](dim3 gr, dim3 bl) { k_gen_edge_inform<<<gr, bl, 0, s>>>(g.full); }));
   PM_LAUNCHED("k_gen_edge_inform", s);
-  DPE_TIMED(ctx, KID_FIND_NEAREST, s,
-            shaped(KID_FIND_NEAREST, [&](dim3 gr, dim3 bl) { k_find_nearest_strong<<<gr, bl, 0, s>>>(g.full); }));
-  PM_LAUNCHED("k_find_nearest_strong", s);
-  DPE_TIMED(ctx, KID_GEN_NEIGHBOURS, s,
-            shaped(KID_GEN_NEIGHBOURS, [&](dim3 gr, dim3 bl) { k_gen_neighbours<<<gr, bl, 0, s>>>(g.full); }));
-  PM_LAUNCHED("k_gen_neighbours", s);
-  DPE_TIMED(ctx, KID_NEIGHBOUR_UPDATE, s, k_neighbour_update<<<g.fg, g.fb, 0, s>>>(g.full));
-  PM_LAUNCHED("k_neighbour_update", s);
   if (P.use_APD) {
+    // only WEAK pixels have neighbours; without APD there is none
+    DPE_TIMED(ctx, KID_FIND_NEAREST, s, k_find_nearest_strong<<<g.fg, g.fb, 0, s>>>(g.full));
+    PM_LAUNCHED("k_find_nearest_strong", s);
+    k_weak_list<<<g.fg, g.fb, 0, s>>>(g.full);
+    PM_LAUNCHED("k_weak_list", s);
+    DPE_TIMED(ctx, KID_GEN_NEIGHBOURS, s, k_gen_neighbours<<<g.gn, 128, 0, s>>>(g.gneigh));
+    PM_LAUNCHED("k_gen_neighbours", s);
+    DPE_TIMED(ctx, KID_NEIGHBOUR_UPDATE, s, k_neighbour_update<<<g.fg, g.fb, 0, s>>>(g.full));
+    PM_LAUNCHED("k_neighbour_update", s);
     // WEAK pixels per colour, in raster order; the states are final for the iterations
     for (int b = 0; b < n; ++b) {
       const PMArgs &a = ps[b].a;
@@ -742,7 +755,7 @@ int pm_run_problems(dpe_ctx *ctx, const dpe_problem *const *problems, int n, dpe
   std::vector<ProblemState> ps(n);
   unsigned long long *counters = A.get<unsigned long long>("counters", 2 * KID_COUNT);
   PMArgs *d_args = A.get<PMArgs>("pm_args", n);
-  int *d_start = n > 1 ? A.get<int>("batch_start", 6 * (n + 1)) : nullptr;
+  int *d_start = n > 1 ? A.get<int>("batch_start", 7 * (n + 1)) : nullptr;
   if (!counters || !d_args || (n > 1 && !d_start)) return DPE_ERR_OUT_OF_MEMORY;
   if (ctx->count_evals) DPE_TRY(cudaMemsetAsync(counters, 0, 16 * KID_COUNT, s));
   for (int b = 0; b < n; ++b) {
@@ -776,7 +789,7 @@ int pm_run_problems(dpe_ctx *ctx, const dpe_problem *const *problems, int n, dpe
   if (n == 1) {
     const PMArgs &a = ps[0].a;
     const Launch one{d_args, nullptr, 1};
-    g.full = g.half = g.prep = g.eval = g.coop = g.sweep = one;
+    g.full = g.half = g.prep = g.eval = g.coop = g.sweep = g.gneigh = one;
     g.sg = sweep_grid(a.W, a.H);
     g.fg = full_grid(a.W, a.H);
     g.hg = half_grid(a.W, a.H);
@@ -785,9 +798,10 @@ int pm_run_problems(dpe_ctx *ctx, const dpe_problem *const *problems, int n, dpe
     g.lr_smem = local_refine_smem_bytes(a.N - 1);
     g.gp = list_grid(ctx, (long long)ps[0].wcap);
     g.ge = list_grid(ctx, (long long)ps[0].wcap * 10 * (a.N - 1));
+    g.gn = list_grid(ctx, (long long)ps[0].L * 8);
   } else {
     // the problems' grids laid end to end: prefix tables per grid kind
-    std::vector<int> start(6 * (n + 1), 0);
+    std::vector<int> start(7 * (n + 1), 0);
     for (int b = 0; b < n; ++b) {
       const PMArgs &a = ps[b].a;
       const dim3 f = full_grid(a.W, a.H), h = half_grid(a.W, a.H), cg = coop_grid(a.W, a.H);
@@ -801,6 +815,7 @@ int pm_run_problems(dpe_ctx *ctx, const dpe_problem *const *problems, int n, dpe
       start[2 * (n + 1) + b + 1] = start[2 * (n + 1) + b] + (int)list_grid(ctx, (long long)ps[b].wcap);
       start[3 * (n + 1) + b + 1] =
           start[3 * (n + 1) + b] + (int)list_grid(ctx, (long long)ps[b].wcap * 10 * (a.N - 1));
+      start[6 * (n + 1) + b + 1] = start[6 * (n + 1) + b] + (int)list_grid(ctx, (long long)ps[b].L * 8);
     }
     DPE_TRY(cudaMemcpyAsync(d_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     g.full = Launch{d_args, d_start + 0 * (n + 1), n};
@@ -815,6 +830,8 @@ int pm_run_problems(dpe_ctx *ctx, const dpe_problem *const *problems, int n, dpe
     g.hg = dim3(start[1 * (n + 1) + n]);
     g.gp = (unsigned)start[2 * (n + 1) + n];
     g.ge = (unsigned)start[3 * (n + 1) + n];
+    g.gneigh = Launch{d_args, d_start + 6 * (n + 1), n};
+    g.gn = (unsigned)start[6 * (n + 1) + n];
     // blocks keep the single-problem shapes (16x8 full, 32x4 half): only the block index is 1D
   }
   DPE_TRY(cudaEventRecord(ctx->ev0, s));

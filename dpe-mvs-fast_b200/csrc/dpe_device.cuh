@@ -70,6 +70,7 @@ struct PMArgs {
   uint8_t *reliable;
   const uint8_t *edge;
   const uint8_t *edge_low;
+  const uint8_t *edge_dist;  // lowW*lowH: 1 where edge_low has no edge within a line's longest walk; null: unknown
   const int32_t *label;
   int32_t *nmap;
   int32_t *radius;

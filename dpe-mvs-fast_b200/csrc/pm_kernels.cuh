@@ -195,10 +195,8 @@ __device__ __forceinline__ void find_nearest_strong_pixel(const PMArgs &a, int p
   }
   a.nearest[center] = res;
 }
-// Resident blocks requested for the one-thread-per-pixel searches (nearest strong point,
-// GenNeighbours, the plane fit): measured on the 10-view 1600x1200 schedule with fixed 16x8
-// blocks, 6 blocks (80 registers) make GenNeighbours 9 % faster than its unbounded 104 registers
-// (4 blocks) and 4 % faster than 8 blocks (64 registers, more stack traffic).
+// Resident blocks requested for the one-thread-per-pixel searches (the nearest strong point and
+// the plane fit), 80 registers each.
 #ifndef DPE_LATENCY_MIN_BLOCKS
 #define DPE_LATENCY_MIN_BLOCKS 6
 #endif
@@ -216,43 +214,91 @@ __global__ void __launch_bounds__(128, DPE_LATENCY_MIN_BLOCKS) k_find_nearest_st
 __device__ __forceinline__ uint8_t edge_at(const PMArgs &a, long idx) {
   return (idx >= 0 && idx < (long)a.W * a.H) ? a.edge[idx] : (uint8_t)0;
 }
-__device__ __forceinline__ uint8_t edge_low_at(const PMArgs &a, long idx) {
-  return (idx >= 0 && idx < (long)a.lowW * a.lowH) ? a.edge_low[idx] : (uint8_t)0;
+
+// Where the low-resolution edge map has an edge within `radius` (chessboard distance): first along the
+// rows (out: 1 where none), then the columns of that.
+__global__ void k_edge_clear_rows(const uint8_t *__restrict__ edge, int w, int h, int radius, uint8_t *__restrict__ out) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= w || y >= h) return;
+  uint8_t clear = 1;
+  for (int k = max(x - radius, 0); k <= min(x + radius, w - 1); ++k)
+    if (edge[(size_t)y * w + k]) clear = 0;
+  out[(size_t)y * w + x] = clear;
+}
+__global__ void k_edge_clear_cols(const uint8_t *__restrict__ rows, int w, int h, int radius, uint8_t *__restrict__ out) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= w || y >= h) return;
+  uint8_t clear = 1;
+  for (int k = max(y - radius, 0); k <= min(y + radius, h - 1); ++k)
+    if (!rows[(size_t)k * w + x]) clear = 0;
+  out[(size_t)y * w + x] = clear;
 }
 
-// BresenhamLine (DPE.cu:162-248); out-of-image linear indices read 0.
-__device__ bool bresenham(const PMArgs &a, int ax, int ay, int bx, int by) {
-  if (edge_at(a, (long)ax + (long)ay * a.W) || edge_at(a, (long)bx + (long)by * a.W)) return false;
-  const float scale_x = 1.0f * a.lowW / (float)a.W;
-  const float scale_y = 1.0f * a.lowH / (float)a.H;
-  const int h = a.lowH, w = a.lowW;
-  const int max_step = a.P.high_res_img ? (int)round(cvmax(h, w) / 60.0) : cvmax(h, w);
-  for (int pass = 0; pass < 2; ++pass) {
-    const int fx = pass == 0 ? bx : ax, fy = pass == 0 ? by : ay;
-    const int tx = pass == 0 ? ax : bx, ty = pass == 0 ? ay : by;
-    int x0 = (int)cvmin(roundf(fx * scale_x), (float)(w - 1));
-    int y0 = (int)cvmin(roundf(fy * scale_y), (float)(h - 1));
-    const int x1 = (int)cvmin(roundf(tx * scale_x), (float)(w - 1));
-    const int y1 = (int)cvmin(roundf(ty * scale_y), (float)(h - 1));
-    const int dx = abs(x1 - x0), sx = x0 < x1 ? 1 : -1;
-    const int dy = abs(y1 - y0), sy = y0 < y1 ? 1 : -1;
-    int err = (dx > dy ? dx : dy) / 2;
-    int step = 0;
-    bool tagx = true, tagy = true;
-    while (tagx || tagy) {
-      if (x0 == x1) tagx = false;
-      if (y0 == y1) tagy = false;
-      const int e2 = err;
-      if (e2 > -dx) { err -= dy; x0 += sx; }
-      if (e2 < dy) { err += dx; y0 += sy; }
-      if (edge_low_at(a, (long)x0 + (long)y0 * w)) return true;
-      step += 1;
-      if (step >= max_step) break;
-    }
+// BresenhamLine (DPE.cu:162-248); out-of-image linear indices read 0.  A point's part (its place in the
+// low-resolution edge map, and whether it lies on an edge itself) is taken once per point.
+struct LinePoint {
+  short x, y;   // in the low-resolution map
+  uint8_t on;     // on an edge of the full-resolution map
+  uint8_t clear;  // no edge within max_step of it: a walk that starts here meets none
+};
+struct LineMap {
+  float scale_x, scale_y;
+  int w, h, max_step;
+};
+__device__ __forceinline__ LineMap line_map(const PMArgs &a) {
+  LineMap m;
+  m.scale_x = 1.0f * a.lowW / (float)a.W;
+  m.scale_y = 1.0f * a.lowH / (float)a.H;
+  m.w = a.lowW;
+  m.h = a.lowH;
+  m.max_step = a.P.high_res_img ? (int)round(cvmax(m.h, m.w) / 60.0) : cvmax(m.h, m.w);
+  return m;
+}
+__device__ __forceinline__ LinePoint line_point(const PMArgs &a, const LineMap &m, int x, int y) {
+  LinePoint p;
+  p.x = (short)(int)cvmin(roundf(x * m.scale_x), (float)(m.w - 1));
+  p.y = (short)(int)cvmin(roundf(y * m.scale_y), (float)(m.h - 1));
+  p.on = edge_at(a, (long)x + (long)y * a.W) ? 1 : 0;
+  // A step moves one place at most in x and in y, so max_step steps stay within that distance.  Near
+  // the left and right borders a walk may pass the border by a step, where its linear index reads the
+  // neighbouring row: such walks are always made.
+  p.clear = a.edge_dist && p.x >= m.max_step && p.x + m.max_step < m.w && a.edge_dist[p.x + p.y * m.w] ? 1 : 0;
+  return p;
+}
+// One walk from (x0, y0) towards (x1, y1).  Out of line: the callers' loops stay in the instruction cache.
+#ifdef __CUDA_ARCH__
+__device__ __noinline__
+#else
+inline
+#endif
+bool line_walk(const uint8_t *edge_low, int w, int h, int max_step, int x0, int y0, int x1, int y1) {
+  const int dx = abs(x1 - x0), sx = x0 < x1 ? 1 : -1;
+  const int dy = abs(y1 - y0), sy = y0 < y1 ? 1 : -1;
+  int err = (dx > dy ? dx : dy) / 2;
+  int step = 0;
+  bool tagx = true, tagy = true;
+  const long n = (long)w * h;
+  while (tagx || tagy) {
+    if (x0 == x1) tagx = false;
+    if (y0 == y1) tagy = false;
+    const int e2 = err;
+    if (e2 > -dx) { err -= dy; x0 += sx; }
+    if (e2 < dy) { err += dx; y0 += sy; }
+    const long idx = (long)x0 + (long)y0 * w;
+    if (idx >= 0 && idx < n && edge_low[idx]) return true;
+    step += 1;
+    if (step >= max_step) break;
   }
   return false;
 }
-
+__device__ __forceinline__ bool line_blocked(const PMArgs &a, const LineMap &m, LinePoint A, LinePoint B) {
+  if (A.on || B.on) return false;
+  for (int pass = 0; pass < 2; ++pass) {  // from B to A, then from A to B
+    const LinePoint s = pass == 0 ? B : A, t = pass == 0 ? A : B;
+    if (!s.clear && line_walk(a.edge_low, m.w, m.h, m.max_step, s.x, s.y, t.x, t.y)) return true;
+  }
+  return false;
+}
 // PointinTriangle (DPE.cu:139-160)
 __device__ __forceinline__ bool point_in_triangle(short2 A, short2 B, short2 C, int px, int py) {
   const float2 AB = make_float2(B.x - A.x, B.y - A.y), BC = make_float2(C.x - B.x, C.y - B.y), CA = make_float2(A.x - C.x, A.y - C.y);
@@ -274,37 +320,133 @@ __device__ __forceinline__ void sort_small(float *d, int n) {
 }
 
 // ------------------------------------------------------------------ GenNeighbours (DPE.cu:2107-2467)
-__device__ __forceinline__ void gen_neighbours_pixel(const PMArgs &a, int px, int py) {
+// A group of kGnLanes threads works on one WEAK pixel.  The reference's thread searches 32 rays by
+// random tries and then runs up to 200 RANSAC rounds, each a test of three points against up to 64;
+// one thread per pixel left three quarters of a warp's lanes idle (only WEAK pixels have work) and
+// kept its 2.3 KB of points in local memory.  Here the lanes split
+//   * the tries of a ray: try t of a ray draws the pixel's numbers 4t..4t+3 from where the ray began
+//     (the stream is counter-based), so the lanes make the next tries side by side and the first that
+//     succeeds ends the ray with the counter behind it, as the sequential loop does;
+//   * the label boundary's points;
+//   * RANSAC rounds: round r draws numbers 3r..3r+2, and its tests (three distinct points, the triangle,
+//     the edge lines, the normals, the plane) do not depend on earlier rounds; the lanes prepare the
+//     next rounds side by side, which are then taken in order under the current state;
+//   * the points' residuals of a round, and the ranks that replace its sorts.
+// Random numbers are made ahead into shared memory, each once; lines that start where no edge is near
+// are not walked (k_edge_clear_*).
+// Bound by instruction issue (0.55 of the slots; 34 k warp instructions per WEAK pixel, half of them the
+// residuals).  Measured, one 1600x1200 view with 403 k WEAK pixels: 126.7 ms one thread per pixel, 43.3
+// with 16 lanes, 29.1 with the numbers ahead and the walks skipped; 32 lanes 35.4, 8 lanes 46.8 (before
+// those two) against 43.1; one 400x300 view 2.0 -> 0.13 ms.
+// Host builds of this source run it with one lane.
+#ifdef __CUDA_ARCH__
+#ifndef DPE_GN_LANES
+#define DPE_GN_LANES 16
+#endif
+constexpr int kGnLanes = DPE_GN_LANES;
+#else
+constexpr int kGnLanes = 1;
+#endif
+constexpr int kGnPoints = 64;
+constexpr int kGnAhead = 4 * kGnLanes;                     // numbers that one step of the group may use
+constexpr int kGnDraws = 2 * kGnAhead;
+struct GnGroup {
+  int lane;
+#ifdef __CUDA_ARCH__
+  int shift;
+  unsigned mask;
+  __device__ __forceinline__ unsigned ballot(bool p) const {
+    return (__ballot_sync(mask, p) & mask) >> shift;
+  }
+  template <class T> __device__ __forceinline__ T from(T v, int src) const { return __shfl_sync(mask, v, src, kGnLanes); }
+  __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+  static __device__ __forceinline__ int first(unsigned b) { return __ffs(b) - 1; }
+  static __device__ __forceinline__ int count(unsigned b) { return __popc(b); }
+#else
+  unsigned ballot(bool p) const { return p ? 1u : 0u; }
+  template <class T> T from(T v, int) const { return v; }
+  void sync() const {}
+  static int first(unsigned) { return 0; }
+  static int count(unsigned b) { return (int)b; }
+#endif
+};
+// The points of one pixel.
+struct GnPoints {
+  union {
+    short2 pts[kGnPoints];  // by ray (0-31) and label boundary (32-63), while they are found
+    float res[kGnPoints];   // then the residuals of a round, or the final weights
+  };
+  short2 sv[kGnPoints];     // the found points in order
+  float2 ray[kGnPoints];    // ((x - cx) / fx, (y - cy) / fy)
+  float3 pos[kGnPoints], nrm[kGnPoints];
+  LinePoint line[kGnPoints];
+  uint32_t draws[kGnDraws];  // the pixel's next random numbers, number n at n % kGnDraws
+};
+// Per-call constants of the search.
+struct GnCall {
+  float cos_a, sin_a, thr;
+  int shift_range;
+  LineMap map;
+};
+__device__ __forceinline__ GnCall gn_call(const PMArgs &a) {
+  GnCall k;
+  const float angle = 45.0f / a.P.rotate_time;
+  k.cos_a = (float)cos(angle * 3.14159265358979323846 / 180.f);
+  k.sin_a = (float)sin(angle * 3.14159265358979323846 / 180.f);
+  k.thr = (float)cos((angle / 2.0f) * 3.14159265358979323846 / 180.0f);
+  k.shift_range = cvmax((int)(tan((angle / 2.0f) * 3.14159265358979323846 / 180.0f) * 20), 1);
+  k.map = LineMap{0.f, 0.f, 0, 0, 0};
+  if (a.P.use_limit) k.map = line_map(a);
+  return k;
+}
+// Step m of a ray: 2, 4, 8, 16, 32, then 25 more each (radius = min(2 radius, radius + 25)).
+__device__ __forceinline__ int gn_radius(int m) { return m < 5 ? 2 << m : 32 + 25 * (m - 4); }
+
+// Makes the numbers ctr .. ctr + kGnAhead - 1 available in S.draws; numbers up to `end` are there.  Each is
+// computed once, by one lane, however many tries turn out to be needed.
+__device__ __forceinline__ void gn_fill(const PMArgs &a, const GnGroup &g, GnPoints &S, int center, uint32_t ctr,
+                                        uint32_t &end) {
+  if ((int)(end - ctr) >= kGnAhead) return;
+  g.sync();  // the numbers being replaced have been read
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t n = end + (uint32_t)(k * kGnLanes + g.lane);
+    S.draws[n % kGnDraws] = philox_word0(n, (uint32_t)center, 0x5EEDu, 0u, a.key[0], a.key[1]);
+  }
+  end += kGnAhead;
+  g.sync();
+}
+
+__device__ __forceinline__ void gen_neighbours_pixel(const PMArgs &a, const GnCall &K, const GnGroup &g, GnPoints &S,
+                                                     int px, int py) {
   const int W = a.W, H = a.H, center = px + py * W;
-  if (a.weak[center] != DPE_WEAK) return;
-  constexpr int kMaxPts = 64;
   const int margin = 6;
   const float depth_diff = a.P.depth_max - a.P.depth_min;
   const dpe_camera &cam = a.cam[0];
-  Rng rng = make_rng(a, center);
+  uint32_t ctr = G(a.rng_ctr, center, (long long)W * H, 106), end = ctr;
+  auto draw = [&](uint32_t n) { return S.draws[n % kGnDraws]; };
   short2 *nbs = &a.neigh[(size_t)a.nmap[center] * kNeighbours];
-  nbs[0] = make_short2(px, py);
-  for (int i = 1; i < kNeighbours; ++i) nbs[i] = make_short2(-1, -1);
-  short2 pts[kMaxPts];
+  for (int i = g.lane; i < kNeighbours; i += kGnLanes) nbs[i] = i == 0 ? make_short2(px, py) : make_short2(-1, -1);
   uint64_t valid = 0;
   int odi = -1, npts = 0;
   const int rt = a.P.rotate_time;
-  const float angle = 45.0f / rt;
-  const float cos_a = (float)cos(angle * 3.14159265358979323846 / 180.f);
-  const float sin_a = (float)sin(angle * 3.14159265358979323846 / 180.f);
-  const float thr = (float)cos((angle / 2.0f) * 3.14159265358979323846 / 180.0f);
-  const int shift_range = cvmax((int)(tan((angle / 2.0f) * 3.14159265358979323846 / 180.0f) * 20), 1);
   const float ransac_thr = a.P.ransac_threshold * depth_diff;
   bool edge_limit = false;
   if (a.P.use_limit) {
     edge_limit = true;
     if (a.P.use_edge) {
       const float cv = a.complexity[center];
-      const float rp = rng.uniform() - FLT_EPSILON;
+      gn_fill(a, g, S, center, ctr, end);
+      const float rp = (float)((draw(ctr++) >> 8) + 1u) * (1.0f / 16777216.0f) - FLT_EPSILON;
+      g.sync();  // every lane has read the complexity
       if (rp < cv) edge_limit = false;
-      else a.complexity[center] = cvmax(0.99f, cv);
+      else if (g.lane == 0) a.complexity[center] = cvmax(0.99f, cv);
     }
   }
+  LinePoint here{0, 0, 0};
+  if (edge_limit) here = line_point(a, K.map, px, py);
   for (int odx = -1; odx <= 1; ++odx)
     for (int ody = -1; ody <= 1; ++ody) {
       if (odx == 0 && ody == 0) continue;
@@ -313,208 +455,345 @@ __device__ __forceinline__ void gen_neighbours_pixel(const PMArgs &a, int px, in
       odi++;
       for (int ri = 0; ri < rt; ++ri) {
         const int di = odi * 4 + ri;
-        for (int radius = 2; radius <= 4096; radius = cvmin(radius * 2, radius + 25)) {
+        for (int t0 = 0;; t0 += kGnLanes) {
+          gn_fill(a, g, S, center, ctr, end);
+          const int t = t0 + g.lane;
+          const int radius = gn_radius(t >> 2);
           const float2 tp = make_float2(px + od.x * radius, py + od.y * radius);
-          if (tp.x < 0 || tp.y < 0 || tp.x >= W || tp.y >= H) break;
-          for (int k = 0; k < 4; ++k) {
-            uint32_t sgn = (rng.u32() % 2 == 0) ? 1u : 0xFFFFFFFFu;
-            const int rxs = (int)((sgn * rng.u32()) % (uint32_t)shift_range);
-            sgn = (rng.u32() % 2 == 0) ? 1u : 0xFFFFFFFFu;
-            const int rys = (int)((sgn * rng.u32()) % (uint32_t)shift_range);
+          const bool out = radius > 4096 || tp.x < 0 || tp.y < 0 || tp.x >= W || tp.y >= H;
+          bool ok = !out;
+          short2 nb = make_short2(-1, -1);
+          if (ok) {
+            const uint32_t c0 = ctr + 4u * (uint32_t)g.lane;
+            uint32_t sgn = (draw(c0) % 2 == 0) ? 1u : 0xFFFFFFFFu;
+            const int rxs = (int)((sgn * draw(c0 + 1)) % (uint32_t)K.shift_range);
+            sgn = (draw(c0 + 2) % 2 == 0) ? 1u : 0xFFFFFFFFu;
+            const int rys = (int)((sgn * draw(c0 + 3)) % (uint32_t)K.shift_range);
             float2 dir = make_float2(od.x * 20 + rxs, od.y * 20 + rys);
             normalize2(&dir);
-            short2 nb = make_short2((short)(int)(px + dir.x * radius), (short)(int)(py + dir.y * radius));
-            if (nb.x < margin || nb.y < margin || nb.x >= W - margin || nb.y >= H - margin) continue;
-            int nbc = nb.x + nb.y * W;
-            if (a.weak[nbc] != DPE_STRONG) {
-              nb = a.nearest[nbc];
-              if (nb.x == -1 || nb.y == -1) continue;
-              nbc = nb.x + nb.y * W;
+            nb = make_short2((short)(int)(px + dir.x * radius), (short)(int)(py + dir.y * radius));
+            ok = !(nb.x < margin || nb.y < margin || nb.x >= W - margin || nb.y >= H - margin);
+            if (ok) {
+              const int nbc = nb.x + nb.y * W;
+              if (a.weak[nbc] != DPE_STRONG) {
+                nb = a.nearest[nbc];
+                ok = !(nb.x == -1 || nb.y == -1);
+              }
             }
-            float2 td = make_float2((float)(nb.x - px), (float)(nb.y - py));
-            normalize2(&td);
-            const float ca = td.x * od.x + td.y * od.y;
-            if (ca > thr && (!edge_limit || !bresenham(a, px, py, nb.x, nb.y))) {
-              pts[di] = nb; valid |= 1ull << di; npts++;
-              break;
+            if (ok) {
+              float2 td = make_float2((float)(nb.x - px), (float)(nb.y - py));
+              normalize2(&td);
+              const float ca = td.x * od.x + td.y * od.y;
+              ok = ca > K.thr && (!edge_limit || !line_blocked(a, K.map, here, line_point(a, K.map, nb.x, nb.y)));
             }
           }
-          if ((valid >> di) & 1ull) break;
+          const unsigned hit = g.ballot(ok), over = g.ballot(out);
+          if (hit) {
+            const int f = g.first(hit);
+            if (g.lane == f) S.pts[di] = nb;
+            valid |= 1ull << di;
+            npts++;
+            ctr += 4u * (uint32_t)(f + 1);
+            break;
+          }
+          if (over) {
+            ctr += 4u * (uint32_t)g.first(over);
+            break;
+          }
+          ctr += 4u * kGnLanes;
         }
-        float2 rd = make_float2(od.x * cos_a - od.y * sin_a, od.x * sin_a + od.y * cos_a);
+        float2 rd = make_float2(od.x * K.cos_a - od.y * K.sin_a, od.x * K.sin_a + od.y * K.cos_a);
         normalize2(&rd);
         od = rd;
       }
     }
   int ext = 31;
   if (a.P.use_label && a.label[center] > 0) {
+    // 2 rt points per pair of opposite directions: the first gets 2 rt - 1 steps, the second one (the
+    // reference's min(1, max(2 rt - 1, ...)) is always 1: quirk Q5)
     const short2 *lb = &a.lab_bound[(size_t)a.nmap[center] * 8];
-    float bd[8];
-    int ds[8];
-    for (int i = 0; i < 8; ++i) {
-      const short2 b = lb[i];
-      float dist = 0.0f;
-      if (b.x != -1 && b.y != -1) {
-        const double ddx = (double)(px - b.x), ddy = (double)(py - b.y);
-        dist = (float)sqrt(ddx * ddx + ddy * ddy);
-        if (i >= 4) dist = (float)(dist / sqrt(2.0));
-      }
-      bd[i] = dist;
-      if (i % 2 == 1) {
-        const float od2 = bd[i - 1];
-        const int step = cvmin(1, cvmax(2 * rt - 1, (int)(2 * rt * dist / (dist + od2))));  // quirk Q5
-        ds[i - 1] = 2 * rt - step;
-        ds[i] = step;
-      }
-    }
-    for (int i = 0; i < 8; ++i) {
-      const float dist = bd[i];
-      const int gap = ds[i] + 1;
-      const int step_len = cvmax(1, (int)floor(1.0 * dist / gap));
-      for (int s = 1; s <= ds[i]; ++s) {
-        short2 nb = make_short2((short)(px + s * step_len * kDir[i][0]), (short)(py + s * step_len * kDir[i][1]));
-        if (nb.x < margin || nb.y < margin || nb.x >= W - margin || nb.y >= H - margin) continue;
-        int nbc = nb.x + nb.y * W;
-        if (a.weak[nbc] != DPE_STRONG) {
-          nb = a.nearest[nbc];
-          if (nb.x == -1 || nb.y == -1) continue;
-          nbc = nb.x + nb.y * W;
+    const int total = 8 * rt;
+    for (int e0 = 0; e0 < total; e0 += kGnLanes) {
+      const int e = e0 + g.lane;
+      bool ok = e < total;
+      short2 nb = make_short2(-1, -1);
+      if (ok) {
+        const int k = e / (2 * rt), r = e - k * 2 * rt;
+        const int i = r < 2 * rt - 1 ? 2 * k : 2 * k + 1, steps = i & 1 ? 1 : 2 * rt - 1, s = i & 1 ? 1 : r + 1;
+        const short2 b = lb[i];
+        float dist = 0.0f;
+        if (b.x != -1 && b.y != -1) {
+          const double ddx = (double)(px - b.x), ddy = (double)(py - b.y);
+          dist = (float)sqrt(ddx * ddx + ddy * ddy);
+          if (i >= 4) dist = (float)(dist / sqrt(2.0));
         }
-        if (a.label[nbc] != 0 && a.label[nbc] != a.label[center]) continue;
-        ext++;
-        pts[ext] = nb; valid |= 1ull << ext; npts++;
+        const int gap = steps + 1;
+        const int step_len = cvmax(1, (int)floor(1.0 * dist / gap));
+        nb = make_short2((short)(px + s * step_len * kDir[i][0]), (short)(py + s * step_len * kDir[i][1]));
+        ok = !(nb.x < margin || nb.y < margin || nb.x >= W - margin || nb.y >= H - margin);
+        int nbc = ok ? nb.x + nb.y * W : 0;
+        if (ok && a.weak[nbc] != DPE_STRONG) {
+          nb = a.nearest[nbc];
+          ok = !(nb.x == -1 || nb.y == -1);
+          nbc = ok ? nb.x + nb.y * W : 0;
+        }
+        if (ok) ok = !(a.label[nbc] != 0 && a.label[nbc] != a.label[center]);
       }
+      const unsigned hit = g.ballot(ok);
+      if (ok) S.pts[ext + 1 + g.count(hit & ((1u << g.lane) - 1u))] = nb;
+      const int m = g.count(hit);
+      for (int q = 0; q < m; ++q) valid |= 1ull << (ext + 1 + q);
+      ext += m;
+      npts += m;
     }
   }
-  if (npts <= 3) { a.reliable[center] = 0; a.rng_ctr[center] = rng.ctr; return; }
+  if (npts <= 3) {
+    if (g.lane == 0) {
+      a.reliable[center] = 0;
+      a.rng_ctr[center] = ctr;
+    }
+    g.sync();  // the points' storage is free for the group's next pixel
+    return;
+  }
 
-  short2 sv[kMaxPts];
-  float3 sv3[kMaxPts], svn[kMaxPts];
-  int vc = 0;
+  // the found points in order: point i of the valid ones is lane i's, i + kGnLanes's, ...
+  g.sync();
   float X[3];
   point3d(cam, px, py, a.plane[center].w, X);
   const float cwz = X[2];
-  for (int i = 0; i < kMaxPts; ++i) {
-    if ((valid >> i) & 1ull) {
-      const short2 sp = pts[i];
-      const int spc = sp.x + sp.y * W;
-      const float4 spl = a.plane[spc];
-      sv[vc] = sp;
-      point3d(cam, sp.x, sp.y, spl.w, X);
-      sv3[vc] = make_float3(X[0], X[1], X[2]);
-      const float4 n4 = normal_to_ref(cam, spl);
-      svn[vc] = make_float3(n4.x, n4.y, n4.z);
-      vc++;
+  const int vc = npts;
+  {
+    int at = 0;
+    for (int i = 0; i < kGnPoints; ++i) {
+      if (!((valid >> i) & 1ull)) continue;
+      if (at % kGnLanes == g.lane) {
+        const short2 sp = S.pts[i];
+        const float4 spl = a.plane[sp.x + sp.y * W];
+        S.sv[at] = sp;
+        point3d(cam, sp.x, sp.y, spl.w, X);
+        S.pos[at] = make_float3(X[0], X[1], X[2]);
+        const float4 n4 = normal_to_ref(cam, spl);
+        S.nrm[at] = make_float3(n4.x, n4.y, n4.z);
+        S.ray[at] = make_float2((sp.x - cam.K[2]) / cam.K[0], (sp.y - cam.K[5]) / cam.K[4]);
+        if (edge_limit) S.line[at] = line_point(a, K.map, sp.x, sp.y);
+      }
+      ++at;
     }
   }
+  g.sync();
+  const float cfx = (px - cam.K[2]) / cam.K[0], cfy = (py - cam.K[5]) / cam.K[4];
   float4 best = make_float4(0, 0, 0, 0);
   bool has_valid = false;
   {
     int iteration = 50, max_iter = a.P.high_res_img ? 200 : 125, max_count = 3;
     float min_cost = FLT_MAX;
-    float residuals[kMaxPts];
-    for (int i = 0; i < kMaxPts; ++i) residuals[i] = 0.0f;
     float tthr = ransac_thr;
     bool has_consist = false;
     bool must_tri = (a.P.use_label && a.label[center] > 0 && edge_limit) ? false : true;
     while (iteration > 0 && max_iter > 0) {
-      max_iter--;
-      const int ia = (int)(rng.u32() % (uint32_t)vc);
-      const int ib = (int)(rng.u32() % (uint32_t)vc);
-      const int ic = (int)(rng.u32() % (uint32_t)vc);
-      if (ia == ib || ib == ic || ia == ic) continue;
-      if (must_tri && !point_in_triangle(sv[ia], sv[ib], sv[ic], px, py)) continue;
-      if (edge_limit) {
-        if (bresenham(a, sv[ia].x, sv[ia].y, sv[ib].x, sv[ib].y) || bresenham(a, sv[ib].x, sv[ib].y, sv[ic].x, sv[ic].y) ||
-            bresenham(a, sv[ic].x, sv[ic].y, sv[ia].x, sv[ia].y))
-          continue;
-      }
-      bool nc = false;
-      if (a.P.geom_consistency && edge_limit) {
-        const float3 AN = svn[ia], BN = svn[ib], CN = svn[ic];
-        nc = true;
-        if ((double)(AN.x * BN.x + AN.y * BN.y + AN.z * BN.z) < 0.8660254 ||
-            (double)(AN.x * CN.x + AN.y * CN.y + AN.z * CN.z) < 0.8660254 ||
-            (double)(BN.x * CN.x + BN.y * CN.y + BN.z * CN.z) < 0.8660254)
-          nc = false;
-        if (has_consist && !nc) continue;
-      }
-      iteration--;
-      const float3 A = sv3[ia], B = sv3[ib], C = sv3[ic];
-      const float3 AC = make_float3(A.x - C.x, A.y - C.y, A.z - C.z), BC = make_float3(B.x - C.x, B.y - C.y, B.z - C.z);
-      float4 cr;
-      cr.x = AC.y * BC.z - BC.y * AC.z;
-      cr.y = -(AC.x * BC.z - BC.x * AC.z);
-      cr.z = AC.x * BC.y - BC.x * AC.y;
-      if ((cr.x == 0 && cr.y == 0 && cr.z == 0) || isnan(cr.x) || isnan(cr.y) || isnan(cr.z)) continue;
-      normalize3(&cr);
-      cr.w = -(cr.x * A.x + cr.y * A.y + cr.z * A.z);
-      int tcount = 0;
-      float sdist = 0.0f;
-      for (int s = 0; s < vc; ++s) {
-        const float fx = (sv[s].x - cam.K[2]) / cam.K[0];
-        const float fy = (sv[s].y - cam.K[5]) / cam.K[4];
-        const float fd = -cr.w / (cr.x * fx + cr.y * fy + cr.z);
-        const float dist = fabsf(fd - sv3[s].z);
-        residuals[s] = dist;
-        if (dist < tthr) { tcount++; sdist += dist; }
-      }
-      if (tcount < 6) continue;
-      const float fx = (px - cam.K[2]) / cam.K[0], fy = (py - cam.K[5]) / cam.K[4];
-      if (tcount > max_count) {
-        if (!must_tri && point_in_triangle(sv[ia], sv[ib], sv[ic], px, py)) must_tri = true;
-        if (!has_consist && nc) has_consist = true;
-        const float fd = -cr.w / (cr.x * fx + cr.y * fy + cr.z);
-        const float cd = fabsf(fd - cwz);
-        best = cr; max_count = tcount; sdist /= tcount; min_cost = cd; has_valid = true;
-        if (tthr > (a.P.high_res_img ? 0.05 : 0.005)) {
-          sort_small(residuals, vc);
-          if (tthr < residuals[kNeighbours]) continue;
-          tthr = (float)(residuals[kNeighbours] - 1e-6);
-          tcount = 0;
-          for (int s = 0; s < vc; ++s) {
-            if (residuals[s] < tthr) tcount++;
-            else break;
-          }
-          max_count = tcount;
+      gn_fill(a, g, S, center, ctr, end);
+      // the next rounds, one per lane: what a round's tests see, whatever the state
+      bool ok = g.lane < max_iter, tri = false, nc = false, flat = true;
+      float4 cr = make_float4(0, 0, 0, 0);
+      if (ok) {
+        const uint32_t c0 = ctr + 3u * (uint32_t)g.lane;
+        const int ia = (int)(draw(c0) % (uint32_t)vc);
+        const int ib = (int)(draw(c0 + 1) % (uint32_t)vc);
+        const int ic = (int)(draw(c0 + 2) % (uint32_t)vc);
+        ok = !(ia == ib || ib == ic || ia == ic);
+        if (ok) {
+          tri = point_in_triangle(S.sv[ia], S.sv[ib], S.sv[ic], px, py);
+          ok = tri || !must_tri;
         }
-      } else if (tcount == max_count) {
-        if (!must_tri && point_in_triangle(sv[ia], sv[ib], sv[ic], px, py)) must_tri = true;
-        const float fd = -cr.w / (cr.x * fx + cr.y * fy + cr.z);
-        const float cd = fabsf(fd - cwz);
-        if (cd < min_cost) { best = cr; max_count = tcount; sdist /= tcount; min_cost = cd; }
+        if (edge_limit) {
+          int i = ia, j = ib;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+          for (int k = 0; ok && k < 3; ++k) {
+            ok = !line_blocked(a, K.map, S.line[i], S.line[j]);
+            i = j;
+            j = k == 0 ? ic : ia;
+          }
+        }
+        if (ok) {
+          if (a.P.geom_consistency && edge_limit) {
+            const float3 AN = S.nrm[ia], BN = S.nrm[ib], CN = S.nrm[ic];
+            nc = !((double)(AN.x * BN.x + AN.y * BN.y + AN.z * BN.z) < 0.8660254 ||
+                   (double)(AN.x * CN.x + AN.y * CN.y + AN.z * CN.z) < 0.8660254 ||
+                   (double)(BN.x * CN.x + BN.y * CN.y + BN.z * CN.z) < 0.8660254);
+          }
+          const float3 A = S.pos[ia], B = S.pos[ib], C = S.pos[ic];
+          const float3 AC = make_float3(A.x - C.x, A.y - C.y, A.z - C.z), BC = make_float3(B.x - C.x, B.y - C.y, B.z - C.z);
+          cr.x = AC.y * BC.z - BC.y * AC.z;
+          cr.y = -(AC.x * BC.z - BC.x * AC.z);
+          cr.z = AC.x * BC.y - BC.x * AC.y;
+          flat = (cr.x == 0 && cr.y == 0 && cr.z == 0) || isnan(cr.x) || isnan(cr.y) || isnan(cr.z);
+          if (!flat) {
+            normalize3(&cr);
+            cr.w = -(cr.x * A.x + cr.y * A.y + cr.z * A.z);
+          }
+        }
       }
+      const unsigned b_ok = g.ballot(ok), b_tri = g.ballot(tri), b_nc = g.ballot(nc), b_flat = g.ballot(flat);
+      const int rounds = max_iter < kGnLanes ? max_iter : kGnLanes;
+      int used = rounds;  // rounds the sequential loop runs of these
+      for (unsigned todo = b_ok; todo; todo &= todo - 1) {
+        const int r = g.first(todo);
+        const bool r_tri = (b_tri >> r) & 1u, r_nc = (b_nc >> r) & 1u;
+        if (must_tri && !r_tri) continue;
+        if (a.P.geom_consistency && edge_limit && has_consist && !r_nc) continue;
+        iteration--;
+        const bool last = iteration == 0;
+        if (last) used = r + 1;
+        if (!((b_flat >> r) & 1u)) {
+          const float4 pl = make_float4(g.from(cr.x, r), g.from(cr.y, r), g.from(cr.z, r), g.from(cr.w, r));
+          int tcount = 0;
+          bool odd = false;  // a residual that is no number
+          for (int s0 = 0; s0 < vc; s0 += kGnLanes) {
+            const int s = s0 + g.lane;
+            bool in = false;
+            if (s < vc) {
+              const float fd = -pl.w / (pl.x * S.ray[s].x + pl.y * S.ray[s].y + pl.z);
+              const float dist = fabsf(fd - S.pos[s].z);
+              S.res[s] = dist;
+              in = dist < tthr;
+              if (isnan(dist)) odd = true;
+            }
+            tcount += g.count(g.ballot(in));
+          }
+          if (tcount >= 6 && tcount >= max_count) {
+            const float cd = fabsf(-pl.w / (pl.x * cfx + pl.y * cfy + pl.z) - cwz);
+            if (!must_tri && r_tri) must_tri = true;
+            if (tcount > max_count) {
+              if (!has_consist && r_nc) has_consist = true;
+              best = pl; max_count = tcount; min_cost = cd; has_valid = true;
+              if (tthr > (a.P.high_res_img ? 0.05 : 0.005)) {
+                // the tenth smallest residual (0 with fewer than ten points)
+                float r9 = 0.0f;
+                g.sync();
+                if (g.ballot(odd)) {  // the reference's insertion sort as it is
+                  if (g.lane == 0) sort_small(S.res, vc);
+                  g.sync();
+                  if (vc > kNeighbours) r9 = S.res[kNeighbours];
+                  if (!(tthr < r9)) {
+                    tthr = (float)(r9 - 1e-6);
+                    int n = 0;
+                    while (n < vc && S.res[n] < tthr) ++n;
+                    max_count = n;
+                  }
+                } else {
+                  if (vc > kNeighbours)
+                    for (int s0 = 0; s0 < vc; s0 += kGnLanes) {
+                      const int s = s0 + g.lane;
+                      int rank = -1;
+                      const float v = s < vc ? S.res[s] : 0.0f;
+                      if (s < vc) {
+                        rank = 0;
+                        for (int k = 0; k < vc; ++k) rank += S.res[k] < v || (S.res[k] == v && k < s);
+                      }
+                      const unsigned b = g.ballot(rank == kNeighbours);
+                      if (b) r9 = g.from(v, g.first(b));
+                    }
+                  if (!(tthr < r9)) {
+                    tthr = (float)(r9 - 1e-6);
+                    max_count = 0;
+                    for (int s0 = 0; s0 < vc; s0 += kGnLanes) {
+                      const int s = s0 + g.lane;
+                      max_count += g.count(g.ballot(s < vc && S.res[s] < tthr));
+                    }
+                  }
+                }
+                g.sync();  // the residuals are read; the next round overwrites them
+              }
+            } else if (cd < min_cost) {
+              best = pl; min_cost = cd;
+            }
+          }
+        }
+        if (last) break;
+      }
+      max_iter -= used;
+      ctr += 3u * (uint32_t)used;
     }
   }
-  a.rng_ctr[center] = rng.ctr;
-  if (!has_valid) { a.reliable[center] = 0; return; }
-  float weight[kMaxPts];
-  for (int i = 0; i < vc; ++i) {
-    const float fx = (sv[i].x - cam.K[2]) / cam.K[0];
-    const float fy = (sv[i].y - cam.K[5]) / cam.K[4];
-    const float fd = -best.w / (best.x * fx + best.y * fy + best.z);
-    const float dist = fabsf(fd - sv3[i].z);
-    if (dist >= ransac_thr) { sv[i] = make_short2(-1, -1); weight[i] = FLT_MAX; continue; }
-    weight[i] = dist;
+  if (g.lane == 0) a.rng_ctr[center] = ctr;
+  if (!has_valid) {
+    if (g.lane == 0) a.reliable[center] = 0;
+    g.sync();
+    return;
   }
-  for (int i = 1; i < vc; ++i) {
-    const short2 tp = sv[i];
-    const float tw = weight[i];
-    int j;
-    for (j = i; j >= 1 && tw < weight[j - 1]; j--) { sv[j] = sv[j - 1]; weight[j] = weight[j - 1]; }
-    sv[j] = tp; weight[j] = tw;
+  // the points within the threshold, nearest to the plane first (equal ones in order)
+  bool odd = false;
+  g.sync();
+  for (int s = g.lane; s < vc; s += kGnLanes) {
+    const float fd = -best.w / (best.x * S.ray[s].x + best.y * S.ray[s].y + best.z);
+    const float dist = fabsf(fd - S.pos[s].z);
+    S.res[s] = dist >= ransac_thr ? FLT_MAX : dist;
+    if (dist >= ransac_thr) S.sv[s] = make_short2(-1, -1);
+    if (isnan(dist)) odd = true;
   }
-  for (int i = 1; i < kNeighbours; ++i) nbs[i] = (i - 1 < vc) ? sv[i - 1] : make_short2(-1, -1);
-  a.reliable[center] = 1;
+  g.sync();
+  if (g.ballot(odd)) {  // a weight that is no number: the reference's insertion sort as it is
+    if (g.lane == 0) {
+      for (int i = 1; i < vc; ++i) {
+        const short2 tp = S.sv[i];
+        const float tw = S.res[i];
+        int j;
+        for (j = i; j >= 1 && tw < S.res[j - 1]; j--) { S.sv[j] = S.sv[j - 1]; S.res[j] = S.res[j - 1]; }
+        S.sv[j] = tp; S.res[j] = tw;
+      }
+      for (int i = 1; i < kNeighbours; ++i) nbs[i] = (i - 1 < vc) ? S.sv[i - 1] : make_short2(-1, -1);
+    }
+  } else {
+    for (int s = g.lane; s < vc; s += kGnLanes) {
+      const float v = S.res[s];
+      int rank = 0;
+      for (int k = 0; k < vc; ++k) rank += S.res[k] < v || (S.res[k] == v && k < s);
+      if (rank < kNeighbours - 1) nbs[1 + rank] = S.sv[s];
+    }
+  }
+  if (g.lane == 0) a.reliable[center] = 1;
+  g.sync();
 }
-// One thread per pixel of a 2D grid: the tiles keep the rays of neighbouring pixels together
-// (measured faster than a work list over the WEAK pixels).
-__global__ void __launch_bounds__(128, DPE_LATENCY_MIN_BLOCKS) k_gen_neighbours(const Launch lc) {
+// The WEAK pixels in raster order, for k_gen_neighbours: slot nmap[c] of the list is pixel c (nmap
+// counts the WEAK pixels before c).  The list lies in the buffer that the colours' lists take later.
+__global__ void k_weak_list(const Launch lc) {
   const Blk B = resolve<kGridFull>(lc);
   const PMArgs &a = *B.a;
   int px, py;
   if (!full_pixel(a, B, &px, &py)) return;
-  gen_neighbours_pixel(a, px, py);
+  const int c = px + py * a.W;
+  if (a.weak[c] == DPE_WEAK) const_cast<int *>(a.wlist[0])[a.nmap[c]] = c;
+}
+// On the device a grid of groups strides over the WEAK pixels' list; host builds of this source call it
+// per pixel.
+__global__ void __launch_bounds__(128) k_gen_neighbours(const Launch lc) {
+#ifdef __CUDA_ARCH__
+  const Blk B = resolve<kGridList>(lc);
+  const PMArgs &a = *B.a;
+  __shared__ GnPoints S[128 / kGnLanes];
+  __shared__ GnCall K;
+  if (threadIdx.x == 0) K = gn_call(a);
+  __syncthreads();
+  const int L = a.W * a.H, slot = (int)threadIdx.x / kGnLanes;
+  const int count = a.nmap[L - 1] + (a.weak[L - 1] == DPE_WEAK ? 1 : 0);
+  GnGroup g;
+  g.lane = (int)threadIdx.x % kGnLanes;
+  g.shift = ((int)threadIdx.x & 31) - g.lane;
+  g.mask = (kGnLanes == 32 ? 0xFFFFFFFFu : (1u << (kGnLanes & 31)) - 1u) << g.shift;
+  for (int i = B.x * (128 / kGnLanes) + slot; i < count; i += B.gx * (128 / kGnLanes)) {
+    const int c = a.wlist[0][i];
+    gen_neighbours_pixel(a, K, g, S[slot], c % a.W, c / a.W);
+  }
+#else
+  const Blk B = resolve<kGridFull>(lc);
+  const PMArgs &a = *B.a;
+  int px, py;
+  if (!full_pixel(a, B, &px, &py) || a.weak[px + py * a.W] != DPE_WEAK) return;
+  GnPoints S;
+  gen_neighbours_pixel(a, gn_call(a), GnGroup{0}, S, px, py);
+#endif
 }
 
 __global__ void k_neighbour_update(const Launch lc) {
@@ -1560,6 +1839,9 @@ __device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, 
   }
   short2 sp[kNeighbours - 1];
   float3 sp3[kNeighbours - 1], spn[kNeighbours - 1];
+  LinePoint line[kNeighbours - 1];
+  LineMap map{0.f, 0.f, 0, 0, 0};
+  if (edge_limit) map = line_map(a);
   int sc = 0;
   float X[3];
   for (int i = 1; i < kNeighbours; ++i) {
@@ -1572,6 +1854,7 @@ __device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, 
     point3d(cam, t.x, t.y, d, X);
     sp3[sc] = make_float3(X[0], X[1], X[2]);
     spn[sc] = make_float3(tpl.x, tpl.y, tpl.z);
+    if (edge_limit) line[sc] = line_point(a, map, t.x, t.y);
     sc++;
   }
   if (sc < 3) { a.fit_plane[center] = a.plane[center]; a.rng_ctr[center] = rng.ctr; return; }
@@ -1597,8 +1880,8 @@ __device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, 
     }
     if (must_tri && !point_in_triangle(sp[ia], sp[ib], sp[ic], px, py)) continue;
     if (edge_limit) {
-      if (bresenham(a, sp[ia].x, sp[ia].y, sp[ib].x, sp[ib].y) || bresenham(a, sp[ib].x, sp[ib].y, sp[ic].x, sp[ic].y) ||
-          bresenham(a, sp[ic].x, sp[ic].y, sp[ia].x, sp[ia].y))
+      if (line_blocked(a, map, line[ia], line[ib]) || line_blocked(a, map, line[ib], line[ic]) ||
+          line_blocked(a, map, line[ic], line[ia]))
         continue;
     }
     const float3 A = sp3[ia], B = sp3[ib], C = sp3[ic];

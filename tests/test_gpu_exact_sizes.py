@@ -53,3 +53,24 @@ def test_refine_sizes(xctx, w, hgt, views, level, geom):  # noqa: F811
     if geom:
         kw["depths"] = [np.ascontiguousarray(sc.depth[i].astype(np.float32)) for i in range(views)]
     _same(xctx.pm_run(images, cams, p, **kw), O.pm_run(images, cams, p, **kw), f"refine {w}x{hgt}x{views}")
+
+
+@pytest.mark.parametrize("rotate,high_res,label,limit,weak_share", [(1, 1, 1, 1, 0.9), (2, 0, 1, 1, 0.5),
+                                                                    (3, 1, 0, 1, 0.2), (4, 0, 0, 0, 0.6)])
+def test_neighbour_search_options(xctx, rotate, high_res, label, limit, weak_share):  # noqa: F811
+    """GenNeighbours and the plane fit: few and many rays, short and long line walks, with and without
+    labels, edge limits and (where almost everything is WEAK) enough strong points."""
+    w, hgt, views = 90, 70, 4
+    sc = _scene(w, hgt, views, seed=rotate)
+    images, cams = _images(sc, True), [h.S.camera_struct(sc, i) for i in range(views)]
+    rng = np.random.default_rng(rotate)
+    state = np.concatenate([sc.normal[0], sc.depth[0][..., None]], -1).astype(np.float32)
+    weak = rng.choice(2, (hgt, w), p=[weak_share, 1 - weak_share]).astype(np.uint8)
+    edge, low, lab = h.synthetic_edges(sc.gray[0], 0.04)
+    lab = np.where(lab == 0, 0, 1 + (np.arange(w)[None, :] > w // 2)).astype(np.int32)
+    p = h.refine_params(sc, views, level=2, state=D.REFINE_ITER, geom=True)
+    p.rotate_time, p.high_res_img, p.use_label, p.use_limit = rotate, high_res, label, limit
+    kw = dict(plane_in=state, views_in=rng.integers(1, 2 ** (views - 1), (hgt, w)).astype(np.uint32), weak_in=weak,
+              edge=edge, edge_low=low, label=np.ascontiguousarray(lab),
+              depths=[np.ascontiguousarray(sc.depth[i].astype(np.float32)) for i in range(views)], seed=5)
+    _same(xctx.pm_run(images, cams, p, **kw), O.pm_run(images, cams, p, **kw), f"rotate {rotate}")
