@@ -35,6 +35,11 @@ constexpr int kMaxWin = 6;  // taps per window side for radius 5 / step 2 (DPE.c
 #ifndef DPE_SWEEP_MIN_BLOCKS
 #define DPE_SWEEP_MIN_BLOCKS 6
 #endif
+// LocalRefine: at 6, 5 blocks and unbounded 3.31, 3.37, 3.38 ms / 14.2, 13.7, 13.4 ms / 0.96, 0.93, 1.15
+// ms (first call, geometric call, 801x603 level)
+#ifndef DPE_LR_MIN_BLOCKS
+#define DPE_LR_MIN_BLOCKS 5
+#endif
 
 // All per-call read-only data (cameras, relative poses, params, buffer pointers).  It lives in a
 // small device buffer written once per call; kernels receive its address.
