@@ -537,21 +537,23 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
     k_pad_image<<<dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8), dim3(32, 8), 0, s>>>(src, img_pad + PL * i, W, H);
     PM_LAUNCHED("k_pad_image", s);
   }
-  // FP32 staging: when every source texel is exact in BF16 (8-bit images, the finest pyramid
-  // level), the cost kernels sample BF16 quads instead: the same values, one load per tap.
+  // FP32 staging: when every source texel is exact in a 16-bit format (BF16: 8-bit images, the finest
+  // pyramid level; FP16: the halved levels), the cost kernels sample 16-bit quads instead: the same
+  // values, one 8-byte load per tap instead of four.
   int staging = ctx->opt.staging;
   if (staging == DPE_STAGE_FP32 && N > 1) {
-    unsigned *flag = get((unsigned *)0, "bf16_flag", 1);
+    unsigned *flag = get((unsigned *)0, "exact_flag", 1);
     if (!flag) return DPE_ERR_OUT_OF_MEMORY;
     DPE_TRY(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
     const long long n = (long long)PL * (N - 1);
     const unsigned blocks = (unsigned)std::max(1LL, std::min((n + 255) / 256, (long long)ctx->sms * 8));
-    k_bf16_exact<<<blocks, 256, 0, s>>>(img_pad + PL, n, flag);
-    PM_LAUNCHED("k_bf16_exact", s);
-    unsigned inexact = 1;
+    k_exact16<<<blocks, 256, 0, s>>>(img_pad + PL, n, flag);
+    PM_LAUNCHED("k_exact16", s);
+    unsigned inexact = 3;
     DPE_TRY(cudaMemcpyAsync(&inexact, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     DPE_TRY(cudaStreamSynchronize(s));
-    if (!inexact) staging = DPE_STAGE_BF16;
+    if (!(inexact & 1u)) staging = DPE_STAGE_BF16;
+    else if (!(inexact & 2u)) staging = DPE_STAGE_FP16;
   }
   ps->staging = staging;
   a.stage = staging;
@@ -589,7 +591,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   cudaStream_t s = ctx->stream;
   Arena &A = ctx->arena;
   const dpe_params &P = ps[0].a.P;
-  // one staging for the sequence: BF16 quads only when every problem has them
+  // one staging for the sequence: 16-bit quads only when every problem has the same
   int staging = ps[0].staging;
   for (int b = 1; b < n; ++b)
     if (ps[b].staging != staging) staging = ctx->opt.staging;
@@ -688,12 +690,13 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
       DPE_TRY(attr);
       PM_LAUNCHED("k_strong_update", s);
     }
-    DPE_TIMED(ctx, KID_RANSAC, s,
-              shaped(KID_RANSAC, [&](dim3 gr, dim3 bl) { k_ransac_fit_plane<<<gr, bl, 0, s>>>(g.full); }));
-    PM_LAUNCHED("k_ransac_fit_plane", s);
+    if (P.use_APD) {
+      DPE_TIMED(ctx, KID_RANSAC, s, k_ransac_fit_plane<<<g.gn, 128, 0, s>>>(g.gneigh));
+      PM_LAUNCHED("k_ransac_fit_plane", s);
+    }
     if (P.use_APD)
       for (int parity = 0; parity < 2; ++parity) {
-        DPE_TIMED(ctx, KID_WEAK_PREPARE, s, k_weak_prepare<<<g.gp, 128, 0, s>>>(g.prep, parity));
+        DPE_TIMED(ctx, KID_WEAK_PREPARE, s, k_weak_prepare<<<g.ge, 128, 0, s>>>(g.eval, parity));
         PM_LAUNCHED("k_weak_prepare", s);
         DPE_TIMED(ctx, KID_WEAK_EVAL, s, with_stage(staging, [&](auto st) { k_weak_eval<false, decltype(st)::value><<<g.ge, 128, 0, s>>>(g.eval, parity); }));
         PM_LAUNCHED("k_weak_eval", s);
@@ -701,7 +704,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
         PM_LAUNCHED("k_weak_decide", s);
         DPE_TIMED(ctx, KID_WEAK_EVAL, s, with_stage(staging, [&](auto st) { k_weak_eval<true, decltype(st)::value><<<g.ge, 128, 0, s>>>(g.eval, parity); }));
         PM_LAUNCHED("k_weak_eval", s);
-        DPE_TIMED(ctx, KID_WEAK_FINISH, s, with_stage(staging, [&](auto st) { k_weak_finish<decltype(st)::value><<<g.gp, 128, 0, s>>>(g.prep, parity); }));
+        DPE_TIMED(ctx, KID_WEAK_FINISH, s, with_stage(staging, [&](auto st) { k_weak_finish<decltype(st)::value><<<g.ge, 128, 0, s>>>(g.eval, parity); }));
         PM_LAUNCHED("k_weak_finish", s);
       }
   }

@@ -941,15 +941,6 @@ __device__ __forceinline__ void ncc_all_sources(const PMArgs &a, int px, int py,
                                                 float *out) {
   for (int j = 0; j < a.N - 1; ++j) out[j] = ncc_strong<kStage, kPairs>(a, px, py, j + 1, pl, rw);
 }
-// Sum over the listed sources act[0..na) (ascending) of vw[j] * cost(j), in list order.
-template <int kStage, class RW, class A>
-__device__ __forceinline__ float weighted_ncc(const PMArgs &a, int px, int py, float4 pl, const RW &rw,
-                                             const A *act, int na, const uint8_t *vw) {
-  float tc = 0.0f;
-  for (int q = 0; q < na; ++q) tc += vw[act[q]] * ncc_strong<kStage>(a, px, py, act[q] + 1, pl, rw);
-  return tc;
-}
-
 __device__ __forceinline__ short2 neighbour(const PMArgs &a, int center, int k) {
   return a.neigh[(size_t)a.nmap[center] * kNeighbours + k];
 }
@@ -973,30 +964,157 @@ __device__ __forceinline__ void weak_window_shape(const PMArgs &a, int center, i
   *radius = r;
   *inc = s;
 }
-__device__ __forceinline__ int weak_window_base(const PMArgs &a, int k) {
-  return k == 0 ? 0 : kMaxWin * kMaxWin + (k - 1) * a.wtaps;
+// Layout of a pixel's table of window taps (wtab, 36 + 8 wtaps float2 per slot).  The centre window:
+// pairs of taps in tap order (win_store).  The 3 x 3 windows (radius 5, step 5): four pairs each, the
+// first two rows of every column and the third row of the first two, all windows' pairs after each other,
+// then the windows' last taps; so a pair is one aligned 16-byte load.  Windows of another size: plain
+// (w, w * (r - c)) in tap order.
+__device__ __forceinline__ bool weak_is3(const PMArgs &a) { return a.wtaps == 9; }
+__device__ __forceinline__ const float4 *weak_pairs(const PMArgs &a, const float2 *tab, int k) {
+  return reinterpret_cast<const float4 *>(tab) + (k == 0 ? 0 : kWinPairs + 4 * (k - 1));
+}
+__device__ __forceinline__ const float2 *weak_last(const float2 *tab, int k) { return tab + kWinTaps + 64 + (k - 1); }
+__device__ __forceinline__ const float2 *weak_plain(const PMArgs &a, const float2 *tab, int k) {
+  return tab + kWinTaps + (k - 1) * a.wtaps;
+}
+// Stores tap t of window k.
+__device__ __forceinline__ void weak_store(const PMArgs &a, float2 *tab, int k, int t, float w, float wr) {
+  if (k == 0) {
+    win_store(reinterpret_cast<float4 *>(tab), t, w, wr);
+  } else if (!weak_is3(a)) {
+    tab[kWinTaps + (k - 1) * a.wtaps + t] = make_float2(w, wr);
+  } else if (t == 8) {
+    tab[kWinTaps + 64 + (k - 1)] = make_float2(w, wr);
+  } else {
+    const int c = t / 3, r = t - 3 * c;
+    win_store(reinterpret_cast<float4 *>(tab) + kWinPairs + 4 * (k - 1), r < 2 ? 2 * c + r : 6 + c, w, wr);
+  }
+}
+__device__ __forceinline__ float2 weak_load(const PMArgs &a, const float2 *tab, int k, int t) {
+  if (k == 0) return win_tap(reinterpret_cast<const float4 *>(tab), t);
+  if (!weak_is3(a)) return weak_plain(a, tab, k)[t];
+  if (t == 8) return *weak_last(tab, k);
+  const int c = t / 3, r = t - 3 * c;
+  return win_tap(weak_pairs(a, tab, k), r < 2 ? 2 * c + r : 6 + c);
 }
 
-// The hypothesis-dependent half of one window: sums of w*s, w*s^2, w*(r-c)*s over the taps.
+// The hypothesis-dependent sums of a window column: w*s, w*s^2, w*(r-c)*s.
+struct WeakSums {
+  float s, ss, rs;
+};
+// One tap.
+template <class Src>
+__device__ __forceinline__ void weak_tap(const PMArgs &a, const float H[9], const Src &src, float x, float y,
+                                         float ref_center, float2 t, WeakSums &r) {
+  const float2 sp = project_tap(H, x, y);
+  const float sv = bilinear_s(src, a.W, a.H, sp.x, sp.y) - ref_center;
+  const float2 m = mul2(t, make_float2(sv, sv));  // (w s, w (r - c) s)
+  r.s += m.x; r.ss += m.x * sv; r.rs += m.y;
+}
+#ifdef __CUDA_ARCH__
+// The samples (minus ref_center) of two taps, given their H p products: colx, coly, colz the x terms (H0 x,
+// H3 x, H6 x) and rowx, rowy, rowz the y terms, per tap.  weak_tap's operations, two at a time.
+template <class Src>
+__device__ __forceinline__ float2 weak_sample2(const PMArgs &a, const float H[9], const Src &src, float2 colx, float2 coly,
+                                               float2 colz, float2 rowx, float2 rowy, float2 rowz, float ref_center) {
+  const float2 X = add2(addp2(colx, rowx), dup2(H[2])), Y = add2(addp2(coly, rowy), dup2(H[5]));
+  const float2 Z = add2(addp2(colz, rowz), dup2(H[8]));
+#ifndef DPE_EXACT
+  const float2 iz = make_float2(tap_rcp(Z.x), tap_rcp(Z.y));
+  float2 u = mul2(X, iz), v = mul2(Y, iz);
+#else
+  float2 u = make_float2(X.x / Z.x, X.y / Z.y), v = make_float2(Y.x / Z.x, Y.y / Z.y);
+#endif
+  const float ux = (float)(a.W - 1), vy = (float)(a.H - 1);
+  u = make_float2(fminf(fmaxf(u.x, -1.0f), ux), fminf(fmaxf(u.y, -1.0f), ux));
+  v = make_float2(fminf(fmaxf(v.x, -1.0f), vy), fminf(fmaxf(v.y, -1.0f), vy));
+  const float2 bias = dup2(12582912.0f);
+  const float2 fu = __fadd2_rd(u, bias), fv = __fadd2_rd(v, bias);
+  const float2 au = sub2(u, sub2(fu, bias)), av = sub2(v, sub2(fv, bias));
+  const float2 ou = sub2(dup2(1.0f), au), ov = sub2(dup2(1.0f), av);
+  const unsigned pw = (unsigned)src.pw, base = (1u - 0x4B400000u) * (pw + 1u);
+  const Foot2 t = fetch2(src, (int)(__float_as_uint(fv.x) * pw + __float_as_uint(fu.x) + base),
+                         (int)(__float_as_uint(fv.y) * pw + __float_as_uint(fu.y) + base));
+  const float2 top = addp2(mul2(ou, t.v00), mul2(au, t.v10)), bot = addp2(mul2(ou, t.v01), mul2(au, t.v11));
+  return sub2(addp2(mul2(ov, top), mul2(av, bot)), dup2(ref_center));
+}
+// Adds the two taps of a pair (w0, w1, w0 (r0 - c), w1 (r1 - c)) to their columns' sums, tap 0 first.
+__device__ __forceinline__ void weak_add2(float4 w, float2 sv, WeakSums &r0, WeakSums &r1) {
+  const float2 ws = mul2(make_float2(w.x, w.y), sv), rs = mul2(make_float2(w.z, w.w), sv), q = mul2(ws, sv);
+  r0.s += ws.x; r0.ss += q.x; r0.rs += rs.x;
+  r1.s += ws.y; r1.ss += q.y; r1.rs += rs.y;
+}
+#endif
+// The hypothesis-dependent half of window k of a pixel, and its cost.
 template <class Src>
 __device__ __forceinline__ float window_ncc_tab(const PMArgs &a, const float H[9], const Src &src, int cx, int cy,
                                                 int radius, int inc, float ref_center, const float2 *__restrict__ tab,
-                                                float4 win) {
+                                                int k, float4 win) {
   float s_s = 0, s_ss = 0, s_rs = 0;
-  int t = 0;
-  // whole-number tap coordinates stepped by exact float adds (no conversion per tap)
   const float finc = (float)inc, y0 = (float)(cy - radius);
   float x = (float)(cx - radius);
-  for (int i = -radius; i <= radius; i += inc, x += finc) {
-    float r_s = 0, r_ss = 0, r_rs = 0;
-    float y = y0;
-    for (int j = -radius; j <= radius; j += inc, y += finc) {
-      const float2 sp = project_tap(H, x, y);
-      const float sv = bilinear_s(src, a.W, a.H, sp.x, sp.y) - ref_center;
-      const float2 m = mul2(tab[t++], make_float2(sv, sv));  // (w s, w (r - c) s)
-      r_s += m.x; r_ss += m.x * sv; r_rs += m.y;
+#ifdef __CUDA_ARCH__
+  const int side = 2 * radius / inc + 1;
+  if (k > 0 && weak_is3(a)) {
+    const float4 *pairs = weak_pairs(a, tab, k);
+    float2 cX[3], rX[3], rY[3], rZ[3];  // column terms (H0 x, H3 x) and H6 x; row terms H1 y, H4 y, H7 y
+    float cZ[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float xi = i == 0 ? x : i == 1 ? x + finc : x + finc + finc;
+      cX[i] = mul2(make_float2(H[0], H[3]), dup2(xi));
+      cZ[i] = H[6] * xi;
     }
-    s_s += r_s; s_ss += r_ss; s_rs += r_rs;
+    float ry[3] = {y0, y0 + finc, y0 + finc + finc};
+    const float rx0 = H[1] * ry[0], rx1 = H[1] * ry[1], rx2 = H[1] * ry[2];
+    const float ry0 = H[4] * ry[0], ry1 = H[4] * ry[1], ry2 = H[4] * ry[2];
+    const float rz0 = H[7] * ry[0], rz1 = H[7] * ry[1], rz2 = H[7] * ry[2];
+    WeakSums r[3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float2 sv = weak_sample2(a, H, src, dup2(cX[i].x), dup2(cX[i].y), dup2(cZ[i]), make_float2(rx0, rx1),
+                                     make_float2(ry0, ry1), make_float2(rz0, rz1), ref_center);
+      weak_add2(pairs[i], sv, r[i], r[i]);
+    }
+    {
+      const float2 sv = weak_sample2(a, H, src, make_float2(cX[0].x, cX[1].x), make_float2(cX[0].y, cX[1].y),
+                                     make_float2(cZ[0], cZ[1]), dup2(rx2), dup2(ry2), dup2(rz2), ref_center);
+      weak_add2(pairs[3], sv, r[0], r[1]);
+    }
+    weak_tap(a, H, src, x + finc + finc, ry[2], ref_center, *weak_last(tab, k), r[2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) { s_s += r[i].s; s_ss += r[i].ss; s_rs += r[i].rs; }
+  } else if (k == 0 && side == 6) {
+    const float4 *pairs = weak_pairs(a, tab, 0);
+    float2 rX[3], rY[3], rZ[3];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const float2 y = make_float2(y0 + (float)(2 * p) * finc, y0 + (float)(2 * p + 1) * finc);  // whole numbers: exact
+      rX[p] = mul2(dup2(H[1]), y); rY[p] = mul2(dup2(H[4]), y); rZ[p] = mul2(dup2(H[7]), y);
+    }
+#pragma unroll 1
+    for (int i = 0; i < 18; i += 3, x += finc) {
+      const float cx0 = H[0] * x, cy0 = H[3] * x, cz0 = H[6] * x;
+      WeakSums r = {0, 0, 0};
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const float2 sv = weak_sample2(a, H, src, dup2(cx0), dup2(cy0), dup2(cz0), rX[p], rY[p], rZ[p], ref_center);
+        weak_add2(pairs[i + p], sv, r, r);
+      }
+      s_s += r.s; s_ss += r.ss; s_rs += r.rs;
+    }
+  } else
+#endif
+  {
+    // whole-number tap coordinates stepped by exact float adds (no conversion per tap)
+    int t = 0;
+    for (int i = -radius; i <= radius; i += inc, x += finc) {
+      WeakSums r = {0, 0, 0};
+      float y = y0;
+      for (int j = -radius; j <= radius; j += inc, y += finc)
+        weak_tap(a, H, src, x, y, ref_center, weak_load(a, tab, k, t++), r);
+      s_s += r.s; s_ss += r.ss; s_rs += r.rs;
+    }
   }
   float s_w = win.x, s_r = win.y, s_rr = win.z;
   const float inv = 1.0f / s_w;
@@ -1037,9 +1155,8 @@ __device__ __forceinline__ float ncc_weak_tab(const PMArgs &a, int slot, int cen
     }
     int radius, inc;
     weak_window_shape(a, center, k, &radius, &inc);
-    const float2 *wt = tab + weak_window_base(a, k);
     const float4 win = a.wwin[(size_t)slot * kNeighbours + k];
-    const float t = window_ncc_tab(a, H, SrcOf<kStage>::make(a, s), nb.x, nb.y, radius, inc, ref_center, wt, win);
+    const float t = window_ncc_tab(a, H, SrcOf<kStage>::make(a, s), nb.x, nb.y, radius, inc, ref_center, tab, k, win);
     if (k == 0) center_cost = t;
     else { strong_cost += t; strong_count++; }
   }

@@ -91,13 +91,18 @@ __global__ void k_stage_quads(const float *__restrict__ pad, uint2 *__restrict__
   out[o] = make_uint2(bits(o) | bits(o + 1) << 16, bits(o + pw) | bits(o + pw + 1) << 16);
 }
 
-// Sets *flag when any of the n floats is not exact in BF16 (a float is exact when its low 16
-// bits are zero: 8-bit images are).  One atomic per block.
-__global__ void k_bf16_exact(const float *__restrict__ p, long long n, unsigned *flag) {
-  unsigned bits = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    bits |= __float_as_uint(p[i]) & 0xFFFFu;
-  if (__syncthreads_or(bits != 0) && threadIdx.x == 0) atomicOr(flag, 1u);
+// Which 16-bit storage holds the n floats exactly: sets bit 0 of *flag when one is not exact in BF16 (its
+// low 16 bits are not all zero; 8-bit images are exact), bit 1 when one is not in FP16 (the pyramid's
+// halved levels are: averages of four 8-bit values, quarters below 256).  One atomic per block.
+__global__ void k_exact16(const float *__restrict__ p, long long n, unsigned *flag) {
+  unsigned b16 = 0, f16 = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const float v = p[i];
+    b16 |= __float_as_uint(v) & 0xFFFFu;
+    f16 |= __float_as_uint(__half2float(__float2half_rn(v))) ^ __float_as_uint(v);
+  }
+  const int b = __syncthreads_or(b16 != 0 ? 1 : 0), f = __syncthreads_or(f16 != 0 ? 1 : 0);
+  if ((b || f) && threadIdx.x == 0) atomicOr(flag, (b ? 1u : 0u) | (f ? 2u : 0u));
 }
 
 __global__ void k_init_state(const Launch lc, const float4 *plane_in, const uint32_t *views_in,
@@ -195,14 +200,9 @@ __device__ __forceinline__ void find_nearest_strong_pixel(const PMArgs &a, int p
   }
   a.nearest[center] = res;
 }
-// Resident blocks requested for the one-thread-per-pixel searches (the nearest strong point and
-// the plane fit), 80 registers each.
-#ifndef DPE_LATENCY_MIN_BLOCKS
-#define DPE_LATENCY_MIN_BLOCKS 6
-#endif
 // One thread per pixel of a 2D grid: the tiles keep the rays of neighbouring pixels together
 // (measured faster than a work list over the WEAK pixels).
-__global__ void __launch_bounds__(128, DPE_LATENCY_MIN_BLOCKS) k_find_nearest_strong(const Launch lc) {
+__global__ void __launch_bounds__(128) k_find_nearest_strong(const Launch lc) {
   const Blk B = resolve<kGridFull>(lc);
   const PMArgs &a = *B.a;
   int px, py;
@@ -1826,91 +1826,135 @@ __global__ void __launch_bounds__(kCoopThreads, DPE_STRONG_MIN_BLOCKS) k_strong_
 
 
 // ------------------------------------------------------------------ RANSACToGetFitPlane (DPE.cu:2895-3128)
-__device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, int py) {
+// A group of kGnLanes threads per WEAK pixel (only WEAK pixels read their fitted plane).  Every one of
+// the 50 rounds draws three numbers, so the lanes prepare the next rounds side by side: points, tests,
+// plane and its summed distance do not depend on earlier rounds; they are then taken in order under the
+// current state.  Host builds of this source run it with one lane.
+// 60 launches at 400x300 and 200x150: 5.4 -> 1.2 ms; three at 1600x1200 with 403 k WEAK pixels 7.7 -> 4.3 ms (one
+// thread per pixel before).
+struct FitPoints {
+  short2 sp[kNeighbours - 1];
+  float3 pos[kNeighbours - 1], nrm[kNeighbours - 1];
+  float2 ray[kNeighbours - 1];
+  LinePoint line[kNeighbours - 1];
+};
+__device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, const LineMap &map, const GnGroup &g, FitPoints &S,
+                                                       int px, int py) {
   const int W = a.W, center = px + py * W;
-  if (a.weak[center] != DPE_WEAK) { a.fit_plane[center] = a.plane[center]; return; }
-  Rng rng = make_rng(a, center);
+  uint32_t ctr = G(a.rng_ctr, center, (long long)W * a.H, 106);
   const dpe_camera &cam = a.cam[0];
   bool edge_limit = false;
   if (a.P.use_limit) {
     edge_limit = true;
     if (a.P.use_edge) {
       const float cv = a.complexity[center];
+      Rng rng{a.key[0], a.key[1], (uint32_t)center, ctr++};
       const float rp = rng.uniform() - FLT_EPSILON;
       if (rp < cv) edge_limit = false;
     }
   }
-  short2 sp[kNeighbours - 1];
-  float3 sp3[kNeighbours - 1], spn[kNeighbours - 1];
-  LinePoint line[kNeighbours - 1];
-  LineMap map{0.f, 0.f, 0, 0, 0};
-  if (edge_limit) map = line_map(a);
+  g.sync();  // the group's last pixel has been read
   int sc = 0;
-  float X[3];
   for (int i = 1; i < kNeighbours; ++i) {
     const short2 t = neighbour(a, center, i);
     if (t.x == -1 || t.y == -1) continue;
-    sp[sc] = t;
-    const int tc = t.x + t.y * W;
-    const float4 tpl = a.plane[tc];
-    const float d = depth_from_plane(cam, tpl, t.x, t.y);
-    point3d(cam, t.x, t.y, d, X);
-    sp3[sc] = make_float3(X[0], X[1], X[2]);
-    spn[sc] = make_float3(tpl.x, tpl.y, tpl.z);
-    if (edge_limit) line[sc] = line_point(a, map, t.x, t.y);
+    if (sc % kGnLanes == g.lane) {
+      S.sp[sc] = t;
+      const float4 tpl = a.plane[t.x + t.y * W];
+      const float d = depth_from_plane(cam, tpl, t.x, t.y);
+      float X[3];
+      point3d(cam, t.x, t.y, d, X);
+      S.pos[sc] = make_float3(X[0], X[1], X[2]);
+      S.nrm[sc] = make_float3(tpl.x, tpl.y, tpl.z);
+      S.ray[sc] = make_float2((t.x - cam.K[2]) / cam.K[0], (t.y - cam.K[5]) / cam.K[4]);
+      if (edge_limit) S.line[sc] = line_point(a, map, t.x, t.y);
+    }
     sc++;
   }
-  if (sc < 3) { a.fit_plane[center] = a.plane[center]; a.rng_ctr[center] = rng.ctr; return; }
+  if (sc < 3) {
+    if (g.lane == 0) {
+      a.fit_plane[center] = a.plane[center];
+      a.rng_ctr[center] = ctr;
+    }
+    return;
+  }
+  g.sync();
   int ua = -1, ub = -1, uc = -1;
   float min_cost = FLT_MAX;
   float4 best = make_float4(0, 0, 0, 0);
   bool has_best = false, has_strong = false;
   bool must_tri = (a.P.use_label && a.label[center] > 0 && edge_limit) ? false : true;
-  for (int iteration = 0; iteration < 50; ++iteration) {
-    const int ia = (int)(rng.u32() % (uint32_t)sc);
-    const int ib = (int)(rng.u32() % (uint32_t)sc);
-    const int ic = (int)(rng.u32() % (uint32_t)sc);
-    if (ia == ib || ib == ic || ia == ic) continue;
-    bool is_strong = false;
-    if (a.P.geom_consistency && edge_limit) {
-      const float3 AN = spn[ia], BN = spn[ib], CN = spn[ic];
-      is_strong = true;
-      if ((double)(AN.x * BN.x + AN.y * BN.y + AN.z * BN.z) < 0.8660254 ||
-          (double)(AN.x * CN.x + AN.y * CN.y + AN.z * CN.z) < 0.8660254 ||
-          (double)(BN.x * CN.x + BN.y * CN.y + BN.z * CN.z) < 0.8660254)
-        is_strong = false;
-      if (has_strong && !is_strong) continue;
-    }
-    if (must_tri && !point_in_triangle(sp[ia], sp[ib], sp[ic], px, py)) continue;
-    if (edge_limit) {
-      if (line_blocked(a, map, line[ia], line[ib]) || line_blocked(a, map, line[ib], line[ic]) ||
-          line_blocked(a, map, line[ic], line[ia]))
-        continue;
-    }
-    const float3 A = sp3[ia], B = sp3[ib], C = sp3[ic];
-    const float3 AC = make_float3(A.x - C.x, A.y - C.y, A.z - C.z), BC = make_float3(B.x - C.x, B.y - C.y, B.z - C.z);
-    float4 cr;
-    cr.x = AC.y * BC.z - BC.y * AC.z;
-    cr.y = -(AC.x * BC.z - BC.x * AC.z);
-    cr.z = AC.x * BC.y - BC.x * AC.y;
-    if ((cr.x == 0 && cr.y == 0 && cr.z == 0) || isnan(cr.x) || isnan(cr.y) || isnan(cr.z)) continue;
-    normalize3(&cr);
-    cr.w = -(cr.x * A.x + cr.y * A.y + cr.z * A.z);
-    if (!has_strong && is_strong) has_strong = true;
+  for (int i0 = 0; i0 < 50; i0 += kGnLanes) {
+    bool ok = i0 + g.lane < 50, tri = false, strong = false;
+    int ia = 0, ib = 0, ic = 0;
+    float4 cr = make_float4(0, 0, 0, 0);
     float tc = 0.0f;
-    for (int s = 0; s < sc; ++s) {
-      if (s == ia || s == ib || s == ic) continue;
-      const float fx = (sp[s].x - cam.K[2]) / cam.K[0];
-      const float fy = (sp[s].y - cam.K[5]) / cam.K[4];
-      const float fd = -cr.w / (cr.x * fx + cr.y * fy + cr.z);
-      tc += fabsf(fd - sp3[s].z);
+    if (ok) {
+      Rng rng{a.key[0], a.key[1], (uint32_t)center, ctr + 3u * (uint32_t)(i0 + g.lane)};
+      ia = (int)(rng.u32() % (uint32_t)sc);
+      ib = (int)(rng.u32() % (uint32_t)sc);
+      ic = (int)(rng.u32() % (uint32_t)sc);
+      ok = !(ia == ib || ib == ic || ia == ic);
     }
-    if (tc < min_cost) {
-      if (!must_tri && point_in_triangle(sp[ia], sp[ib], sp[ic], px, py)) must_tri = true;
-      min_cost = tc; best = cr; has_best = true; ua = ia; ub = ib; uc = ic;
+    if (ok && a.P.geom_consistency && edge_limit) {
+      const float3 AN = S.nrm[ia], BN = S.nrm[ib], CN = S.nrm[ic];
+      strong = !((double)(AN.x * BN.x + AN.y * BN.y + AN.z * BN.z) < 0.8660254 ||
+                 (double)(AN.x * CN.x + AN.y * CN.y + AN.z * CN.z) < 0.8660254 ||
+                 (double)(BN.x * CN.x + BN.y * CN.y + BN.z * CN.z) < 0.8660254);
+      ok = strong || !has_strong;
+    }
+    if (ok) {
+      tri = point_in_triangle(S.sp[ia], S.sp[ib], S.sp[ic], px, py);
+      ok = tri || !must_tri;
+    }
+    if (edge_limit) {
+      int i = ia, j = ib;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+      for (int k = 0; ok && k < 3; ++k) {
+        ok = !line_blocked(a, map, S.line[i], S.line[j]);
+        i = j;
+        j = k == 0 ? ic : ia;
+      }
+    }
+    if (ok) {
+      const float3 A = S.pos[ia], B = S.pos[ib], C = S.pos[ic];
+      const float3 AC = make_float3(A.x - C.x, A.y - C.y, A.z - C.z), BC = make_float3(B.x - C.x, B.y - C.y, B.z - C.z);
+      cr.x = AC.y * BC.z - BC.y * AC.z;
+      cr.y = -(AC.x * BC.z - BC.x * AC.z);
+      cr.z = AC.x * BC.y - BC.x * AC.y;
+      ok = !((cr.x == 0 && cr.y == 0 && cr.z == 0) || isnan(cr.x) || isnan(cr.y) || isnan(cr.z));
+      if (ok) {
+        normalize3(&cr);
+        cr.w = -(cr.x * A.x + cr.y * A.y + cr.z * A.z);
+        for (int s = 0; s < sc; ++s) {
+          if (s == ia || s == ib || s == ic) continue;
+          const float fd = -cr.w / (cr.x * S.ray[s].x + cr.y * S.ray[s].y + cr.z);
+          tc += fabsf(fd - S.pos[s].z);
+        }
+      }
+    }
+    const unsigned b_tri = g.ballot(tri), b_strong = g.ballot(strong);
+    for (unsigned todo = g.ballot(ok); todo; todo &= todo - 1) {
+      const int r = g.first(todo);
+      const bool r_tri = (b_tri >> r) & 1u, r_strong = (b_strong >> r) & 1u;
+      if (a.P.geom_consistency && edge_limit && has_strong && !r_strong) continue;
+      if (must_tri && !r_tri) continue;
+      if (r_strong) has_strong = true;
+      const float t = g.from(tc, r);
+      if (t < min_cost) {
+        if (r_tri) must_tri = true;
+        min_cost = t;
+        best = make_float4(g.from(cr.x, r), g.from(cr.y, r), g.from(cr.z, r), g.from(cr.w, r));
+        has_best = true;
+        ua = g.from(ia, r); ub = g.from(ib, r); uc = g.from(ic, r);
+      }
     }
   }
-  a.rng_ctr[center] = rng.ctr;
+  ctr += 150u;
+  if (g.lane != 0) return;
+  a.rng_ctr[center] = ctr;
   if (has_best) {
     const float depth = depth_from_plane(cam, a.plane[center], px, py);
     const float4 v = view_direction(cam, px, py, depth);
@@ -1918,7 +1962,7 @@ __device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, 
     a.fit_plane[center] = best;
     if (a.P.use_radius) {
       if (must_tri) {
-        const short2 A = sp[ua], B = sp[ub], C = sp[uc];
+        const short2 A = S.sp[ua], B = S.sp[ub], C = S.sp[uc];
         const float la = sqrtf((float)((A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y)));
         const float lb = sqrtf((float)((B.x - C.x) * (B.x - C.x) + (B.y - C.y) * (B.y - C.y)));
         const float lc = sqrtf((float)((C.x - A.x) * (C.x - A.x) + (C.y - A.y) * (C.y - A.y)));
@@ -1965,14 +2009,31 @@ __device__ __forceinline__ void ransac_fit_plane_pixel(const PMArgs &a, int px, 
     if (a.P.use_radius) a.radius[center] = a.P.strong_radius;
   }
 }
-// One thread per pixel of a 2D grid: the tiles keep the rays of neighbouring pixels together
-// (measured faster than a work list over the WEAK pixels).
-__global__ void __launch_bounds__(128, DPE_LATENCY_MIN_BLOCKS) k_ransac_fit_plane(const Launch lc) {
+// On the device a grid of groups strides over both colours' lists; host builds call it per pixel.
+__global__ void __launch_bounds__(128) k_ransac_fit_plane(const Launch lc) {
+#ifdef __CUDA_ARCH__
+  const Blk B = resolve<kGridList>(lc);
+  const PMArgs &a = *B.a;
+  __shared__ FitPoints S[128 / kGnLanes];
+  const LineMap map = a.P.use_limit ? line_map(a) : LineMap{0.f, 0.f, 0, 0, 0};
+  const int slot = (int)threadIdx.x / kGnLanes;
+  GnGroup g;
+  g.lane = (int)threadIdx.x % kGnLanes;
+  g.shift = ((int)threadIdx.x & 31) - g.lane;
+  g.mask = (kGnLanes == 32 ? 0xFFFFFFFFu : (1u << (kGnLanes & 31)) - 1u) << g.shift;
+  const int n0 = a.wcount[0], count = n0 + a.wcount[1];
+  for (int i = B.x * (128 / kGnLanes) + slot; i < count; i += B.gx * (128 / kGnLanes)) {
+    const int c = i < n0 ? a.wlist[0][i] : a.wlist[1][i - n0];
+    ransac_fit_plane_pixel(a, map, g, S[slot], c % a.W, c / a.W);
+  }
+#else
   const Blk B = resolve<kGridFull>(lc);
   const PMArgs &a = *B.a;
   int px, py;
-  if (!full_pixel(a, B, &px, &py)) return;
-  ransac_fit_plane_pixel(a, px, py);
+  if (!full_pixel(a, B, &px, &py) || a.weak[px + py * a.W] != DPE_WEAK) return;
+  FitPoints S;
+  ransac_fit_plane_pixel(a, a.P.use_limit ? line_map(a) : LineMap{0.f, 0.f, 0, 0, 0}, GnGroup{0}, S, px, py);
+#endif
 }
 
 // ------------------------------------------------------------------ weak update (DPE.cu:1672-1866, 1124-1216)
@@ -1991,39 +2052,40 @@ __global__ void __launch_bounds__(128, DPE_LATENCY_MIN_BLOCKS) k_ransac_fit_plan
 // list does not matter.  Work items are strided over a grid sized for the GPU; the list lengths
 // stay on the device.
 
+// A thread per (pixel, window): the longest chain is the centre window's 36 taps (60 launches at 400x300
+// and 200x150: 4.4 -> 1.5 ms against a thread per pixel).
 __global__ void __launch_bounds__(128) k_weak_prepare(const Launch lc, int parity) {
   const Blk B = resolve<kGridList>(lc);
   const PMArgs &a = *B.a;
-  const int count = a.wcount[parity];
+  const long long total = (long long)a.wcount[parity] * kNeighbours;
   const int *list = a.wlist[parity];
-  for (int slot = B.x * blockDim.x + threadIdx.x; slot < count; slot += B.gx * blockDim.x) {
+  for (long long i = (long long)B.x * blockDim.x + threadIdx.x; i < total; i += (long long)B.gx * blockDim.x) {
+    const int slot = (int)(i / kNeighbours), k = (int)(i - (long long)slot * kNeighbours);
     const int center = list[slot];
     const int px = center % a.W, py = center / a.W;
     const float ref_center = texel(a, 0, px, py);
     float2 *tab = a.wtab + (size_t)slot * a.wtab_stride;
-    for (int k = 0; k < kNeighbours; ++k) {
-      const short2 nb = neighbour(a, center, k);
-      float4 win = make_float4(0, 0, 0, 0);
-      if (nb.x != -1 && nb.y != -1) {
-        int radius, inc;
-        weak_window_shape(a, center, k, &radius, &inc);
-        int t = weak_window_base(a, k);
-        float s_r = 0, s_rr = 0, s_w = 0;
-        for (int i = -radius; i <= radius; i += inc) {
-          float r_r = 0, r_rr = 0, r_w = 0;
-          for (int j = -radius; j <= radius; j += inc) {
-            const float rp = texel(a, 0, nb.x + i, nb.y + j);
-            const float w = bilateral_weight((float)i, (float)j, rp, ref_center, a.P.sigma_spatial, a.P.sigma_color);
-            const float rc = rp - ref_center;
-            tab[t++] = make_float2(w, w * rc);
-            r_r += w * rc; r_rr += w * rc * rc; r_w += w;
-          }
-          s_r += r_r; s_rr += r_rr; s_w += r_w;
+    const short2 nb = neighbour(a, center, k);
+    float4 win = make_float4(0, 0, 0, 0);
+    if (nb.x != -1 && nb.y != -1) {
+      int radius, inc;
+      weak_window_shape(a, center, k, &radius, &inc);
+      int t = 0;
+      float s_r = 0, s_rr = 0, s_w = 0;
+      for (int x = -radius; x <= radius; x += inc) {
+        float r_r = 0, r_rr = 0, r_w = 0;
+        for (int y = -radius; y <= radius; y += inc) {
+          const float rp = texel(a, 0, nb.x + x, nb.y + y);
+          const float w = bilateral_weight((float)x, (float)y, rp, ref_center, a.P.sigma_spatial, a.P.sigma_color);
+          const float rc = rp - ref_center;
+          weak_store(a, tab, k, t++, w, w * rc);
+          r_r += w * rc; r_rr += w * rc * rc; r_w += w;
         }
-        win = make_float4(s_w, s_r, s_rr, 0.0f);
+        s_r += r_r; s_rr += r_rr; s_w += r_w;
       }
-      a.wwin[(size_t)slot * kNeighbours + k] = win;
+      win = make_float4(s_w, s_r, s_rr, 0.0f);
     }
+    a.wwin[(size_t)slot * kNeighbours + k] = win;
   }
 }
 
@@ -2031,52 +2093,105 @@ __global__ void __launch_bounds__(128) k_weak_prepare(const Launch lc, int parit
 // 8 the current plane, 9 the fitted plane.  kRandom = true: the five random hypotheses, for the
 // sources the pixel sampled.  Unevaluated candidates keep the fused form's initial costs (0, and 2
 // for the first candidate's first source: quirk Q2).
-template <bool kRandom, int kStage>
-// Resident blocks requested for the deformable evaluation (__launch_bounds__): measured on the
-// 10-view 1600x1200 schedule, 8 blocks (64 registers, a few spills) make it 21 % faster than the
-// unbounded 96 registers and 5 blocks: it waits on its gathers, and more warps hide them.
+// A warp takes one pixel: its threads split the (hypothesis, source) pairs that have a cost, the
+// hypotheses of one source next to each other, so that a gather reads one image and the windows, their
+// shapes and their tables are the warp's.  (A thread per pair of the whole list, sources next to each
+// other, spent 72 - 84 % of L1's cycles on gathers spread over nine images, with 20 - 25 of 32
+// threads active.)  Host builds of this source run it with one lane.
+// Measured (12 launches; 1600x1200 geometric call / 801x603 level / 20 calls at 400x300 and 200x150): 64.6 /
+// 14.9 / 7.3 -> 49.7 / 11.4 / 6.0 ms at 4 blocks (128 registers); 6 blocks 49.6 / 11.3 / 6.5, 8 blocks
+// 51.2 / - / 6.8.
 #ifndef DPE_WEAK_MIN_BLOCKS
-#define DPE_WEAK_MIN_BLOCKS 8
+#define DPE_WEAK_MIN_BLOCKS 4
 #endif
+#ifdef __CUDA_ARCH__
+constexpr int kWeakLanes = 32;
+#else
+constexpr int kWeakLanes = 1;
+#endif
+struct WeakItems {
+  float4 pl[10];
+  uint8_t hyp[16], src[32];  // the hypotheses and sources that are evaluated
+  int nh, ns;
+};
+template <bool kRandom>
+__device__ __forceinline__ void weak_items(const PMArgs &a, int slot, int center, int lane, WeakItems &S) {
+  const int n = a.N - 1;
+  for (int h = lane; h < (kRandom ? 5 : 10); h += kWeakLanes) {
+    bool on = true;
+    float4 pl;
+    if (kRandom) {
+      pl = a.whyp[(size_t)slot * 5 + h];
+    } else if (h < 8) {
+      const short2 nb = neighbour(a, center, h + 1);
+      on = !(nb.x == -1 || nb.y == -1 || a.weak[nb.x + nb.y * a.W] != DPE_STRONG);
+      if (on) pl = a.plane[nb.x + nb.y * a.W];
+    } else {
+      pl = h == 8 ? a.plane[center] : a.fit_plane[center];
+      if (h == 9) on = !(pl.x == 0 && pl.y == 0 && pl.z == 0);  // unused: refinement skipped
+    }
+    if (on) S.pl[h] = pl;
+    S.hyp[h] = on ? 1 : 0;
+    if (!on && h < 8)
+      for (int j = 0; j < n; ++j) {
+        a.wcost[((size_t)slot * 10 + h) * n + j] = (h == 0 && j == 0) ? 2.0f : 0.0f;
+        a.wgeom[((size_t)slot * 10 + h) * n + j] = 0.0f;
+      }
+  }
+}
+// The lists of what is evaluated, from the flags (one thread).
+template <bool kRandom>
+__device__ __forceinline__ void weak_lists(const PMArgs &a, int center, WeakItems &S) {
+  int m = 0;
+  for (int h = 0; h < (kRandom ? 5 : 10); ++h)
+    if (S.hyp[h]) S.hyp[m++] = (uint8_t)h;
+  S.nh = m;
+  m = 0;
+  const uint4 vw = kRandom ? a.vweight[center] : make_uint4(0, 0, 0, 0);
+  for (int j = 0; j < a.N - 1; ++j)
+    if (!kRandom || vweight_at(vw, j) != 0) S.src[m++] = (uint8_t)j;
+  S.ns = m;
+}
+template <bool kRandom, int kStage>
 __global__ void __launch_bounds__(128, DPE_WEAK_MIN_BLOCKS) k_weak_eval(const Launch lc, int parity) {
   const Blk B = resolve<kGridList>(lc);
   const PMArgs &a = *B.a;
-  const int n = a.N - 1;
-  const int hyps = kRandom ? 5 : 10;
-  const long long per = (long long)hyps * n;
-  const long long total = (long long)a.wcount[parity] * per;
+#ifdef __CUDA_ARCH__
+  __shared__ WeakItems sh[128 / kWeakLanes];
+  WeakItems &S = sh[threadIdx.x / kWeakLanes];
+#else
+  WeakItems S;
+#endif
+  const int n = a.N - 1, hyps = kRandom ? 5 : 10;
+  const int count = a.wcount[parity];
   const int *list = a.wlist[parity];
   const bool geom = a.P.geom_consistency != 0;
   float *costs = kRandom ? a.wcost_r : a.wcost;
   float *geoms = kRandom ? a.wgeom_r : a.wgeom;
-  for (long long t = (long long)B.x * blockDim.x + threadIdx.x; t < total; t += (long long)B.gx * blockDim.x) {
-    const int slot = (int)(t / per);
-    const int r = (int)(t - (long long)slot * per);
-    const int h = r / n, j = r - h * n;
+  const int lane = (int)threadIdx.x % kWeakLanes, per = blockDim.x / kWeakLanes;
+  for (int slot = B.x * per + (int)threadIdx.x / kWeakLanes; slot < count; slot += B.gx * per) {
     const int center = list[slot];
     const int px = center % a.W, py = center / a.W;
-    float4 pl;
     if (kRandom) {
       const float4 fp = a.fit_plane[center];
       if (fp.x == 0 && fp.y == 0 && fp.z == 0) continue;  // no random refinement for this pixel
-      if (vweight_at(a.vweight[center], j) == 0) continue;
-      pl = a.whyp[(size_t)slot * 5 + h];
-    } else if (h < 8) {
-      const short2 nb = neighbour(a, center, h + 1);
-      if (nb.x == -1 || nb.y == -1 || a.weak[nb.x + nb.y * a.W] != DPE_STRONG) {
-        costs[t] = (h == 0 && j == 0) ? 2.0f : 0.0f;
-        geoms[t] = 0.0f;
-        continue;
-      }
-      pl = a.plane[nb.x + nb.y * a.W];
-    } else if (h == 8) {
-      pl = a.plane[center];
-    } else {
-      pl = a.fit_plane[center];
-      if (pl.x == 0 && pl.y == 0 && pl.z == 0) continue;  // unused: refinement skipped
     }
-    costs[t] = ncc_weak_tab<kStage>(a, slot, center, px, py, j + 1, pl, KID_WEAK_EVAL);
-    geoms[t] = geom ? geom_cost(a, px, py, j + 1, pl) : 0.0f;
+    DPE_WARP_BARRIER();  // the last pixel's lists have been read
+    weak_items<kRandom>(a, slot, center, lane, S);
+    DPE_WARP_BARRIER();
+    if (lane == 0) weak_lists<kRandom>(a, center, S);
+    DPE_WARP_BARRIER();
+    const int total = S.nh * S.ns;
+    for (int i0 = 0; i0 < total; i0 += kWeakLanes) {
+      DPE_WARP_BARRIER();
+      const int i = i0 + lane;
+      if (i >= total) continue;
+      const int jj = i / S.nh, h = S.hyp[i - jj * S.nh], j = S.src[jj];
+      const float4 pl = S.pl[h];
+      const size_t at = ((size_t)slot * hyps + h) * n + j;
+      costs[at] = ncc_weak_tab<kStage>(a, slot, center, px, py, j + 1, pl, KID_WEAK_EVAL);
+      geoms[at] = geom ? geom_cost(a, px, py, j + 1, pl) : 0.0f;
+    }
   }
 }
 
@@ -2180,10 +2295,31 @@ __global__ void __launch_bounds__(128) k_weak_decide(const Launch lc, int iter, 
   }
 }
 
+// 8 threads per pixel: they split the window's taps and the sources of the final cost; the first of them
+// takes the decisions (60 launches at 400x300 and 200x150: 3.8 -> 1.2 ms against a thread per pixel, whose
+// chain of evaluations was the launch's length; 2.5 -> 3.2 ms for six at 1600x1200, where threads abound).
+// Host builds of this source run it with one.
+#ifdef __CUDA_ARCH__
+constexpr int kFinishLanes = 8;
+#else
+constexpr int kFinishLanes = 1;
+#endif
+struct FinishPixel {
+  float4 win[kWinPairs];
+  float rc[kWinTaps];  // w (r - c)^2 per tap
+  float cost[kMaxSrc];
+  float4 pl;
+};
 template <int kStage>
 __global__ void __launch_bounds__(128) k_weak_finish(const Launch lc, int parity) {
   const Blk B = resolve<kGridList>(lc);
   const PMArgs &a = *B.a;
+#ifdef __CUDA_ARCH__
+  __shared__ FinishPixel sh[128 / kFinishLanes];
+  FinishPixel &S = sh[threadIdx.x / kFinishLanes];
+#else
+  FinishPixel S;
+#endif
   const int n = a.N - 1, W = a.W;
   const int count = a.wcount[parity];
   const int *list = a.wlist[parity];
@@ -2191,52 +2327,94 @@ __global__ void __launch_bounds__(128) k_weak_finish(const Launch lc, int parity
   const bool geom = a.P.geom_consistency != 0;
   const float gf = a.P.geom_factor;
   const float dmin = a.P.depth_min, dmax = a.P.depth_max;
-  for (int slot = B.x * blockDim.x + threadIdx.x; slot < count; slot += B.gx * blockDim.x) {
-    const int center = list[slot];
+  const int lane = (int)threadIdx.x % kFinishLanes, per = blockDim.x / kFinishLanes;
+  const int first = B.x * per + (int)threadIdx.x / kFinishLanes;
+  // every thread makes every round (the barriers are the warp's)
+  for (int s0 = 0; s0 < count; s0 += B.gx * per) {
+    const int slot = s0 + first;
+    const bool on = slot < count;
+    const int center = on ? list[slot] : 0;
     const int px = center % W, py = center / W;
-    float4 pl_now = a.wstate[(size_t)slot * 2];
-    const float4 st = a.wstate[(size_t)slot * 2 + 1];
-    float cost_now = st.y;
-    const float cost_written = st.z, wn = st.w;
-    const uint4 vwp = a.vweight[center];
-    const float4 fp = a.fit_plane[center];
-    if (!(fp.x == 0 && fp.y == 0 && fp.z == 0)) {
-      const float *cr = a.wcost_r + (size_t)slot * 5 * n;
-      const float *gr = a.wgeom_r + (size_t)slot * 5 * n;
-      for (int h = 0; h < 5; ++h) {
-        const float4 t = a.whyp[(size_t)slot * 5 + h];
-        float tc = 0.0f;
-        for (int j = 0; j < n; ++j) {
-          const int v = vweight_at(vwp, j);
-          if (v > 0) {
-            const float c = cr[h * n + j];
-            if (geom) tc += v * (c + gf * gr[h * n + j]);
-            else tc += v * c;
-          }
-        }
-        tc /= wn;
-        const float db = depth_from_plane(rc, t, px, py);
-        if (db >= dmin && db <= dmax && tc < cost_now) { pl_now = t; cost_now = tc; }
+    const uint4 vwp = on ? a.vweight[center] : make_uint4(0, 0, 0, 0);
+    const float wn = on ? a.wstate[(size_t)slot * 2 + 1].w : 0.0f;
+    DPE_WARP_BARRIER();  // the last round's shared values have been read
+    float center_val = 0.0f;
+    if (on) {
+      // window taps of the final re-cost with the strong window (DPE.cu:1849-1865; the radius swap there
+      // has no effect)
+      const int r = a.P.strong_radius, inc = a.P.strong_increment, side = 2 * r / inc + 1;
+      center_val = texel(a, 0, px, py);
+      for (int k = lane; k < side * side; k += kFinishLanes) {
+        const int i = -r + (k / side) * inc, j = -r + (k % side) * inc;
+        const float rp = texel(a, 0, px + i, py + j);
+        const float w = bilateral_weight((float)i, (float)j, rp, center_val, a.P.sigma_spatial, a.P.sigma_color);
+        const float d = rp - center_val, wr = w * d;
+        win_store(S.win, k, w, wr);
+        S.rc[k] = wr * d;
       }
     }
-    float4 pl_final = a.plane[center];
-    if (a.P.state == DPE_REFINE_INIT) {
-      if ((double)cost_now < (double)cost_written - 0.1) pl_final = pl_now;
-    } else {
-      pl_final = pl_now;
+    if (on && lane == 0) {
+      float4 pl_now = a.wstate[(size_t)slot * 2];
+      const float4 st = a.wstate[(size_t)slot * 2 + 1];
+      float cost_now = st.y;
+      const float cost_written = st.z;
+      const float4 fp = a.fit_plane[center];
+      if (!(fp.x == 0 && fp.y == 0 && fp.z == 0)) {
+        const float *cr = a.wcost_r + (size_t)slot * 5 * n;
+        const float *gr = a.wgeom_r + (size_t)slot * 5 * n;
+        for (int h = 0; h < 5; ++h) {
+          const float4 t = a.whyp[(size_t)slot * 5 + h];
+          float tc = 0.0f;
+          for (int j = 0; j < n; ++j) {
+            const int v = vweight_at(vwp, j);
+            if (v > 0) {
+              const float c = cr[h * n + j];
+              if (geom) tc += v * (c + gf * gr[h * n + j]);
+              else tc += v * c;
+            }
+          }
+          tc /= wn;
+          const float db = depth_from_plane(rc, t, px, py);
+          if (db >= dmin && db <= dmax && tc < cost_now) { pl_now = t; cost_now = tc; }
+        }
+      }
+      float4 pl_final = a.plane[center];
+      if (a.P.state == DPE_REFINE_INIT) {
+        if ((double)cost_now < (double)cost_written - 0.1) pl_final = pl_now;
+      } else {
+        pl_final = pl_now;
+      }
+      a.plane[center] = pl_final;
+      S.pl = pl_final;
     }
-    a.plane[center] = pl_final;
-    // final re-cost with the strong window (DPE.cu:1849-1865); the radius swap there has no effect
-    DPE_REF_WINDOW(rw);
-    build_ref_window(a, px, py, rw, KID_WEAK_FINISH);
-    uint8_t vw[32];
-    int act[kMaxSrc];
-    int na = 0;
-    for (int i = 0; i < n; ++i) {
-      vw[i] = (uint8_t)vweight_at(vwp, i);
-      if (vw[i] > 0) act[na++] = i;
+    DPE_WARP_BARRIER();
+    if (on) {
+      const int side = 2 * a.P.strong_radius / a.P.strong_increment + 1;
+      float sw = 0.f, swr = 0.f, swrr = 0.f;
+      for (int k = 0; k < side * side; ++k) {
+        const float2 t = win_tap(S.win, k);
+        sw += t.x; swr += t.y; swrr += S.rc[k];
+      }
+      SmemWindow rw;
+      rw.t_ = S.win;
+      rw.center = center_val;
+      rw.inv_wsum = 1.0f / sw;
+      rw.mean_r = swr * rw.inv_wsum;
+      rw.var_r = swrr * rw.inv_wsum - rw.mean_r * rw.mean_r;
+      rw.cnt = a.counters ? a.counters + 2 * KID_WEAK_FINISH : nullptr;
+      const float4 pl = S.pl;
+      for (int j = lane; j < n; j += kFinishLanes)
+        if (vweight_at(vwp, j) > 0) S.cost[j] = ncc_strong<kStage, true>(a, px, py, j + 1, pl, rw);
     }
-    a.cost[center] = weighted_ncc<kStage>(a, px, py, pl_final, rw, act, na, vw) / wn;
+    DPE_WARP_BARRIER();
+    if (on && lane == 0) {
+      float tc = 0.0f;
+      for (int j = 0; j < n; ++j) {
+        const int v = vweight_at(vwp, j);
+        if (v > 0) tc += v * S.cost[j];
+      }
+      a.cost[center] = tc / wn;
+    }
   }
 }
 
