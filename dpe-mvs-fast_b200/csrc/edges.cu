@@ -19,6 +19,7 @@
 // The hysteresis is a connected-components pass: union-find over the candidate pixels with
 // atomicMin on the roots (the lock-free union of Playne and Hawick, "A new algorithm for
 // parallel connected-component labelling on GPUs", IEEE TPDS 2018), then one flag per root.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -278,57 +279,86 @@ __global__ void k_threshold(uint8_t *d, int n, int thr) {
 // both neighbours with different labels records the join connection[larger] = smaller; the
 // reference overwrites earlier joins of the same label, so only the last in raster order counts,
 // kept as atomicMax of (pixel index << 32 | smaller label).
-constexpr int kConnectThreads = 512;
+// The scan also counts the openings: within a run only its first pixel opens, so a run without an upper
+// join takes the label of the last opening up to it.  Each thread takes kConnectItems neighbouring
+// pixels, so a row of up to 2048 is one step of one scan; the step's length is its barriers and the
+// loads behind them, not its pixels.  (With a pixel per thread and a scan each for the count and the
+// minimum, a 1600x1200 map took 5.2 ms more than a 400x300 one; now 1.9 ms.)
+constexpr int kConnectThreads = 512, kConnectItems = 4;
 
-struct SegMin {
+struct RunScan {
   int start;  // a run starts within the scanned prefix
-  int v;
+  int v;      // smallest upper label since
+  int opens;  // openings
 };
-struct SegMinOp {
-  __device__ __forceinline__ SegMin operator()(const SegMin &a, const SegMin &b) const {
-    return SegMin{a.start | b.start, b.start ? b.v : min(a.v, b.v)};
+struct RunScanOp {
+  __device__ __forceinline__ RunScan operator()(const RunScan &a, const RunScan &b) const {
+    return RunScan{a.start | b.start, b.start ? b.v : min(a.v, b.v), a.opens + b.opens};
   }
 };
 
 __global__ void __launch_bounds__(kConnectThreads) k_connect_rows(const uint8_t *__restrict__ img, int cols, int rows,
                                                                  int *__restrict__ lab,
                                                                  unsigned long long *__restrict__ join, int *nlab) {
-  typedef cub::BlockScan<int, kConnectThreads> ScanI;
-  typedef cub::BlockScan<SegMin, kConnectThreads> ScanS;
-  __shared__ typename ScanI::TempStorage ts_i;
-  __shared__ typename ScanS::TempStorage ts_s;
-  __shared__ int s_next, s_carry;
+  typedef cub::BlockScan<RunScan, kConnectThreads> Scan;
+  __shared__ typename Scan::TempStorage ts;
+  __shared__ int s_next, s_carry, s_last[kConnectThreads];
   const int tid = threadIdx.x;
-  if (tid == 0) s_next = 1;
+  if (tid == 0) {
+    s_next = 1;
+    s_carry = 0;
+  }
   __syncthreads();
   for (int y = 0; y < rows; ++y) {
-    for (int base = 0; base < cols; base += kConnectThreads) {
-      const int x = base + tid;
-      const bool in = x < cols;
-      const size_t p = (size_t)y * cols + x;
-      const int v = in ? img[p] : 255;
-      const bool labelled = in && v != 255, zero = in && v == 0;
-      const bool leftj = zero && x > 0 && img[p - 1] == 0;
-      const bool upj = zero && y > 0 && img[p - cols] == 0;
-      const bool opens = labelled && !leftj && !upj;
-      int pre, total;
-      ScanI(ts_i).ExclusiveSum(opens ? 1 : 0, pre, total);
-      const int up = upj ? lab[p - cols] : 0;
-      const int val = upj ? up : (opens ? s_next + pre : INT_MAX);
-      SegMin o;
-      ScanS(ts_s).InclusiveScan(SegMin{leftj ? 0 : 1, val}, o, SegMinOp());
-      const int run = (o.start || base == 0) ? o.v : min(s_carry, o.v);
-      if (in) lab[p] = labelled ? run : 0;
-      __syncthreads();  // this chunk's labels are written; s_next and s_carry are read
-      if (in && leftj && upj) {
-        const int left = lab[p - 1];
-        if (left != up) {
-          const int big = left > up ? left : up, small = left > up ? up : left;
-          atomicMax(&join[big], ((unsigned long long)p << 32) | (unsigned)small);
+    for (int base = 0; base < cols; base += kConnectThreads * kConnectItems) {
+      const int x0 = base + tid * kConnectItems;
+      const size_t p0 = (size_t)y * cols + x0;
+      bool in[kConnectItems], leftj[kConnectItems], upj[kConnectItems], labelled[kConnectItems], opens[kConnectItems];
+      int up[kConnectItems];
+      bool left_zero = x0 > 0 && x0 <= cols && img[p0 - 1] == 0;
+      RunScan agg{0, INT_MAX, 0};
+#pragma unroll
+      for (int i = 0; i < kConnectItems; ++i) {
+        in[i] = x0 + i < cols;
+        const int v = in[i] ? img[p0 + i] : 255;
+        labelled[i] = in[i] && v != 255;
+        const bool zero = in[i] && v == 0;
+        leftj[i] = zero && left_zero;
+        upj[i] = zero && y > 0 && img[p0 + i - cols] == 0;
+        up[i] = upj[i] ? lab[p0 + i - cols] : INT_MAX;  // this thread wrote it
+        opens[i] = labelled[i] && !leftj[i] && !upj[i];
+        left_zero = zero;
+        agg = RunScanOp()(agg, RunScan{leftj[i] ? 0 : 1, up[i], opens[i] ? 1 : 0});
+      }
+      RunScan pre, total;
+      Scan(ts).ExclusiveScan(agg, pre, RunScan{0, INT_MAX, 0}, RunScanOp(), total);
+      const int next = s_next, carry = s_carry;
+      int run[kConnectItems], last = 0;
+      RunScan o = pre;
+#pragma unroll
+      for (int i = 0; i < kConnectItems; ++i) {
+        o = RunScanOp()(o, RunScan{leftj[i] ? 0 : 1, up[i], opens[i] ? 1 : 0});
+        run[i] = !o.start ? min(carry, o.v) : o.v != INT_MAX ? o.v : next + o.opens - 1;
+        if (!labelled[i]) run[i] = 0;
+        if (in[i]) {
+          lab[p0 + i] = run[i];
+          last = run[i];
         }
       }
-      if (x == min(base + kConnectThreads, cols) - 1) s_carry = run;
-      if (tid == 0) s_next += total;
+      s_last[tid] = last;
+      __syncthreads();  // this step's last labels are written; s_next and s_carry are read
+      int left = tid > 0 ? s_last[tid - 1] : carry;
+#pragma unroll
+      for (int i = 0; i < kConnectItems; ++i) {
+        if (leftj[i] && upj[i] && left != up[i]) {
+          const int big = left > up[i] ? left : up[i], small = left > up[i] ? up[i] : left;
+          atomicMax(&join[big], ((unsigned long long)(p0 + i) << 32) | (unsigned)small);
+        }
+        left = run[i];
+      }
+      const int end = min(base + kConnectThreads * kConnectItems, cols) - 1;
+      if (end >= x0 && end < x0 + kConnectItems) s_carry = last;
+      if (tid == 0) s_next = next + total.opens;
       __syncthreads();
     }
   }
@@ -377,17 +407,34 @@ __global__ void k_list_large(const int *__restrict__ counts, int cap, int weak_t
 
 // ---- HoughLinesP on one weak region's outer border, and its segments drawn --------------------
 // cv::HoughLinesP(img_weak, 1, CV_PI / 180, thr, thr, thr) (DPE.cpp:185-188): OpenCV's progressive
-// probabilistic Hough transform.  One CTA per region runs the reference's sequential loop; the
-// votes of a point over the angles are spread over the threads, the rest (the generator, the
-// segment walks) runs on thread 0.  The walks are bounded by the image, a guard counts steps.
+// probabilistic Hough transform, one region per CTA or cluster of CTAs, with the results of the
+// reference's sequential loop:
+//   * the order of the points depends only on the generator and the number left, so a warp that has no
+//     angles draws the next 32 points while the others vote;
+//   * a thread owns an angle and votes for up to kHoughVotes points at once: the counts it would see are
+//     the stored ones plus its own earlier votes of the round for the same bin.  Only when some count
+//     reaches the threshold does a point's argmax matter: the votes up to the first such point are
+//     stored, its segment is handled, and the next round starts behind it.  Otherwise all are stored;
+//   * the counts lie in shared memory, 16 bits each (a bin cannot hold more points than its line has
+//     pixels): a vote touches 180 rows, from L2 or L1 180 separate lines.  Where one CTA's shared
+//     memory is too small, 2, 4 or 8 CTAs of a cluster split the angles; each keeps its own copy of the
+//     mask and of the order and makes every walk, and a round exchanges only which points reached the
+//     threshold and with what angle;
+//   * a segment's walk looks at 16 steps of both directions at a time, and the mask is one bit per pixel.
+// What bounds it is the chain of rounds of the largest border (on a 1600x1200 view 30 k points, 17 k of
+// them voting, 2088 segments).  One point at a time, every load from L2, took 68 ms; rounds with the counts
+// in global memory 17 ms; now 11 ms, a chain of short dependent pieces: 900 cycles of a round to vote,
+// 1100 at its barrier, 2500 of a segment for its walk.
 struct HoughArgs {
   const int *labels;  // first labelling, w x h
   const int *regions; // region labels, one per CTA
   int w, h, threshold, line_length, line_gap, numangle, numrho;
   const float2 *tab;  // (cos, sin) / rho in float, from the host's libm as OpenCV computes it
-  uint8_t *mask;      // per CTA: w*h
+  unsigned *mask;     // per CTA: w*h bits; null: in shared memory (it is there whenever the counts are)
   int2 *points;       // per CTA: w*h
-  int *accum;         // per CTA: numangle*numrho
+  short *accum;       // per region: numangle*len counts; null: in shared memory
+  int first, len;     // the bins that a point of the image can vote for
+  int split;          // CTAs of a cluster that share a region's angles
   int4 *lines;        // per CTA: line_cap
   int line_cap;
   uint8_t *dst;       // the thresholded Roberts map the segments are drawn on
@@ -415,23 +462,49 @@ __device__ void draw_line8(uint8_t *img, int width, int x1, int y1, int x2, int 
   }
 }
 
-constexpr int kHoughThreads = 256;
+constexpr int kHoughThreads = 256, kHoughVotes = 8, kHoughMaxSplit = 8;
+// Shared bytes a CTA may take for the walk, the mask and the counts.
+constexpr size_t kHoughShared = 200 * 1024;
+inline size_t hough_walk_bytes(int w, int h) { return (size_t)2 * (std::max(w, h) + 2) * sizeof(int2); }
+inline size_t hough_mask_words(size_t pixels) { return (pixels + 31) / 32; }
+
+inline size_t hough_acc_bytes(int numangle, int split, int len) {
+  return (size_t)((numangle + split - 1) / split) * len * sizeof(short);
+}
 
 __global__ void __launch_bounds__(kHoughThreads) k_hough_region(const __grid_constant__ HoughArgs a) {
-  extern __shared__ int2 walk[];  // pixels withdrawn by one segment, both directions
+  extern __shared__ int2 walk[];  // pixels withdrawn by one segment, both directions; then the mask, the counts
   typedef cub::BlockScan<int, kHoughThreads> ScanI;
-  typedef cub::BlockReduce<unsigned long long, kHoughThreads> RedU;
   __shared__ typename ScanI::TempStorage ts_i;
-  __shared__ typename RedU::TempStorage ts_r;
-  __shared__ int s_count, s_idx_x, s_idx_y, s_skip, s_nwalk, s_good, s_nlines, s_best_n, s_best_v;
-  const int tid = threadIdx.x;
-  const int region = a.regions[blockIdx.x];
+  __shared__ int s_count, s_nwalk, s_nlines;
+  __shared__ int2 s_pt[2][32];
+  __shared__ float2 s_tab[kHoughThreads];
+  // per round: each CTA's best (count, angle) of every point that reaches the threshold there
+  // (and whether there is any)
+  __shared__ unsigned s_key[3][kHoughMaxSplit][kHoughVotes], s_any[3];
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int split = a.split, rank = split > 1 ? (int)cluster.block_rank() : 0;
+  auto barrier = [&]() {
+    if (split > 1) cluster.sync();
+    else __syncthreads();
+  };
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kDrawWarp = kHoughThreads / 32 - 1;  // no angle is its (numangle is 180)
+  const int region = a.regions[blockIdx.x / split];
   const int w = a.w, h = a.h, n = w * h;
-  uint8_t *mask = a.mask + (size_t)blockIdx.x * n;
-  int2 *pts = a.points + (size_t)blockIdx.x * n;
-  int *acc = a.accum + (size_t)blockIdx.x * a.numangle * a.numrho;
-  int4 *lines = a.lines + (size_t)blockIdx.x * a.line_cap;
   const int walk_cap = 2 * (max(w, h) + 2);
+  unsigned *shared_mask = reinterpret_cast<unsigned *>(walk + walk_cap);
+  unsigned *mask = a.mask ? a.mask + (size_t)blockIdx.x * ((n + 31) / 32) : shared_mask;
+  const int per = (a.numangle + split - 1) / split;  // angles of this CTA: rank * per + 0 .. per - 1
+  short *acc = a.accum ? a.accum + (size_t)blockIdx.x * a.numangle * a.len
+                       : reinterpret_cast<short *>(shared_mask + (n + 31) / 32);
+  auto masked = [&](int x, int y) {
+    const int p = y * w + x;
+    return ((mask[p >> 5] >> (p & 31)) & 1u) != 0;
+  };
+  int2 *pts = a.points + (size_t)blockIdx.x * n;
+  int4 *lines = a.lines + (size_t)(blockIdx.x / split) * a.line_cap;
   // the region's outer border in raster order (DPE.cpp:168-182): not the region, 4-adjacent to it
   if (tid == 0) s_count = 0;
   __syncthreads();
@@ -443,118 +516,246 @@ __global__ void __launch_bounds__(kHoughThreads) k_hough_region(const __grid_con
       on = (x > 0 && a.labels[p - 1] == region) || (x < w - 1 && a.labels[p + 1] == region) ||
            (y > 0 && a.labels[p - w] == region) || (y < h - 1 && a.labels[p + w] == region);
     }
+    const unsigned bits = __ballot_sync(0xffffffffu, on);
+    if (lane == 0 && p < n) mask[p >> 5] = bits;
+    if (!__syncthreads_or(on)) continue;
     int pre, total;
     ScanI(ts_i).ExclusiveSum(on ? 1 : 0, pre, total);
-    if (p < n) mask[p] = on ? 1 : 0;
     if (on) pts[s_count + pre] = make_int2(p % w, p / w);
     __syncthreads();
     if (tid == 0) s_count += total;
     __syncthreads();
   }
-  for (int i = tid; i < a.numangle * a.numrho; i += kHoughThreads) acc[i] = 0;
+  for (int i = tid; i < per * a.len; i += kHoughThreads) acc[i] = 0;
   if (tid == 0) s_nlines = 0;
-  __syncthreads();
-  uint64_t state = ~0ull;  // cv::RNG((uint64)-1), thread 0 only
+  for (int i = tid; i < 3 * kHoughMaxSplit * kHoughVotes; i += kHoughThreads) (&s_key[0][0][0])[i] = 0;
+  if (tid < 3) s_any[tid] = 0;
+  if (tid < a.numangle) s_tab[tid] = a.tab[tid];
+  barrier();  // every CTA's keys are ready for the others
+  uint64_t state = ~0ull;  // cv::RNG((uint64)-1), the drawing warp only
   const int shift = 16;
-  for (int count = s_count; count > 0; --count) {
-    // Every thread has read the previous point's shared values (s_skip, s_idx_*, s_best_*) before
-    // thread 0 overwrites them: the `continue`s below leave an iteration without a later barrier.
-    __syncthreads();
-    if (tid == 0) {
+  int left = s_count;  // points not drawn yet
+  // The next m <= 32 points of the order (one warp): a drawn point's place is taken by the last one.
+  // Lane i makes draw i.  The places drawn do not depend on the points, so the loads go out together; a
+  // place that an earlier draw of the batch filled holds what that draw put there.
+  auto draw = [&](int2 *out, int m) {
+    uint64_t mine = 0;
+    for (int i = 0; i < m; ++i) {
       state = (uint64_t)(unsigned)state * 4164903690u + (unsigned)(state >> 32);
-      const int idx = (int)((unsigned)state % (unsigned)count);
-      const int2 pt = pts[idx];
-      pts[idx] = pts[count - 1];
-      s_idx_x = pt.x;
-      s_idx_y = pt.y;
-      s_skip = mask[pt.y * w + pt.x] ? 0 : 1;
+      if (i == lane) mine = state;
     }
-    __syncthreads();
-    if (s_skip) continue;  // uniform: already withdrawn by an earlier segment
-    const int j = s_idx_x, i = s_idx_y;
-    // vote, and the first angle with the largest count.  Counts can be negative: a segment
-    // withdraws the votes of every mask pixel on it, also of pixels that have not voted yet (as
-    // OpenCV does).  The key's high word is the count with its sign bit flipped, so unsigned
-    // order is the counts' signed order; the low word prefers the smaller angle on ties.
-    unsigned long long best = 0;
-    for (int nn = tid; nn < a.numangle; nn += kHoughThreads) {
-      const int r = hough_bin(a, a.tab[nn], j, i);
-      const int val = ++acc[(size_t)nn * a.numrho + r];
-      const unsigned long long key =
-          ((unsigned long long)((unsigned)val ^ 0x80000000u) << 32) | (unsigned)(0x7fffffff - nn);
-      best = key > best ? key : best;
+    const bool in = lane < m;
+    const int end = left - lane - 1;
+    const int idx = in ? (int)((unsigned)mine % (unsigned)(end + 1)) : -1;
+    int2 at_idx = make_int2(0, 0), at_end = make_int2(0, 0);
+    if (in) {
+      at_idx = pts[idx];
+      at_end = pts[end];
     }
-    best = RedU(ts_r).Reduce(best, cub::Max());
-    if (tid == 0) {
-      s_best_v = (int)((unsigned)(best >> 32) ^ 0x80000000u);
-      s_best_n = 0x7fffffff - (int)(best & 0xffffffffu);
-    }
-    __syncthreads();
-    if (s_best_v < a.threshold) continue;  // uniform
-    if (tid == 0) {
-      const float2 t = a.tab[s_best_n];
-      const float fa = -t.y, fb = t.x;
-      int x0 = j, y0 = i, dx0, dy0;
-      bool xflag;
-      if (fabsf(fa) > fabsf(fb)) {
-        xflag = true;
-        dx0 = fa > 0 ? 1 : -1;
-        dy0 = __float2int_rn(__fdiv_rn(__fmul_rn(fb, (float)(1 << shift)), fabsf(fa)));
-        y0 = (y0 << shift) + (1 << (shift - 1));
-      } else {
-        xflag = false;
-        dy0 = fb > 0 ? 1 : -1;
-        dx0 = __float2int_rn(__fdiv_rn(__fmul_rn(fa, (float)(1 << shift)), fabsf(fb)));
-        x0 = (x0 << shift) + (1 << (shift - 1));
-      }
-      int ex[2] = {j, j}, ey[2] = {i, i};
-      for (int k = 0; k < 2; ++k) {
-        int gap = 0, x = x0, y = y0;
-        const int dx = k ? -dx0 : dx0, dy = k ? -dy0 : dy0;
-        for (int step = 0;; x += dx, y += dy, ++step) {
-          const int j1 = xflag ? x : x >> shift, i1 = xflag ? y >> shift : y;
-          if (j1 < 0 || j1 >= w || i1 < 0 || i1 >= h) break;
-          if (mask[i1 * w + j1]) {
-            gap = 0;
-            ex[k] = j1;
-            ey[k] = i1;
-          } else if (++gap > a.line_gap) {
-            break;
-          }
-          if (step > w + h + 4) { atomicExch(a.error, 1); break; }
+    bool store = in;
+    // rarely: a place drawn twice, or one of the last places drawn
+    const unsigned same = __match_any_sync(0xffffffffu, in ? idx : -1 - lane);
+    const bool clash = in && (__popc(same) > 1 || idx >= left - m);
+    if (__any_sync(0xffffffffu, clash)) {
+      for (int j = 0; j < m; ++j) {
+        const int fill = __shfl_sync(0xffffffffu, idx, j);
+        const int2 by = make_int2(__shfl_sync(0xffffffffu, at_end.x, j), __shfl_sync(0xffffffffu, at_end.y, j));
+        if (lane > j) {
+          if (idx == fill) at_idx = by;
+          if (end == fill) at_end = by;
+        } else if (lane < j && idx == fill) {
+          store = false;  // a later draw fills this place
         }
       }
-      const bool good = abs(ex[1] - ex[0]) >= a.line_length || abs(ey[1] - ey[0]) >= a.line_length;
-      int nw = 0;
-      for (int k = 0; k < 2; ++k) {
-        int x = x0, y = y0;
-        const int dx = k ? -dx0 : dx0, dy = k ? -dy0 : dy0;
-        for (int step = 0;; x += dx, y += dy, ++step) {
-          const int j1 = xflag ? x : x >> shift, i1 = xflag ? y >> shift : y;
-          if (j1 < 0 || j1 >= w || i1 < 0 || i1 >= h || step > w + h + 4) { atomicExch(a.error, 1); break; }
-          uint8_t &m = mask[i1 * w + j1];
+    }
+    if (in) out[lane] = at_idx;
+    if (store) pts[idx] = at_end;
+    __syncwarp();
+  };
+  const int ang = rank * per + tid;
+  const bool voter = tid < per && ang < a.numangle;
+  const float2 angle = voter ? s_tab[ang] : make_float2(0.f, 0.f);
+  short *row = acc + (size_t)(voter ? tid : 0) * a.len - a.first;
+  int cur = min(left, 32), par = 0, buf = 0;
+  if (warp == kDrawWarp) draw(s_pt[0], cur);
+  left -= cur;
+  __syncthreads();
+  while (cur > 0) {
+    const int ahead = min(left, 32);
+    if (warp == kDrawWarp) draw(s_pt[buf ^ 1], ahead);
+    left -= ahead;
+    int start = 0;
+    while (true) {
+      // the next points of the batch that no segment has withdrawn (every warp looks for itself)
+      bool on = false;
+      if (lane >= start && lane < cur) on = masked(s_pt[buf][lane].x, s_pt[buf][lane].y);
+      const unsigned all = __ballot_sync(0xffffffffu, on);
+      if (!all) break;  // uniform: the mask is the same for every warp
+      unsigned live = all;
+      int bin[kHoughVotes], val[kHoughVotes], at[kHoughVotes];
+      unsigned hit = 0;
+#pragma unroll
+      for (int i = 0; i < kHoughVotes; ++i) {
+        at[i] = live ? __ffs(live) - 1 : -1;
+        live &= live - 1;
+        bin[i] = -1 - i;
+        val[i] = 0;
+        if (voter && at[i] >= 0) {
+          const int2 pt = s_pt[buf][at[i]];
+          bin[i] = hough_bin(a, angle, pt.x, pt.y);
+          val[i] = row[bin[i]];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kHoughVotes; ++i) {
+#pragma unroll
+        for (int j = 0; j < i; ++j)
+          if (bin[j] == bin[i]) val[i] = val[j];  // the latest earlier vote of the round for this bin
+        val[i] += 1;
+        if (voter && at[i] >= 0 && val[i] >= a.threshold) hit |= 1u << i;
+      }
+      // The first angle with the largest count, for every point that reaches the threshold: the count is
+      // not negative there; the low byte prefers the smaller angle on ties.
+      const unsigned whit = __reduce_or_sync(0xffffffffu, hit);
+#pragma unroll
+      for (int i = 0; i < kHoughVotes; ++i) {
+        if (!((whit >> i) & 1u)) continue;
+        const unsigned key =
+            __reduce_max_sync(0xffffffffu, ((hit >> i) & 1u) ? (unsigned)val[i] << 8 | (unsigned)(255 - ang) : 0u);
+        if (lane < split) {  // to every CTA of the cluster
+          unsigned *to = &s_key[par][rank][i];
+          atomicMax(split > 1 ? cluster.map_shared_rank(to, lane) : to, key);
+        }
+      }
+      if (whit && lane < split) atomicOr(split > 1 ? cluster.map_shared_rank(&s_any[par], lane) : &s_any[par], whit);
+      barrier();
+      const unsigned any = s_any[par];
+      const int upto = any ? __ffs(any) : kHoughVotes;  // votes of points before this one count now
+      // the place in the batch of the last of these points
+      unsigned rest = all;
+      for (int i = min(upto, __popc(all)); i > 1; --i) rest &= rest - 1;
+      const int final_pt = __ffs(rest) - 1;
+      start = final_pt + 1;
+      if (voter) {
+#pragma unroll
+        for (int i = 0; i < kHoughVotes; ++i)
+          if (at[i] >= 0 && i < upto) row[bin[i]] = (short)val[i];
+      }
+      unsigned best = 0;
+      if (any)
+        for (int c = 0; c < split; ++c) best = max(best, s_key[par][c][upto - 1]);
+      // Free the slots of the round after next: their last readers are behind this round's barrier, their
+      // next writers behind the next one's.
+      const int old = par == 0 ? 2 : par - 1;
+      if (warp == kDrawWarp) {
+        for (int i = lane; i < kHoughMaxSplit * kHoughVotes; i += 32) (&s_key[old][0][0])[i] = 0;
+        if (lane == 0) s_any[old] = 0;
+      }
+      par = par == 2 ? 0 : par + 1;
+      const int2 pt = s_pt[buf][final_pt];
+      if (!any) continue;  // uniform
+      if (warp == 0) {
+        const int j = pt.x, i = pt.y;
+        const float2 t = s_tab[255 - (int)(best & 255u)];
+        const float fa = -t.y, fb = t.x;
+        int x0 = j, y0 = i, dx0, dy0;
+        bool xflag;
+        if (fabsf(fa) > fabsf(fb)) {
+          xflag = true;
+          dx0 = fa > 0 ? 1 : -1;
+          dy0 = __float2int_rn(__fdiv_rn(__fmul_rn(fb, (float)(1 << shift)), fabsf(fa)));
+          y0 = (y0 << shift) + (1 << (shift - 1));
+        } else {
+          xflag = false;
+          dy0 = fb > 0 ? 1 : -1;
+          dx0 = __float2int_rn(__fdiv_rn(__fmul_rn(fa, (float)(1 << shift)), fabsf(fb)));
+          x0 = (x0 << shift) + (1 << (shift - 1));
+        }
+        // step s of direction k; the major coordinate moves by one a step, so every step is another pixel
+        // and a walk leaves the image for good
+        auto step = [&](int k, int s) {
+          const int x = x0 + (k ? -dx0 : dx0) * s, y = y0 + (k ? -dy0 : dy0) * s;
+          return xflag ? make_int2(x, y >> shift) : make_int2(x >> shift, y);
+        };
+        // Half the warp per direction, 16 steps of each at a time.  Every mask pixel up to where a walk ends
+        // is withdrawn, whether the segment counts or not, so one pass finds and clears them.
+        const int k = lane >> 4, hl = lane & 15;
+        int last = 0, nw = 0;  // last: the direction's last mask pixel so far
+        bool open = true;
+        for (int base = 0; __any_sync(0xffffffffu, open); base += 16) {
+          const int2 q = step(k, base + hl);
+          const bool in = open && q.x >= 0 && q.x < w && q.y >= 0 && q.y < h;
+          const unsigned ins = __ballot_sync(0xffffffffu, in);
+          const unsigned hits = __ballot_sync(0xffffffffu, in && masked(q.x, q.y));
+          unsigned set = 0;
+          if (open) {
+            const unsigned out = ~(ins >> (16 * k)) & 0xffffu;
+            const int inside = out ? __ffs(out) - 1 : 16;
+            set = (hits >> (16 * k)) & ((1u << inside) - 1u);
+            // reach: the steps within line_gap behind a set one (or behind the last of earlier steps); the
+            // walk ends at the first that is not
+            unsigned reach = set;
+            for (int have = 0; have < min(a.line_gap, 15);) {
+              const int by = min(have + 1, min(a.line_gap, 15) - have);
+              reach |= reach << by;
+              have += by;
+            }
+            const int tail = last + a.line_gap - base;  // the last step the earlier ones reach
+            if (tail >= 0) reach |= tail >= 15 ? 0xffffu : (2u << tail) - 1u;
+            const unsigned gap = ~reach & 0xffffu;
+            const int stop = gap ? __ffs(gap) - 1 : 16;
+            set &= (1u << stop) - 1u;
+            if (set) last = base + 31 - __clz(set);
+            if (stop < 16 || inside < 16) open = false;
+            if (base > w + h + 36) {
+              atomicExch(a.error, 1);
+              open = false;
+            }
+          }
+          // the second direction's first step is the first's: found and cleared there
+          const bool m = ((set >> hl) & 1u) && !(k == 1 && base + hl == 0);
+          const unsigned take = __ballot_sync(0xffffffffu, m);
           if (m) {
-            if (good && nw < walk_cap) walk[nw++] = make_int2(j1, i1);
-            m = 0;
+            const int to = nw + __popc(take & ((1u << lane) - 1u));
+            if (to < walk_cap) walk[to] = q;
+            const int p = q.y * w + q.x;
+            atomicAnd(&mask[p >> 5], ~(1u << (p & 31)));
           }
-          if (i1 == ey[k] && j1 == ex[k]) break;
+          nw += __popc(take);
+        }
+        const int2 e = step(k, last);
+        const int2 e0 = make_int2(__shfl_sync(0xffffffffu, e.x, 0), __shfl_sync(0xffffffffu, e.y, 0));
+        const int2 e1 = make_int2(__shfl_sync(0xffffffffu, e.x, 16), __shfl_sync(0xffffffffu, e.y, 16));
+        const bool good = abs(e1.x - e0.x) >= a.line_length || abs(e1.y - e0.y) >= a.line_length;
+        if (lane == 0) {
+          s_nwalk = good ? min(nw, walk_cap) : 0;
+          if (good && s_nlines < a.line_cap) lines[s_nlines] = make_int4(e0.x, e0.y, e1.x, e1.y);
+          if (good) s_nlines++;
         }
       }
-      s_nwalk = good ? nw : 0;
-      s_good = good ? 1 : 0;
-      if (good && s_nlines < a.line_cap) lines[s_nlines] = make_int4(ex[0], ey[0], ex[1], ey[1]);
-      if (good) s_nlines++;
+      __syncthreads();
+      // withdraw the segment's votes: each thread owns whole angle rows, so no two threads meet
+      if (voter) {
+        const int m = s_nwalk;
+        int q = 0;
+        for (; q + 4 <= m; q += 4) {  // four bins ahead of the counts they change
+          int b4[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) b4[i] = hough_bin(a, angle, walk[q + i].x, walk[q + i].y);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) row[b4[i]] -= 1;
+        }
+        for (; q < m; ++q) row[hough_bin(a, angle, walk[q].x, walk[q].y)] -= 1;
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    // withdraw the segment's votes: each thread owns whole angle rows, so no two threads meet
-    for (int q = 0; q < s_nwalk; ++q) {
-      const int2 pq = walk[q];
-      for (int nn = tid; nn < a.numangle; nn += kHoughThreads)
-        --acc[(size_t)nn * a.numrho + hough_bin(a, a.tab[nn], pq.x, pq.y)];
-    }
-    __syncthreads();
+    __syncthreads();  // the next points are drawn, this batch's are read
+    cur = ahead;
+    buf ^= 1;
   }
   __syncthreads();
+  if (split > 1) cluster.sync();  // no CTA leaves while another may write to its keys
+  if (rank != 0) return;
   if (s_nlines > a.line_cap && tid == 0) atomicExch(a.error, 2);
   const int nl = min(s_nlines, a.line_cap);
   for (int q = tid; q < nl; q += kHoughThreads) draw_line8(a.dst, w, lines[q].x, lines[q].y, lines[q].z, lines[q].w);
@@ -779,6 +980,7 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
     const float theta = (float)(3.14159265358979323846 / 180.0);
     int numangle = (int)std::floor(3.14159265358979323846 / theta) + 1;
     if (numangle > 1 && std::fabs(3.14159265358979323846 - (numangle - 1) * (double)theta) < theta / 2) --numangle;
+    if (numangle > kHoughThreads - 32) return DPE_ERR_INVALID_ARGUMENT;  // 180: an angle per thread, a warp to draw
     const int numrho = (int)std::nearbyint((double)((c2 + r2) * 2 + 1));
     std::vector<float2> tab(numangle);
     for (int k = 0; k < numangle; ++k)
@@ -791,19 +993,42 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
     ha.w = c2; ha.h = r2; ha.threshold = thr; ha.line_length = thr; ha.line_gap = thr;
     ha.numangle = numangle; ha.numrho = numrho;
     ha.tab = tab_d;
-    ha.mask = A.get<uint8_t>("lb_mask", n2 * nreg);
-    ha.points = A.get<int2>("lb_points", n2 * nreg);
-    ha.accum = A.get<int>("lb_accum", (size_t)numangle * numrho * nreg);
+    // Bins a point can vote for: x cos + y sin lies in [-(c2 - 1), diagonal] (a bin more on each side for
+    // the rounding).
+    ha.first = (numrho - 1) / 2 - c2;
+    ha.len = std::min(c2 + (int)std::ceil(std::sqrt((double)c2 * c2 + (double)r2 * r2)) + 2, numrho - ha.first);
+    const size_t walk_bytes = hough_walk_bytes(c2, r2), mask_bytes = hough_mask_words(n2) * sizeof(unsigned);
+    int split = 1;
+    auto shared = [&](int k) { return walk_bytes + mask_bytes + hough_acc_bytes(numangle, k, ha.len); };
+    while (split < kHoughMaxSplit && shared(split) > kHoughShared) split *= 2;
+    const bool in_shared = shared(split) <= kHoughShared;
+    if (!in_shared) split = 1;
+    ha.split = split;
+    ha.mask = in_shared ? nullptr : A.get<unsigned>("lb_mask", hough_mask_words(n2) * nreg);
+    ha.points = A.get<int2>("lb_points", n2 * nreg * split);
+    ha.accum = in_shared ? nullptr : A.get<short>("lb_accum", (size_t)numangle * ha.len * nreg);
     ha.lines = A.get<int4>("lb_lines", (size_t)line_cap * nreg);
     ha.line_cap = line_cap;
     ha.dst = dst;
     ha.error = error;
     if (!A.ok()) return DPE_ERR_OUT_OF_MEMORY;
     DPE_TRY(cudaMemcpyAsync(tab_d, tab.data(), numangle * sizeof(float2), cudaMemcpyHostToDevice, s));
-    const size_t walk_bytes = (size_t)2 * (std::max(c2, r2) + 2) * sizeof(int2);
-    if (walk_bytes > 48 * 1024)
-      DPE_TRY(cudaFuncSetAttribute(k_hough_region, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_bytes));
-    DPE_TIMED(ctx, KID_EDGE_LABELS, s, k_hough_region<<<nreg, kHoughThreads, walk_bytes, s>>>(ha));
+    const size_t smem = in_shared ? shared(split) : walk_bytes;
+    if (smem > 48 * 1024)
+      DPE_TRY(cudaFuncSetAttribute(k_hough_region, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {(unsigned)split, 1, 1};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nreg * split));
+    cfg.blockDim = dim3(kHoughThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaError_t launched = cudaSuccess;
+    DPE_TIMED(ctx, KID_EDGE_LABELS, s, launched = cudaLaunchKernelEx(&cfg, k_hough_region, ha));
+    DPE_TRY(launched);
     DPE_LAUNCHED("k_hough_region", s);
   }
   // to the level, threshold, border rule, second labelling, small regions -1 (DPE.cpp:224-285)
