@@ -58,6 +58,8 @@ struct FuseArgs {
   int ns;
   int src[kMaxSrc];
   const FuseView *views;  // device array
+  // a pixel's entries together: the rounds read them one after another, and find the next in the line
+  // they have (source-major, contiguous per warp, the rounds took 2.1 ms against 1.8)
   int *entry_q;           // W*H*ns: source pixel index, -1 when the entry is not consistent
   double *entry_score;    // W*H*ns: exp(-(e + 200 dd + 10 angle)) of a consistent entry
   uint8_t *status;        // W*H: 1 accepted, 3 rejected (this round), 2 not a candidate
@@ -94,81 +96,131 @@ template <class T> __device__ __forceinline__ void project(const T X[3], const d
   v = ((T)c.K[3] * tx + (T)c.K[4] * ty + (T)c.K[5] * tz) / d;
 }
 
-// Per reference pixel: candidate test and every source entry (DPE.cpp:1468-1516).
-__global__ void k_entries(const __grid_constant__ FuseArgs f) {
+// A camera as the FP64 mode computes with it, converted and its centre composed once per block: both are
+// the same for every pixel, and conversions run at an eighth of the FP64 rate.
+struct CameraD {
+  double K[9], R[9], t[3], C[3];
+};
+__device__ __forceinline__ void camera_d(const dpe_camera &c, CameraD &o) {
+  for (int i = 0; i < 9; ++i) {
+    o.K[i] = (double)c.K[i];
+    o.R[i] = (double)c.R[i];
+  }
+  for (int i = 0; i < 3; ++i) o.t[i] = (double)c.t[i];
+  for (int i = 0; i < 3; ++i) o.C[i] = -(o.R[i] * o.t[0] + o.R[3 + i] * o.t[1] + o.R[6 + i] * o.t[2]);
+}
+// world_point<double> and project<double> on such a camera: the same operations.
+__device__ __forceinline__ void world_point(double x, double y, double depth, const CameraD &c, double out[3]) {
+  const double px = depth * (x - c.K[2]) / c.K[0];
+  const double py = depth * (y - c.K[5]) / c.K[4];
+  const double pz = depth;
+  out[0] = (c.R[0] * px + c.R[3] * py + c.R[6] * pz) + c.C[0];
+  out[1] = (c.R[1] * px + c.R[4] * py + c.R[7] * pz) + c.C[1];
+  out[2] = (c.R[2] * px + c.R[5] * py + c.R[8] * pz) + c.C[2];
+}
+__device__ __forceinline__ void project(const double X[3], const CameraD &c, double &u, double &v, double &d) {
+  const double tx = c.R[0] * X[0] + c.R[1] * X[1] + c.R[2] * X[2] + c.t[0];
+  const double ty = c.R[3] * X[0] + c.R[4] * X[1] + c.R[5] * X[2] + c.t[1];
+  const double tz = c.R[6] * X[0] + c.R[7] * X[1] + c.R[8] * X[2] + c.t[2];
+  d = c.K[6] * tx + c.K[7] * ty + c.K[8] * tz;
+  u = (c.K[0] * tx + c.K[1] * ty + c.K[2] * tz) / d;
+  v = (c.K[3] * tx + c.K[4] * ty + c.K[5] * tz) / d;
+}
+
+// Per reference pixel: candidate test and every source entry (DPE.cpp:1468-1516).  In the FP64 mode it is
+// bound by the FP64 pipe (nine divisions, an arc cosine and an exponential per pair): the cameras come
+// converted from shared memory, and the last two are taken only for pairs that pass the first two tests.
+// Ten 1600x1200 views: 6.91 -> 5.52 ms.
+template <bool kDouble>
+__global__ void __launch_bounds__(256) k_entries(const __grid_constant__ FuseArgs f) {
+  __shared__ CameraD cams[kDouble ? kMaxSrc + 1 : 1];  // the sources, then the reference
   const FuseView &V = f.views[f.ref];
+  if (kDouble) {
+    for (int j = threadIdx.x; j <= f.ns; j += blockDim.x) camera_d(f.views[j < f.ns ? f.src[j] : f.ref].cam, cams[j]);
+    __syncthreads();
+  }
+  const int npix = V.W * V.H;
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= V.W * V.H) return;
+  if (pix >= npix) return;
   const int c = pix % V.W, r = pix / V.W;
-  int *eq = f.entry_q + (size_t)pix * f.ns;
-  double *es = f.entry_score + (size_t)pix * f.ns;
-  for (int j = 0; j < f.ns; ++j) eq[j] = -1;
   uint8_t st = 2;
   const float ref_depth = V.depth[pix];
-  if (!(V.block && V.block[pix] < 128) && V.mask[pix] != 1 && !(ref_depth <= 0.0)) {
-    const float rn0 = V.normal[3 * pix], rn1 = V.normal[3 * pix + 1], rn2 = V.normal[3 * pix + 2];
-    double Xd[3];
-    float Xf[3];
-    world_point<double>((double)c, (double)r, (double)ref_depth, V.cam, Xd);
-    world_point<float>((float)c, (float)r, ref_depth, V.cam, Xf);
-    int n_pass = 0;
-    double dyn_d = 0.0;
-    float dyn_f = 0.0f;
-    for (int j = 0; j < f.ns; ++j) {
-      const FuseView &S = f.views[f.src[j]];
+  const bool visited = !(V.block && V.block[pix] < 128) && V.mask[pix] != 1 && !(ref_depth <= 0.0);
+  float rn0 = 0.f, rn1 = 0.f, rn2 = 0.f;
+  double Xd[3] = {0.0, 0.0, 0.0};
+  float Xf[3] = {0.f, 0.f, 0.f};
+  if (visited) {
+    rn0 = V.normal[3 * pix]; rn1 = V.normal[3 * pix + 1]; rn2 = V.normal[3 * pix + 2];
+    if (kDouble) world_point((double)c, (double)r, (double)ref_depth, cams[f.ns], Xd);
+    else world_point<float>((float)c, (float)r, ref_depth, V.cam, Xf);
+  }
+  int n_pass = 0;
+  double dyn_d = 0.0;
+  float dyn_f = 0.0f;
+  for (int j = 0; j < f.ns; ++j) {
+    const FuseView &S = f.views[f.src[j]];
+    int q = -1;
+    double score = 0.0;
+    if (visited) {
       int sr, sc;
-      if (f.mode == DPE_FUSE_FP64) {
+      if (kDouble) {
         double u, v, pd;
-        project<double>(Xd, S.cam, u, v, pd);
+        project(Xd, cams[j], u, v, pd);
         sr = (int)(v + 0.5); sc = (int)(u + 0.5);
       } else {
         float u, v, pd;
         project<float>(Xf, S.cam, u, v, pd);
         sr = (int)(v + 0.5f); sc = (int)(u + 0.5f);
       }
-      if (!(sc >= 0 && sc < S.W && sr >= 0 && sr < S.H)) continue;
-      const int sp = sr * S.W + sc;
-      if (S.mask[sp] == 1) continue;
-      const float sd = S.depth[sp];
-      if (sd <= 0.0) continue;
-      const float sn0 = S.normal[3 * sp], sn1 = S.normal[3 * sp + 1], sn2 = S.normal[3 * sp + 2];
-      bool ok;
-      double score;
-      if (f.mode == DPE_FUSE_FP64) {
-        double T[3], u, v, pd;
-        world_point<double>((double)sc, (double)sr, (double)sd, S.cam, T);
-        project<double>(T, V.cam, u, v, pd);
-        const double ex = (double)c - u, ey = (double)r - v;
-        const double reproj = sqrt(ex * ex + ey * ey);
-        const double rel = fabs(pd - (double)ref_depth) / (double)ref_depth;
-        const double dot = (double)rn0 * sn0 + (double)rn1 * sn1 + (double)rn2 * sn2;
-        double ang = acos(dot);
-        if (ang != ang) ang = 0.0;
-        ok = reproj < 2.0 && rel < 0.01 && ang < (double)0.174533f;
-        score = exp(-(reproj + 200.0 * rel + ang * 10.0));
-      } else {
-        float T[3], u, v, pd;
-        world_point<float>((float)sc, (float)sr, sd, S.cam, T);
-        project<float>(T, V.cam, u, v, pd);
-        const float ex = (float)c - u, ey = (float)r - v;
-        const float reproj = (float)sqrt((double)ex * (double)ex + (double)ey * (double)ey);
-        const float rel = fabsf(pd - ref_depth) / ref_depth;
-        const float dot = rn0 * sn0 + rn1 * sn1 + rn2 * sn2;
-        float ang = acosf(dot);
-        if (ang != ang) ang = 0.0f;
-        ok = reproj < 2.0f && rel < 0.01f && ang < 0.174533f;
-        score = (double)(float)exp(-(double)(reproj + 200 * rel + ang * 10));
+      if (sc >= 0 && sc < S.W && sr >= 0 && sr < S.H) {
+        const int sp = sr * S.W + sc;
+        const float sd = S.depth[sp];
+        if (S.mask[sp] != 1 && !(sd <= 0.0)) {
+          const float sn0 = S.normal[3 * sp], sn1 = S.normal[3 * sp + 1], sn2 = S.normal[3 * sp + 2];
+          bool ok;
+          if (kDouble) {
+            double T[3], u, v, pd;
+            world_point((double)sc, (double)sr, (double)sd, cams[j], T);
+            project(T, cams[f.ns], u, v, pd);
+            const double ex = (double)c - u, ey = (double)r - v;
+            const double reproj = sqrt(ex * ex + ey * ey);
+            const double rel = fabs(pd - (double)ref_depth) / (double)ref_depth;
+            ok = reproj < 2.0 && rel < 0.01;
+            if (ok) {
+              const double dot = (double)rn0 * sn0 + (double)rn1 * sn1 + (double)rn2 * sn2;
+              double ang = acos(dot);
+              if (ang != ang) ang = 0.0;
+              ok = ang < (double)0.174533f;
+              if (ok) score = exp(-(reproj + 200.0 * rel + ang * 10.0));
+            }
+          } else {
+            float T[3], u, v, pd;
+            world_point<float>((float)sc, (float)sr, sd, S.cam, T);
+            project<float>(T, V.cam, u, v, pd);
+            const float ex = (float)c - u, ey = (float)r - v;
+            const float reproj = (float)sqrt((double)ex * (double)ex + (double)ey * (double)ey);
+            const float rel = fabsf(pd - ref_depth) / ref_depth;
+            const float dot = rn0 * sn0 + rn1 * sn1 + rn2 * sn2;
+            float ang = acosf(dot);
+            if (ang != ang) ang = 0.0f;
+            ok = reproj < 2.0f && rel < 0.01f && ang < 0.174533f;
+            if (ok) score = (double)(float)exp(-(double)(reproj + 200 * rel + ang * 10));
+          }
+          if (ok) {
+            q = sp;
+            n_pass++;
+            dyn_d += score;
+            dyn_f += (float)score;
+          }
+        }
       }
-      if (!ok) continue;
-      eq[j] = sp;
-      es[j] = score;
-      n_pass++;
-      dyn_d += score;
-      dyn_f += (float)score;
     }
-    // the starting point of the rounds: the decision with every entry live
-    if (n_pass > 0) st = fuse_accept(f, V, pix, n_pass, dyn_d, dyn_f) ? 1 : 3;
+    const size_t at = (size_t)pix * f.ns + j;
+    f.entry_q[at] = q;
+    if (q >= 0) f.entry_score[at] = score;
   }
+  // the starting point of the rounds: the decision with every entry live
+  if (n_pass > 0) st = fuse_accept(f, V, pix, n_pass, dyn_d, dyn_f) ? 1 : 3;
   f.status[pix] = st;
 }
 
@@ -181,8 +233,8 @@ __global__ void k_claim(const __grid_constant__ FuseArgs f, int npix, unsigned s
   if (pix >= npix || f.status[pix] != 1) return;
   const int *eq = f.entry_q + (size_t)pix * f.ns;
   const unsigned long long key = ((unsigned long long)stamp << 32) | (unsigned)pix;
-  for (int j = 0; j < f.ns; ++j)
-    if (eq[j] >= 0) atomicMin(&f.views[f.src[j]].claim[eq[j]], key);
+  for (int j = 0; j < f.ns; ++j, ++eq)
+    if (*eq >= 0) atomicMin(&f.views[f.src[j]].claim[*eq], key);
 }
 
 // One round, second half: every candidate's decision from the round's claims.  An entry is live
@@ -193,18 +245,19 @@ __global__ void k_redecide(const __grid_constant__ FuseArgs f, int npix, unsigne
   if (pix >= npix) return;
   const uint8_t st = f.status[pix];
   if (st != 1 && st != 3) return;
-  const int *eq = f.entry_q + (size_t)pix * f.ns;
-  const double *es = f.entry_score + (size_t)pix * f.ns;
   int n = 0;
   double dyn_d = 0.0;
   float dyn_f = 0.0f;
   for (int j = 0; j < f.ns; ++j) {
-    if (eq[j] < 0) continue;
-    const unsigned long long u = f.views[f.src[j]].claim[eq[j]];
+    const size_t at = (size_t)pix * f.ns + j;
+    const int q = f.entry_q[at];
+    if (q < 0) continue;
+    const unsigned long long u = f.views[f.src[j]].claim[q];
     if ((unsigned)(u >> 32) == stamp && (int)(unsigned)u < pix) continue;  // claimed earlier
+    const double e = f.entry_score[at];
     n++;
-    dyn_d += es[j];
-    dyn_f += (float)es[j];
+    dyn_d += e;
+    dyn_f += (float)e;
   }
   const uint8_t now = fuse_accept(f, V, pix, n, dyn_d, dyn_f) ? 1 : 3;
   if (now != st) {
@@ -225,17 +278,17 @@ __global__ void k_emit(const __grid_constant__ FuseArgs f, const int *offsets, l
   const int npix = V.W * V.H;
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
   if (pix >= npix || f.status[pix] != 1) return;
-  const int *eq = f.entry_q + (size_t)pix * f.ns;
   const int c = pix % V.W, r = pix / V.W;
   float col0 = V.bgr[3 * pix], col1 = V.bgr[3 * pix + 1], col2 = V.bgr[3 * pix + 2];
   int n = 0;
   for (int j = 0; j < f.ns; ++j) {
-    if (eq[j] < 0) continue;
+    const int q = f.entry_q[(size_t)pix * f.ns + j];
+    if (q < 0) continue;
     const FuseView &S = f.views[f.src[j]];
-    const unsigned long long u = S.claim[eq[j]];
+    const unsigned long long u = S.claim[q];
     if ((unsigned)(u >> 32) != stamp || (int)(unsigned)u != pix) continue;  // claimed by an earlier pixel
-    S.mask[eq[j]] = 1;
-    col0 += S.bgr[3 * eq[j]]; col1 += S.bgr[3 * eq[j] + 1]; col2 += S.bgr[3 * eq[j] + 2];
+    S.mask[q] = 1;
+    col0 += S.bgr[3 * q]; col1 += S.bgr[3 * q + 1]; col2 += S.bgr[3 * q + 2];
     n++;
   }
   col0 /= (n + 1); col1 /= (n + 1); col2 /= (n + 1);
@@ -637,7 +690,8 @@ extern "C" int dpe_fuse(dpe_ctx *ctx, const dpe_fusion_in *in, dpe_fusion_out *o
     for (int j = 0; j < v.num_src; ++j) f.src[j] = v.src_views[j];
     unsigned stamp = 0xFFFFFFFFu;
     if (v.num_src > 0) {
-      DPE_TIMED(ctx, KID_FUSE_ENTRIES, s, k_entries<<<blocks, 256, 0, s>>>(f));
+      DPE_TIMED(ctx, KID_FUSE_ENTRIES, s, if (f.mode == DPE_FUSE_FP64) k_entries<true><<<blocks, 256, 0, s>>>(f);
+                else k_entries<false><<<blocks, 256, 0, s>>>(f));
       DPE_LAUNCHED("k_entries", s);
       // Jacobi rounds until one changes nothing.  Each round makes at least the first undecided
       // pixel of the dependency order final, so npix + 1 rounds always suffice.
