@@ -211,6 +211,10 @@ dim3 coop_grid(int W, int H) { return dim3((W + kCoopPix - 1) / kCoopPix, (H + 1
 // the cooperative sweeps (DepthToWeak, LocalRefine): 16 pixels of one row per block
 dim3 sweep_grid(int W, int H) { return dim3((W + kCoopPix - 1) / kCoopPix, H); }
 
+// k_pad_images: a thread per padded texel, an image per z
+const dim3 kPadBlock(32, 8);
+dim3 pad_grid(int W, int H, int N) { return dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8, N); }
+
 // Blocks of 128 threads for a strided work list of up to `items` entries: enough to fill every
 // multiprocessor, no more than the list needs.
 unsigned list_grid(const dpe_ctx *ctx, long long items) {
@@ -527,16 +531,14 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
       }
     }
   }
+  for (int i = 0; i < N; ++i) a.img[i] = img_pad + PL * i;
+  PadSet pads = pad_set(a);
   for (int i = 0; i < N; ++i) {
-    const float *src = p->images[i];
-    if (host) {
-      DPE_TRY(cudaMemcpyAsync(stage + L * i, p->images[i], L * 4, h2d, s));
-      src = stage + L * i;
-    }
-    a.img[i] = img_pad + PL * i;
-    k_pad_image<<<dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8), dim3(32, 8), 0, s>>>(src, img_pad + PL * i, W, H);
-    PM_LAUNCHED("k_pad_image", s);
+    pads.src[i] = host ? stage + L * i : p->images[i];
+    if (host) DPE_TRY(cudaMemcpyAsync(stage + L * i, p->images[i], L * 4, h2d, s));
   }
+  k_pad_images<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads);
+  PM_LAUNCHED("k_pad_images", s);
   // FP32 staging: when every source texel is exact in a 16-bit format (BF16: 8-bit images, the finest
   // pyramid level; FP16: the halved levels), the cost kernels sample 16-bit quads instead: the same
   // values, one 8-byte load per tap instead of four.
@@ -559,17 +561,14 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
   a.stage = staging;
   uint2 *img_quads = staging != DPE_STAGE_FP32 ? get((uint2 *)0, "img_quads", PL * N) : nullptr;
   if (staging != DPE_STAGE_FP32 && !img_quads) return DPE_ERR_OUT_OF_MEMORY;
-  for (int i = 1; i < N; ++i) {
-    if (staging != DPE_STAGE_FP32) {
-      uint2 *quads = img_quads + PL * i;
-      const unsigned blocks = (unsigned)((PL + 255) / 256);
-      a.quad[i] = quads;
-      if (staging == DPE_STAGE_BF16)
-        k_stage_quads<true><<<blocks, 256, 0, s>>>(img_pad + PL * i, quads, (long long)PL, W + 2);
-      else
-        k_stage_quads<false><<<blocks, 256, 0, s>>>(img_pad + PL * i, quads, (long long)PL, W + 2);
-      PM_LAUNCHED("k_stage_quads", s);
-    }
+  if (staging != DPE_STAGE_FP32) {
+    for (int i = 1; i < N; ++i) a.quad[i] = img_quads + PL * i;
+    const dim3 grid((unsigned)((PL + 255) / 256), N - 1);
+    if (staging == DPE_STAGE_BF16)
+      k_stage_quads<true><<<grid, 256, 0, s>>>(img_pad + PL, img_quads + PL, (long long)PL, W + 2);
+    else
+      k_stage_quads<false><<<grid, 256, 0, s>>>(img_pad + PL, img_quads + PL, (long long)PL, W + 2);
+    PM_LAUNCHED("k_stage_quads", s);
   }
   return DPE_OK;
 }
@@ -612,8 +611,6 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
       void *tmp = A.get<uint8_t>("scan_tmp", tmp_bytes + 16);
       if (!tmp) return DPE_ERR_OUT_OF_MEMORY;
       DPE_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, ps[b].weak_flag, a.nmap, L, s));
-    } else {
-      DPE_TRY(cudaMemsetAsync(a.nmap, 0, (size_t)L * 4, s));
     }
   }
   // Launch settings the tuner picks (results do not depend on them): the block shape of the random
@@ -643,9 +640,13 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
     launch(kCarveCands[t.cand]);
     t.finish();
   };
-  DPE_TIMED(ctx, KID_GEN_EDGE_INFORM, s,
-            shaped(KID_GEN_EDGE_INFORM, [&](dim3 gr, dim3 bl) { k_gen_edge_inform<<<gr, bl, 0, s>>>(g.full); }));
-  PM_LAUNCHED("k_gen_edge_inform", s);
+  // edge distances with edges, label boundaries of WEAK pixels with APD: else nothing to do
+  bool inform = P.use_edge != 0;
+  for (int b = 0; b < n; ++b) inform = inform || (P.use_APD && ps[b].a.P.use_label);
+  if (inform) {
+    DPE_TIMED(ctx, KID_GEN_EDGE_INFORM, s, k_gen_edge_inform<<<g.fg, g.fb, 0, s>>>(g.full));
+    PM_LAUNCHED("k_gen_edge_inform", s);
+  }
   if (P.use_APD) {
     // only WEAK pixels have neighbours; without APD there is none
     DPE_TIMED(ctx, KID_FIND_NEAREST, s, k_find_nearest_strong<<<g.fg, g.fb, 0, s>>>(g.full));
@@ -894,6 +895,19 @@ extern "C" int dpe_pm_run_batch(dpe_ctx *ctx, const dpe_problem *problems, int c
 
 // ------------------------------------------------------------------ dpe_ncc_eval
 namespace {
+// Pads the images of a call on the caller's stream and writes its argument block to device memory.  The
+// block travels as a kernel parameter (captured by value at launch), so no host buffer has to outlive
+// the call and no copy waits for one.
+__global__ void k_pad_store_args(const __grid_constant__ PadSet pads, const __grid_constant__ PMArgs a, PMArgs *dst) {
+  static_assert(sizeof(PMArgs) % 4 == 0, "argument block is copied as 32-bit words");
+  pad_image_z(pads);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+    const uint32_t *s = reinterpret_cast<const uint32_t *>(&a);
+    uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+    for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < (int)(sizeof(PMArgs) / 4); i += blockDim.x * blockDim.y)
+      d[i] = s[i];
+  }
+}
 // kDeviceCheck: queries in device memory, which the host cannot validate, are checked here; a
 // query outside the problem gets NaN.
 template <bool kDeviceCheck>
@@ -953,12 +967,14 @@ int upload_queries(dpe_ctx *ctx, const dpe_ncc_query *q, QueryUpload *u) {
   u->plane = A.get<float4>("q_plane", n);
   u->d_args = A.get<PMArgs>("pm_args", 1);
   if (!A.ok()) return DPE_ERR_OUT_OF_MEMORY;
+  for (int i = 0; i < N; ++i) a.img[i] = img_pad + PL * i;
+  PadSet pads = pad_set(a);
   for (int i = 0; i < N; ++i) {
     DPE_TRY(cudaMemcpyAsync(stage + L * i, q->images[i], L * 4, cudaMemcpyHostToDevice, s));
-    a.img[i] = img_pad + PL * i;
-    k_pad_image<<<dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8), dim3(32, 8), 0, s>>>(stage + L * i, img_pad + PL * i, W, H);
-    PM_LAUNCHED("k_pad_image", s);
+    pads.src[i] = stage + L * i;
   }
+  k_pad_images<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads);
+  PM_LAUNCHED("k_pad_images", s);
   DPE_TRY(cudaMemcpyAsync(u->px, q->px, n * 4, cudaMemcpyHostToDevice, s));
   DPE_TRY(cudaMemcpyAsync(u->py, q->py, n * 4, cudaMemcpyHostToDevice, s));
   DPE_TRY(cudaMemcpyAsync(u->src, q->src, n * 4, cudaMemcpyHostToDevice, s));
@@ -1082,12 +1098,11 @@ extern "C" int dpe_ncc_grad_device(dpe_ctx *ctx, const dpe_ncc_query *q, const f
   float *img_pad = A.get<float>("gd_img_pad", PL * N);
   PMArgs *d_args = A.get<PMArgs>("gd_args", 1);
   if (!A.ok()) return DPE_ERR_OUT_OF_MEMORY;
-  for (int i = 0; i < N; ++i) {
-    a.img[i] = img_pad + PL * i;
-    k_pad_image<<<dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8), dim3(32, 8), 0, s>>>(q->images[i], img_pad + PL * i, W, H);
-    PM_LAUNCHED("k_pad_image", s);
-  }
-  DPE_TRY(cudaMemcpyAsync(d_args, &a, sizeof(PMArgs), cudaMemcpyHostToDevice, s));
+  for (int i = 0; i < N; ++i) a.img[i] = img_pad + PL * i;
+  PadSet pads = pad_set(a);
+  for (int i = 0; i < N; ++i) pads.src[i] = q->images[i];
+  k_pad_store_args<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads, a, d_args);
+  PM_LAUNCHED("k_pad_store_args", s);
   if (grad_images_out) DPE_TRY(cudaMemsetAsync(grad_images_out, 0, L * (N - 1) * 4, s));
   const int64_t n = q->count;
   k_ncc_grad<true><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d_args, n, q->px, q->py, q->src,
@@ -1096,7 +1111,6 @@ extern "C" int dpe_ncc_grad_device(dpe_ctx *ctx, const dpe_ncc_query *q, const f
                                                                reinterpret_cast<float4 *>(grad_depth_normal_out),
                                                                grad_images_out);
   PM_LAUNCHED("k_ncc_grad", s);
-  // the argument block is read by the kernels above: keep the host copy alive until they ran
   DPE_TRY(cudaStreamSynchronize(s));
   return DPE_OK;
 }
@@ -1155,14 +1169,6 @@ unsigned char *g_static_addr[kMaxDevices] = {};
 
 size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Writes the call's argument block into the static scratch.  The block travels as a kernel
-// parameter (captured by value at launch), so no host buffer has to outlive the call.
-__global__ void k_store_args(const __grid_constant__ PMArgs a, PMArgs *dst) {
-  static_assert(sizeof(PMArgs) % 4 == 0, "argument block is copied as 32-bit words");
-  const uint32_t *s = reinterpret_cast<const uint32_t *>(&a);
-  uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-  for (int i = threadIdx.x; i < (int)(sizeof(PMArgs) / 4); i += blockDim.x) d[i] = s[i];
-}
 }  // namespace
 
 extern "C" int dpe_ncc_eval_noalloc(const dpe_ncc_query *q, float *costs_out, void *stream) {
@@ -1210,13 +1216,10 @@ extern "C" int dpe_ncc_eval_noalloc(const dpe_ncc_query *q, float *costs_out, vo
   unsigned char *img_base = base + round256(sizeof(PMArgs));
   for (int i = 0; i < N; ++i) a.img[i] = reinterpret_cast<const float *>(img_base + (size_t)i * img_bytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  k_store_args<<<1, 256, 0, s>>>(a, reinterpret_cast<PMArgs *>(base));
-  DPE_LAUNCHED("k_store_args", s);
-  for (int i = 0; i < N; ++i) {
-    k_pad_image<<<dim3((W + 2 + 31) / 32, (H + 2 + 7) / 8), dim3(32, 8), 0, s>>>(
-        q->images[i], reinterpret_cast<float *>(img_base + (size_t)i * img_bytes), W, H);
-    DPE_LAUNCHED("k_pad_image", s);
-  }
+  PadSet pads = pad_set(a);
+  for (int i = 0; i < N; ++i) pads.src[i] = q->images[i];
+  k_pad_store_args<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads, a, reinterpret_cast<PMArgs *>(base));
+  DPE_LAUNCHED("k_pad_store_args", s);
   const int64_t n = q->count;
   k_ncc_queries<true><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(reinterpret_cast<const PMArgs *>(base), n, q->px,
                                                                     q->py, q->src,
