@@ -60,6 +60,8 @@ struct PMArgs {
   const uint2 *quad[kMaxImages];
   int stage;  // DPE_STAGE_*: storage the cost kernels sample the source images from
   int gn;     // 1: Gauss-Newton plane hypothesis in the strong update (dpe_options::gn_refine)
+  int far;    // 1: byte offsets into a staged image need more than 32 bits (fetch_bytes)
+  int six;    // 1: the strong window is the 6 x 6 one (radius 5, step 2) and the image not far
   const float *dep[kMaxImages];  // W*H depth maps (geom consistency)
   // state
   float4 *plane;
@@ -140,7 +142,7 @@ inline void homography_base(const dpe_camera &rc, const dpe_camera &sc, double A
   b[1] = (double)sc.K[4] * tr[1] + (double)sc.K[5] * tr[2];
   b[2] = (double)sc.K[8] * tr[2];
 }
-// Fills the homography bases of every source of a call (cameras already in a.cam).
+// Fills the homography bases of every source of a call (size, parameters and cameras already in a).
 inline void set_homography_bases(PMArgs &a) {
   for (int s = 1; s < a.N; ++s) {
     homography_base(a.cam[0], a.cam[s], a.dA[s], a.db[s], a.dm);
@@ -150,6 +152,8 @@ inline void set_homography_bases(PMArgs &a) {
     for (int k = 0; k < 3; ++k) a.hb[s][k] = (float)a.db[s][k];
   }
   for (int k = 0; k < 4; ++k) a.hm[k] = (float)a.dm[k];
+  a.far = (unsigned long long)(a.W + 2) * (a.H + 2) * 8 > 0xFFFFFFFFull ? 1 : 0;
+  a.six = a.P.strong_radius == 5 && a.P.strong_increment == 2 && !a.far ? 1 : 0;
 }
 
 // ------------------------------------------------------------------ checked builds
@@ -317,6 +321,7 @@ __device__ __forceinline__ float bilinear(const float *__restrict__ img, int pad
 // padded offset o, (P[o], P[o+1], P[o+pw], P[o+pw+1]), in FP32; the interpolation is shared, so
 // samplers differ only in storage.  FP32 samples equal bilinear() above exactly.
 struct SrcF32 {
+  static constexpr unsigned kBytes = 4;
   const float *p;
   int pw;
   long long n;
@@ -334,11 +339,12 @@ __device__ __forceinline__ uint2 quad_ld(const uint2 *p, long long off, long lon
 }
 // FP16 quads: the footprint's upper row in x, its lower row in y, left texels in the low halves.
 struct SrcF16 {
+  static constexpr unsigned kBytes = 8;
   const uint2 *p;
   int pw;
   long long n;
-  __device__ __forceinline__ float4 fetch(int o) const {
-    const uint2 t = quad_ld(p, (unsigned)o, n, 108);
+  __device__ __forceinline__ float4 fetch(int o) const { return widen(quad_ld(p, (unsigned)o, n, 108)); }
+  static __device__ __forceinline__ float4 widen(uint2 t) {
     return make_float4(__half2float(__ushort_as_half((unsigned short)(t.x & 0xFFFFu))),
                        __half2float(__ushort_as_half((unsigned short)(t.x >> 16))),
                        __half2float(__ushort_as_half((unsigned short)(t.y & 0xFFFFu))),
@@ -347,11 +353,12 @@ struct SrcF16 {
 };
 // BF16 quads: a bfloat16 is the top half of an FP32 word, so widening is a shift.
 struct SrcBF16 {
+  static constexpr unsigned kBytes = 8;
   const uint2 *p;
   int pw;
   long long n;
-  __device__ __forceinline__ float4 fetch(int o) const {
-    const uint2 t = quad_ld(p, (unsigned)o, n, 110);
+  __device__ __forceinline__ float4 fetch(int o) const { return widen(quad_ld(p, (unsigned)o, n, 110)); }
+  static __device__ __forceinline__ float4 widen(uint2 t) {
     return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16),
                        __uint_as_float(t.y & 0xFFFF0000u));
   }
@@ -360,9 +367,39 @@ struct SrcBF16 {
 struct Foot2 {
   float2 v00, v10, v01, v11;
 };
-template <class Src> __device__ __forceinline__ Foot2 fetch2(const Src &src, int o0, int o1) {
-  const float4 a = src.fetch(o0), b = src.fetch(o1);
+// ... at 32-bit byte offsets from the image (padded offset x kBytes): the address is the base plus the
+// offset, which the integer pipe adds; a scaled 64-bit index would multiply on the FMA pipe, the tap
+// loops' bound (DepthToWeak 49.2 -> 47.3 ms on a 1600x1200 view).  Images whose offsets do not fit
+// (PMArgs::far) take the one-tap loops.
+template <class T> __device__ __forceinline__ T ld_bytes(const T *p, unsigned off, long long n, int tag) {
+#ifdef DPE_CHECKED
+  return *dpe_chk(p, (long long)(off / sizeof(T)), n, tag);
+#else
+  return __ldg(reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + off));
+#endif
+}
+__device__ __forceinline__ float4 fetch_bytes(const SrcF32 &s, unsigned off) {
+  const unsigned down = off + 4u * (unsigned)s.pw;
+  return make_float4(ld_bytes(s.p, off, s.n, 102), ld_bytes(s.p, off + 4u, s.n, 103), ld_bytes(s.p, down, s.n, 104),
+                     ld_bytes(s.p, down + 4u, s.n, 105));
+}
+__device__ __forceinline__ float4 fetch_bytes(const SrcF16 &s, unsigned off) {
+  return SrcF16::widen(ld_bytes(s.p, off, s.n, 108));
+}
+__device__ __forceinline__ float4 fetch_bytes(const SrcBF16 &s, unsigned off) {
+  return SrcBF16::widen(ld_bytes(s.p, off, s.n, 110));
+}
+template <class Src> __device__ __forceinline__ Foot2 fetch2(const Src &src, unsigned o0, unsigned o1) {
+  const float4 a = fetch_bytes(src, o0), b = fetch_bytes(src, o1);
   return Foot2{make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), make_float2(a.w, b.w)};
+}
+// The byte offsets of two taps from their biased floors (floor_split: 0x4B400000 + the texel), modulo 2^32;
+// base: the byte offset of texel (0, 0) minus both biases.
+template <class Src>
+__device__ __forceinline__ Foot2 fetch2_biased(const Src &src, float2 fu, float2 fv, unsigned base) {
+  const unsigned pitch = (unsigned)src.pw * Src::kBytes;
+  return fetch2(src, __float_as_uint(fv.x) * pitch + (__float_as_uint(fu.x) * Src::kBytes + base),
+                __float_as_uint(fv.y) * pitch + (__float_as_uint(fu.y) * Src::kBytes + base));
 }
 // kClamp = false: the caller knows -1 <= x <= W-1 and -1 <= y <= H-1, where the clamp is the
 // identity.
@@ -751,10 +788,8 @@ __device__ __forceinline__ void strong_tap2(const WinProj &wp, const WinClamp &w
   const float2 fu = __fadd2_rd(u, bias), fv = __fadd2_rd(v, bias);  // 1.5 * 2^23 + floor (floor_split)
   const float2 au = sub2(u, sub2(fu, bias)), av = sub2(v, sub2(fv, bias));
   const float2 ou = sub2(dup2(1.0f), au), ov = sub2(dup2(1.0f), av);
-  // the texel index straight from the biased floors: base holds the window's origin minus the biases
-  const unsigned pw = (unsigned)src.pw;
-  const Foot2 t = fetch2(src, (int)(__float_as_uint(fv.x) * pw + __float_as_uint(fu.x) + base),
-                         (int)(__float_as_uint(fv.y) * pw + __float_as_uint(fu.y) + base));
+  // the texels straight from the biased floors: base holds the window's origin minus the biases
+  const Foot2 t = fetch2_biased(src, fu, fv, base);
   const float2 top = addp2(mul2(ou, t.v00), mul2(au, t.v10)), bot = addp2(mul2(ou, t.v01), mul2(au, t.v11));
   const float2 sv = sub2(addp2(mul2(ov, top), mul2(av, bot)), dup2(rw.center));
   const float4 w = rw.tap2(p);
@@ -803,7 +838,8 @@ __device__ __forceinline__ void strong_window6(const PMArgs &a, const WinProj &w
     gz[p] = mul2(dup2(wp.h7), dy);
   }
   // (V0 + iy + 1) * pw + (U0 + ix + 1) with iy, ix = biased floor - 0x4B400000, modulo 2^32
-  const unsigned base = ((unsigned)wp.V0 + 1u - 0x4B400000u) * (unsigned)src.pw + ((unsigned)wp.U0 + 1u - 0x4B400000u);
+  const unsigned base = (((unsigned)wp.V0 + 1u - 0x4B400000u) * (unsigned)src.pw +
+                         ((unsigned)wp.U0 + 1u - 0x4B400000u)) * Src::kBytes;
   float dx = -5.0f;
 #pragma unroll 1
   for (int ii = 0; ii < 18; ii += 3, dx += 2.0f) {
@@ -818,7 +854,7 @@ template <class Src, bool kPairs, class RW>
 __device__ __forceinline__ float ncc_strong_src(const PMArgs &a, const WinProj &wp, const Src &src, const RW &rw) {
   float s_s = 0.f, s_ss = 0.f, s_rs = 0.f;
 #ifdef __CUDA_ARCH__
-  if (kPairs && a.P.strong_radius == 5 && a.P.strong_increment == 2) {
+  if (kPairs && a.six) {
     // one path per warp: the clamped taps are right for every window, and running both would cost more
     if (__all_sync(__activemask(), window_inside(a, wp, 5.0f))) strong_window6<false>(a, wp, src, rw, s_s, s_ss, s_rs);
     else strong_window6<true>(a, wp, src, rw, s_s, s_ss, s_rs);
@@ -1032,9 +1068,7 @@ __device__ __forceinline__ float2 weak_sample2(const PMArgs &a, const float H[9]
   const float2 fu = __fadd2_rd(u, bias), fv = __fadd2_rd(v, bias);
   const float2 au = sub2(u, sub2(fu, bias)), av = sub2(v, sub2(fv, bias));
   const float2 ou = sub2(dup2(1.0f), au), ov = sub2(dup2(1.0f), av);
-  const unsigned pw = (unsigned)src.pw, base = (1u - 0x4B400000u) * (pw + 1u);
-  const Foot2 t = fetch2(src, (int)(__float_as_uint(fv.x) * pw + __float_as_uint(fu.x) + base),
-                         (int)(__float_as_uint(fv.y) * pw + __float_as_uint(fu.y) + base));
+  const Foot2 t = fetch2_biased(src, fu, fv, (1u - 0x4B400000u) * ((unsigned)src.pw + 1u) * Src::kBytes);
   const float2 top = addp2(mul2(ou, t.v00), mul2(au, t.v10)), bot = addp2(mul2(ou, t.v01), mul2(au, t.v11));
   return sub2(addp2(mul2(ov, top), mul2(av, bot)), dup2(ref_center));
 }
@@ -1055,7 +1089,7 @@ __device__ __forceinline__ float window_ncc_tab(const PMArgs &a, const float H[9
   float x = (float)(cx - radius);
 #ifdef __CUDA_ARCH__
   const int side = 2 * radius / inc + 1;
-  if (k > 0 && weak_is3(a)) {
+  if (k > 0 && weak_is3(a) && !a.far) {
     const float4 *pairs = weak_pairs(a, tab, k);
     float2 cX[3], rX[3], rY[3], rZ[3];  // column terms (H0 x, H3 x) and H6 x; row terms H1 y, H4 y, H7 y
     float cZ[3];
@@ -1084,7 +1118,7 @@ __device__ __forceinline__ float window_ncc_tab(const PMArgs &a, const float H[9
     weak_tap(a, H, src, x + finc + finc, ry[2], ref_center, *weak_last(tab, k), r[2]);
 #pragma unroll
     for (int i = 0; i < 3; ++i) { s_s += r[i].s; s_ss += r[i].ss; s_rs += r[i].rs; }
-  } else if (k == 0 && side == 6) {
+  } else if (k == 0 && side == 6 && !a.far) {
     const float4 *pairs = weak_pairs(a, tab, 0);
     float2 rX[3], rY[3], rZ[3];
 #pragma unroll
