@@ -484,7 +484,8 @@ __device__ __forceinline__ void normalize2(float2 *v) {
 }
 
 // Marsaglia sphere point facing the camera (DPE.cu:365-391); rejection capped at 64 tries.
-__device__ __forceinline__ float4 random_normal(const dpe_camera &c, int x, int y, Rng &rng, float depth) {
+template <class R>
+__device__ __forceinline__ float4 random_normal(const dpe_camera &c, int x, int y, R &rng, float depth) {
   float q1 = 1.0f, q2 = 1.0f, s = 2.0f;
   for (int tries = 0; s >= 1.0f && tries < 64; ++tries) {
     q1 = 2.0f * rng.uniform() - 1.0f;
@@ -500,7 +501,8 @@ __device__ __forceinline__ float4 random_normal(const dpe_camera &c, int x, int 
 }
 
 // Euler-angle perturbation (DPE.cu:393-428)
-__device__ __forceinline__ float4 perturbed_normal(const dpe_camera &c, int x, int y, float4 n, Rng &rng, float pert) {
+template <class R>
+__device__ __forceinline__ float4 perturbed_normal(const dpe_camera &c, int x, int y, float4 n, R &rng, float pert) {
   const float4 v = view_direction(c, x, y, 1.0f);
   const float a1 = (rng.uniform() - 0.5f) * pert;
   const float a2 = (rng.uniform() - 0.5f) * pert;

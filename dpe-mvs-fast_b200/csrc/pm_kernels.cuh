@@ -1064,7 +1064,8 @@ struct CoopPixel {
     };                    // view selection
     float4 hyp[5];        // from the refinement planes on
   };
-  float u[16];            // the uniform draws; then the refinement planes' weighted costs
+  float u[16];            // the uniform draws of the view sampling; then the refinement planes' costs
+  float ahead[16];        // the uniform draws after them (the refinement's)
   float fc[8];            // the candidates' weighted costs
   float4 pl_cur, pl_now, n_rand, n_pert;
   float center, inv_wsum, mean_r, var_r;
@@ -1072,7 +1073,7 @@ struct CoopPixel {
   int pos[kCurRow];
   uint32_t views_new, temp_sel, rng_ctr;
   int cnt;                 // entries of this pixel in its warp's list
-  uint8_t uniq[kCurRow];   // candidate h has a cost row of its own
+  alignas(4) uint8_t uniq[kCurRow];   // candidate h has a cost row of its own
   uint8_t dup[kRows];      // the row that holds candidate h's costs (itself, or an equal plane's)
   uint8_t row[8];          // the row of the candidate kept for direction d
   uint8_t flag[8];         // direction d has a candidate
@@ -1082,7 +1083,7 @@ struct CoopPixel {
   uint8_t act[32];         // the sampled sources (source index - 1), ascending
   uint8_t alive[8];        // refinement plane h can still be taken
   uint8_t first, second;   // positions in act of the two heaviest sources
-  uint8_t na;
+  uint8_t na, live;
 };
 // Shared bytes of one block: the pixels' states, the warps' lists, then per pixel kRows cost rows of
 // n = N - 1 floats.
@@ -1090,6 +1091,21 @@ __host__ __device__ inline size_t coop_smem_bytes(int n) {
   return sizeof(CoopPixel) * kCoopPix + sizeof(uint16_t) * kListCap * (kCoopThreads / 32) +
          sizeof(float) * (size_t)kCoopPix * kRows * n;
 }
+
+// A pixel's stream whose next 16 numbers are at hand; a long rejection in random_normal goes on from the
+// generator.
+struct AheadRng {
+  Rng next;
+  const float *u;
+  int used;
+  __device__ __forceinline__ float uniform() {
+    if (used < 16) {
+      next.ctr++;
+      return u[used++];
+    }
+    return next.uniform();
+  }
+};
 
 struct CoopCtx {
   const PMArgs *a;
@@ -1195,55 +1211,31 @@ __device__ __forceinline__ void strong_taps(const CoopCtx &c) {
 
 // Candidate search of the non-edge propagation (8 slots: 0 up_near, 1 up_far, 2 down_near,
 // 3 down_far, 4 left_near, 5 left_far, 6 right_near, 7 right_far), slot d only.
-__device__ __forceinline__ int strong_search_plain(const PMArgs &a, int px, int py, int center, int d) {
+__device__ __forceinline__ int strong_search_plain(const PMArgs &a, int px, int py, int d) {
   const int W = a.W, H = a.H;
   [[maybe_unused]] const long long L = (long long)W * H;
   const int f = d >> 1;
-  if (d & 1) {  // far: every second pixel from distance 3 on
-    const int starts[4] = {center - 3 * W, center + 3 * W, center - 3, center + 3};
-    const int strides[4] = {-W, W, -1, 1};
-    const bool oks[4] = {py > 2, py < H - 3, px > 2, px < W - 3};
-    if (!oks[f]) return -1;
-    float m = G(a.cost, starts[f], L, 206);
-    int mp = starts[f];
-    for (int i = 1; i < 11; ++i) {
-      bool ok;
-      switch (f) {
-        case 0: ok = py > 2 + 2 * i; break;
-        case 1: ok = py < H - 3 - 2 * i; break;
-        case 2: ok = px > 2 + 2 * i; break;
-        default: ok = px < W - 3 - 2 * i; break;
-      }
-      if (ok) {
-        const int t = starts[f] + 2 * i * strides[f];
-        const float ct = G(a.cost, t, L, 207);
-        if (ct < m) { m = ct; mp = t; }
-      }
-    }
-    return mp;
+  const int dx = f == 2 ? -1 : f == 3 ? 1 : 0, dy = f == 0 ? -1 : f == 1 ? 1 : 0;
+  // far: every second pixel from distance 3 on; near: the pixel one step away, then the pairs k to either
+  // side at distance 1 + k, k = 1..3 (before the other side first).  A pixel outside the image ends the
+  // far ones and skips the near one.
+  const bool far = d & 1;
+  float m = 0.0f;
+  int mp = -1;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+  for (int i = 0; i < (far ? 11 : 7); ++i) {
+    const int k = (i + 1) >> 1;
+    const int along = far ? 3 + 2 * i : 1 + k, side = far ? 0 : i & 1 ? -k : k;
+    const int x = px + dx * along + (dy != 0 ? side : 0), y = py + dy * along + (dx != 0 ? side : 0);
+    const bool in = x >= 0 && x < W && y >= 0 && y < H;
+    if (i == 0 && !in) return -1;
+    if (!in) continue;
+    const int t = y * W + x;
+    const float ct = G(a.cost, t, L, 207);
+    if (i == 0 || ct < m) { m = ct; mp = t; }
   }
-  // near: base pixel one step away, then diagonal pairs at distance 1..3
-  const int nbase[4] = {center - W, center + W, center - 1, center + 1};
-  const bool nok[4] = {py > 0, py < H - 1, px > 0, px < W - 1};
-  if (!nok[f]) return -1;
-  float m = G(a.cost, nbase[f], L, 208);
-  int mp = nbase[f];
-  for (int i = 0; i < 3; ++i)
-    for (int side = 0; side < 2; ++side) {
-      bool ok;
-      int t;
-      const int k = 1 + i;
-      switch (f) {
-        case 0: t = nbase[0] - k * W + (side ? k : -k); ok = py > 1 + i && (side ? px < W - 1 - i : px > i); break;
-        case 1: t = nbase[1] + k * W + (side ? k : -k); ok = py < H - 2 - i && (side ? px < W - 1 - i : px > i); break;
-        case 2: t = nbase[2] - k + (side ? k * W : -k * W); ok = px > 1 + i && (side ? py < H - 1 - i : py > i); break;
-        default: t = nbase[3] + k + (side ? k * W : -k * W); ok = px < W - 2 - i && (side ? py < H - 1 - i : py > i); break;
-      }
-      if (ok) {
-        const float ct = G(a.cost, t, L, 209);
-        if (ct < m) { m = ct; mp = t; }
-      }
-    }
   return mp;
 }
 
@@ -1316,7 +1308,7 @@ __device__ __forceinline__ void strong_search(const CoopCtx &c, int iter) {
     pos = strong_search_edge(a, c.px, c.py, c.center, d, iter);
     if (G(a.edge, c.center, L, 203) == 0) pos2 = strong_search_edge2(a, c.px, c.py, d, iter);
   } else {
-    pos = strong_search_plain(a, c.px, c.py, c.center, d);
+    pos = strong_search_plain(a, c.px, c.py, d);
   }
   P.pos[d] = pos;
   P.pos[8 + d] = pos2;
@@ -1350,10 +1342,8 @@ __device__ __forceinline__ bool same_rec(const HypProj &x, const HypProj &y) {
 // plane too.
 __device__ __forceinline__ void strong_distinct(const CoopCtx &c) {
   CoopPixel &P = *c.P;
-  if (!c.live) {
-    if (c.lane == 0) P.cnt = 0;
-    return;
-  }
+  if (c.lane == 0) P.live = c.live ? 1 : 0;
+  if (!c.live) return;
   const int last = c.a->P.use_edge ? kCurRow : 8;
   for (int h = c.lane; h < last; h += 8) {
     int to = h;
@@ -1370,25 +1360,29 @@ __device__ __forceinline__ void strong_distinct(const CoopCtx &c) {
     P.dup[kCurRow] = (uint8_t)to;
   }
 }
-__device__ __forceinline__ void strong_count(const CoopCtx &c) {
-  if (!c.live || c.lane != 0) return;
-  CoopPixel &P = *c.P;
-  const int last = c.a->P.use_edge ? kCurRow : 8;
+// Sum of the bytes 0 .. h - 1 of a pixel's uniq flags.
+__device__ __forceinline__ int uniq_before(const CoopPixel &P, int h) {
   int m = 0;
-  for (int h = 0; h < last; ++h) m += P.uniq[h];
-  P.cnt = m;
+  for (int w = 0; w < kCurRow / 4 && 4 * w < h; ++w) {
+    uint32_t v = reinterpret_cast<const uint32_t *>(P.uniq)[w];
+    if (h < 4 * w + 4) v &= (1u << (8 * (h - 4 * w))) - 1u;
+    m += (int)((v * 0x01010101u) >> 24);
+  }
+  return m;
 }
 __device__ __forceinline__ void strong_list(const CoopCtx &c) {
+  const int last = c.a->P.use_edge ? kCurRow : 8;
+  int off = 0, mine = 0;
+  for (int k = 0; k < kWarpPix; ++k) {
+    const int m = c.W0[k].live ? uniq_before(c.W0[k], last) : 0;
+    if (k < (c.slot & (kWarpPix - 1))) off += m;
+    if (k == (c.slot & (kWarpPix - 1))) mine = m;
+  }
+  if (c.lane == 0) c.P->cnt = mine;
   if (!c.live) return;
   const CoopPixel &P = *c.P;
-  const int last = c.a->P.use_edge ? kCurRow : 8;
-  const int off = coop_offset(c);
-  for (int h = c.lane; h < last; h += 8) {
-    if (!P.uniq[h]) continue;
-    int rank = 0;
-    for (int e = 0; e < h; ++e) rank += P.uniq[e];
-    c.list[off + rank] = coop_entry(c, h, 0);
-  }
+  for (int h = c.lane; h < last; h += 8)
+    if (P.uniq[h]) c.list[off + uniq_before(P, h)] = coop_entry(c, h, 0);
 }
 
 // The candidate kept for direction d and its cost row (lane d): the edge form takes the second search
@@ -1427,8 +1421,8 @@ __device__ __forceinline__ void strong_choose(const CoopCtx &c, int iter) {
 }
 
 // The view-selection probability of each source (sample_views' first loop, with the priors of
-// DPE.cu:1551-1563), lane j taking sources j, j + 8, ...; and the 15 uniform draws of the sampling
-// (counter-based, so draw s is the pixel's counter + s), split over the lanes.
+// DPE.cu:1551-1563), lane j taking sources j, j + 8, ...; and the 15 uniform draws of the sampling and the
+// 16 after them (counter-based, so draw s is the pixel's counter + s), split over the lanes.
 __device__ __forceinline__ void strong_probs(const CoopCtx &c, int iter) {
   if (!c.live) return;
   const PMArgs &a = *c.a;
@@ -1436,9 +1430,12 @@ __device__ __forceinline__ void strong_probs(const CoopCtx &c, int iter) {
   const long long L = (long long)W * a.H;
   CoopPixel &P = *c.P;
   const uint32_t ctr0 = G(a.rng_ctr, center, L, 106);
-  for (int s = c.lane; s < 15; s += kCoopLanes) {
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+  for (int s = c.lane; s < 15 + 16; s += kCoopLanes) {
     Rng r{a.key[0], a.key[1], (uint32_t)center, ctr0 + (uint32_t)s};
-    P.u[s] = r.uniform();
+    (s < 15 ? P.u[s] : P.ahead[s - 15]) = r.uniform();
   }
   const long total = (long)W * a.H;
   const long nbr[4] = {(long)center - W, (long)center + W, (long)center - 1, (long)center + 1};
@@ -1568,7 +1565,7 @@ __device__ __forceinline__ void strong_accept(const CoopCtx &c) {
       views_new = P.temp_sel;
     }
   }
-  Rng rng{a.key[0], a.key[1], (uint32_t)c.center, P.rng_ctr};
+  AheadRng rng{{a.key[0], a.key[1], (uint32_t)c.center, P.rng_ctr}, P.ahead, 0};
   const float dmin = a.P.depth_min, dmax = a.P.depth_max;
   P.depth_rand = rng.uniform() * (dmax - dmin) + dmin;
   P.n_rand = random_normal(rc, c.px, c.py, rng, depth_now);
@@ -1579,7 +1576,7 @@ __device__ __forceinline__ void strong_accept(const CoopCtx &c) {
   P.depth_now = depth_now;
   P.cost_now = cost_now;
   P.views_new = views_new;
-  P.rng_ctr = rng.ctr;
+  P.rng_ctr = rng.next.ctr;
 }
 // Refinement plane h (lane h): (random depth, normal now), (depth now, random normal), both random,
 // (depth now, perturbed normal), (perturbed depth, normal now).  Its first sources: the heaviest, and
@@ -1772,7 +1769,7 @@ __device__ __forceinline__ void strong_gn_decide(const CoopCtx &c) {
 // The phases between barriers, one thread's part of each (host builds of this source run them in
 // lock-step over a block).
 enum {
-  kPhTaps, kPhSearch, kPhDistinct, kPhCount, kPhList, kPhEval0, kPhChoose, kPhProbs, kPhCumulate, kPhSample, kPhWeigh,
+  kPhTaps, kPhSearch, kPhDistinct, kPhList, kPhEval0, kPhChoose, kPhProbs, kPhCumulate, kPhSample, kPhWeigh,
   kPhActive, kPhWeighted, kPhEval1, kPhAccept, kPhPlanes, kPhFirstCount, kPhFirstList, kPhEval2, kPhDrop, kPhRestCount,
   kPhRestList, kPhEval3, kPhRefineSum, kPhDecide, kStrongPhases
 };
@@ -1782,7 +1779,6 @@ __device__ __forceinline__ void strong_phase(const CoopCtx &c, int phase, int it
     case kPhTaps: strong_taps(c); break;
     case kPhSearch: strong_search(c, iter); break;
     case kPhDistinct: strong_distinct(c); break;
-    case kPhCount: strong_count(c); break;
     case kPhList: strong_list(c); break;
     case kPhChoose: strong_choose(c, iter); break;
     case kPhProbs: strong_probs(c, iter); break;
