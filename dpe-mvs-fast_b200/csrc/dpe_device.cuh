@@ -41,6 +41,13 @@ constexpr int kMaxWin = 6;  // taps per window side for radius 5 / step 2 (DPE.c
 #define DPE_LR_MIN_BLOCKS 5
 #endif
 
+// What a window's projection takes from one source: A and b (PMArgs), the camera's (width, height), and
+// where a kernel holds its sources in shared memory, the image as it samples it.
+struct SrcConst {
+  double A[9], b[3], size[2];
+  const void *texels;
+};
+
 // All per-call read-only data (cameras, relative poses, params, buffer pointers).  It lives in a
 // small device buffer written once per call; kernels receive its address.
 struct PMArgs {
@@ -48,9 +55,9 @@ struct PMArgs {
   dpe_params P;
   dpe_camera cam[kMaxImages];
   // Plane-independent parts of each source's homography H = A - b m^T / w (homography_base):
-  // composed in double (window centres are projected in double), and the same rounded to float.
-  double dA[kMaxImages][9], db[kMaxImages][3], dm[4];
-  double dsize[kMaxImages][2];  // each source camera's (width, height)
+  // composed in double (src, dm: window centres are projected in double), and the same rounded to float.
+  SrcConst src[kMaxImages];
+  double dm[4];
   float hA[kMaxImages][9], hb[kMaxImages][3], hm[4];
   uint32_t key[2];
   const float *img[kMaxImages];  // padded (W+2)*(H+2) float images
@@ -145,11 +152,13 @@ inline void homography_base(const dpe_camera &rc, const dpe_camera &sc, double A
 // Fills the homography bases of every source of a call (size, parameters and cameras already in a).
 inline void set_homography_bases(PMArgs &a) {
   for (int s = 1; s < a.N; ++s) {
-    homography_base(a.cam[0], a.cam[s], a.dA[s], a.db[s], a.dm);
-    a.dsize[s][0] = a.cam[s].width;
-    a.dsize[s][1] = a.cam[s].height;
-    for (int k = 0; k < 9; ++k) a.hA[s][k] = (float)a.dA[s][k];
-    for (int k = 0; k < 3; ++k) a.hb[s][k] = (float)a.db[s][k];
+    SrcConst &c = a.src[s];
+    homography_base(a.cam[0], a.cam[s], c.A, c.b, a.dm);
+    c.size[0] = a.cam[s].width;
+    c.size[1] = a.cam[s].height;
+    c.texels = nullptr;
+    for (int k = 0; k < 9; ++k) a.hA[s][k] = (float)c.A[k];
+    for (int k = 0; k < 3; ++k) a.hb[s][k] = (float)c.b[k];
   }
   for (int k = 0; k < 4; ++k) a.hm[k] = (float)a.dm[k];
   a.far = (unsigned long long)(a.W + 2) * (a.H + 2) * 8 > 0xFFFFFFFFull ? 1 : 0;
@@ -428,6 +437,9 @@ __device__ __forceinline__ SrcF16 src_f16(const PMArgs &a, int s) {
 __device__ __forceinline__ SrcBF16 src_bf16(const PMArgs &a, int s) {
   return SrcBF16{a.quad[s], a.pad_w, (long long)a.pad_w * (a.H + 2)};
 }
+template <class Src> __device__ __forceinline__ Src src_of(const PMArgs &a, const void *texels) {
+  return Src{static_cast<decltype(Src::p)>(texels), a.pad_w, (long long)a.pad_w * (a.H + 2)};
+}
 // The sampler of a staging (DPE_STAGE_*), chosen at compile time: each cost kernel is built once
 // per staging, so a kernel carries only its own tap loop.
 template <int kStage> struct SrcOf;
@@ -676,8 +688,8 @@ __device__ __forceinline__ PlaneProj plane_projection(const PMArgs &a, float4 pl
 struct PixelProj {
   double x, y, z;
 };
-__device__ __forceinline__ PixelProj pixel_projection(const PMArgs &a, int s, int px, int py) {
-  const double *A = a.dA[s];
+__device__ __forceinline__ PixelProj pixel_projection(const SrcConst &sc, int px, int py) {
+  const double *A = sc.A;
   const double x = (double)px, y = (double)py;
   return PixelProj{A[0] * x + A[1] * y + A[2], A[3] * x + A[4] * y + A[5], A[6] * x + A[7] * y + A[8]};
 }
@@ -696,16 +708,15 @@ __device__ __forceinline__ double floor_split(double x, int *ix) {
 }
 // Fills wp for a plane at a pixel and source s; false when the centre does not project inside the
 // source (the cost is then 2, DPE.cu:709-712).
-__device__ __forceinline__ bool window_projection(const PMArgs &a, int s, const PlaneProj &p, const PixelProj &c,
+__device__ __forceinline__ bool window_projection(const SrcConst &sc, const PlaneProj &p, const PixelProj &c,
                                                   WinProj &wp) {
-  const double *A = a.dA[s], *b = a.db[s];
+  const double *A = sc.A, *b = sc.b;
   const double X = c.x - b[0] * p.q;
   const double Y = c.y - b[1] * p.q;
   const double Z = c.z - b[2] * p.q;
   const double iz = 1.0 / Z;
   const double uc = X * iz, vc = Y * iz;
-  const double *size = a.dsize[s];
-  if (!(uc >= 0.0 && uc < size[0] && vc >= 0.0 && vc < size[1])) return false;
+  if (!(uc >= 0.0 && uc < sc.size[0] && vc >= 0.0 && vc < sc.size[1])) return false;
   const double U = floor_split(uc, &wp.U0), V = floor_split(vc, &wp.V0);
   wp.fuv = make_float2((float)(uc - U), (float)(vc - V));
   wp.zc = (float)Z;
@@ -718,7 +729,7 @@ __device__ __forceinline__ bool window_projection(const PMArgs &a, int s, const 
   return true;
 }
 __device__ __forceinline__ bool window_projection(const PMArgs &a, int s, float4 pl, int px, int py, WinProj &wp) {
-  return window_projection(a, s, plane_projection(a, pl, px, py), pixel_projection(a, s, px, py), wp);
+  return window_projection(a.src[s], plane_projection(a, pl, px, py), pixel_projection(a.src[s], px, py), wp);
 }
 // The texture clamp [-1, W-1] x [-1, H-1] relative to (U0, V0).
 struct WinClamp {
@@ -870,12 +881,24 @@ __device__ __forceinline__ float ncc_strong_src(const PMArgs &a, const WinProj &
   return fmaxf(0.0f, fminf(2.0f, 1.0f - cov / sqrtf(rw.var_r * var_s)));
 }
 template <int kStage, bool kPairs, class RW>
-__device__ __forceinline__ float ncc_strong_proj(const PMArgs &a, int px, int py, int s, const PlaneProj &pp,
+__device__ __forceinline__ float ncc_strong_proj(const PMArgs &a, int px, int py, const SrcConst &sc, const PlaneProj &pp,
                                                  const RW &rw) {
   WinProj wp;
-  if (!window_projection(a, s, pp, pixel_projection(a, s, px, py), wp)) return 2.0f;
+  if (!window_projection(sc, pp, pixel_projection(sc, px, py), wp)) return 2.0f;
   if (rw.cnt) atomicAdd(rw.cnt, 1ull);
-  return ncc_strong_src<decltype(SrcOf<kStage>::make(a, s)), kPairs, RW>(a, wp, SrcOf<kStage>::make(a, s), rw);
+  using Src = decltype(SrcOf<kStage>::make(a, 0));
+  return ncc_strong_src<Src, kPairs, RW>(a, wp, src_of<Src>(a, sc.texels), rw);
+}
+// The sources of a call with the images that a kernel of staging kStage samples, copied by the block's
+// threads (to shared memory: every evaluation reads 15 values of its source, which the gathers push out of
+// L1; strong update on 1600x1200 views 51.3 -> 50.2 and 51.9 -> 51.0 ms.  DepthToWeak, whose warps stay
+// with a source for long, is 2 % slower with it and reads the argument block).
+template <int kStage>
+__device__ __forceinline__ void load_sources(const PMArgs &a, SrcConst *out, int thread, int threads) {
+  for (int j = thread; j < a.N - 1; j += threads) {
+    out[j] = a.src[j + 1];
+    out[j].texels = SrcOf<kStage>::make(a, j + 1).p;
+  }
 }
 template <int kStage = DPE_STAGE_FP32, bool kPairs = false, class RW>
 __device__ __forceinline__ float ncc_strong(const PMArgs &a, int px, int py, int s, float4 pl, const RW &rw) {

@@ -1,10 +1,10 @@
-// pm_kernels.cuh -- the per-view PatchMatch kernels (one thread per pixel of a pass).
+// pm_kernels.cuh -- the per-view PatchMatch kernels.
 //
 // Kernel order and per-pixel semantics follow DPE::RunPatchMatch (DPE.cu:3130-3262).  B200
 // design points: all per-call constants (cameras, relative poses, params, pointers) live in one
 // argument block in device memory (one per problem of a batch); state is structure-of-arrays; view weights are packed as
 // 4-bit counts (16 B per pixel instead of 32); the strong NCC's reference window is built once
-// per thread and reused by every hypothesis and source view; the same-colour race of the
+// per pixel and pass and reused by every hypothesis and source view; the same-colour race of the
 // edge-aware update is removed by reading candidates from a pre-pass snapshot.
 #pragma once
 
@@ -1017,7 +1017,7 @@ __device__ __forceinline__ bool gn_solve(const PMArgs &a, int px, int py, float4
 // reference's order, so the random draws and the order of each weighted sum are those of one thread
 // doing it all.  Everything a pixel needs stays within its warp, so phases end with a warp barrier; the
 // block barriers around an evaluation only keep the block's warps in the same code, which they fetch
-// together (without them the kernel waits on instruction fetch: 62.4 against 55.8 ms below).
+// together (without them the kernel waits on instruction fetch: 62.4 against 55.8 ms at that time).
 //
 // What bounds it: instruction issue and register reads of the tap loop (strong_tap2) and, with
 // several inlined copies of it, instruction fetch.  Hence one evaluation loop (strong_eval) that
@@ -1028,8 +1028,8 @@ __device__ __forceinline__ bool gn_solve(const PMArgs &a, int px, int py, float4
 //     sources already reaches the cost to beat neither: costs are not negative and rounded sums and
 //     quotients of such terms are monotone, so the full sum cannot fall below it.
 // Both leave every decision, and so every result bit, as it was.
-// Six launches on a 1600x1200 view: first call with 10 sources 69.1 -> 55.8 ms, geometric call with 9
-// and a fifth of the pixels WEAK 77.6 -> 55.3 ms; on a 801x603 level image 19.9 -> 12.6 ms.
+// Six launches on a 1600x1200 view: first call with 10 sources 69.1 -> 50.2 ms, geometric call with 9
+// and a fifth of the pixels WEAK 77.6 -> 51.0 ms; on a 801x603 level image 19.9 -> 12.1 ms.
 //
 // Stages (each: evaluate the list, then the work that follows from the costs and the next list):
 //   start  window taps, candidate search, the list of distinct candidates x all sources
@@ -1085,12 +1085,13 @@ struct CoopPixel {
   uint8_t first, second;   // positions in act of the two heaviest sources
   uint8_t na, live;
 };
-// Shared bytes of one block: the pixels' states, the warps' lists, then per pixel kRows cost rows of
-// n = N - 1 floats.
+// Shared bytes of one block: the pixels' states, the warps' lists, the n = N - 1 sources, then per pixel
+// kRows cost rows of n floats.
 __host__ __device__ inline size_t coop_smem_bytes(int n) {
-  return sizeof(CoopPixel) * kCoopPix + sizeof(uint16_t) * kListCap * (kCoopThreads / 32) +
+  return sizeof(CoopPixel) * kCoopPix + sizeof(uint16_t) * kListCap * (kCoopThreads / 32) + sizeof(SrcConst) * n +
          sizeof(float) * (size_t)kCoopPix * kRows * n;
 }
+static_assert(sizeof(uint16_t) * kListCap * (kCoopThreads / 32) % 8 == 0, "the sources are 8-byte aligned");
 
 // A pixel's stream whose next 16 numbers are at hand; a long rejection in random_normal goes on from the
 // generator.
@@ -1116,6 +1117,7 @@ struct CoopCtx {
   float *cost;       // this pixel's rows
   float *cost0;      // the rows of the warp's first pixel
   uint16_t *list;    // the warp's list: pixel of the warp | row << 2 | source << 7
+  SrcConst *src;     // the sources
 };
 
 __device__ __forceinline__ CoopCtx coop_ctx(const Launch &lc, int parity, void *smem) {
@@ -1138,7 +1140,8 @@ __device__ __forceinline__ CoopCtx coop_ctx(const Launch &lc, int parity, void *
   c.W0 = base + warp * kWarpPix;
   uint16_t *lists = reinterpret_cast<uint16_t *>(base + kCoopPix);
   c.list = lists + (size_t)warp * kListCap;
-  float *rows = reinterpret_cast<float *>(lists + (size_t)kListCap * (kCoopThreads / 32));
+  c.src = reinterpret_cast<SrcConst *>(lists + (size_t)kListCap * (kCoopThreads / 32));
+  float *rows = reinterpret_cast<float *>(c.src + c.n);
   c.cost = rows + (size_t)c.slot * kRows * c.n;
   c.cost0 = rows + (size_t)warp * kWarpPix * kRows * c.n;
   return c;
@@ -1187,13 +1190,15 @@ __device__ __forceinline__ void strong_eval(const CoopCtx &c, int ns) {
     const PlaneProj pp{(double)hp.nx * a.dm[0], (double)hp.ny * a.dm[1], hp.iw, hp.q};
     const SmemWindow rw{Q.win, Q.center, Q.inv_wsum, Q.mean_r, Q.var_r,
                         a.counters ? a.counters + 2 * KID_STRONG_UPDATE : nullptr};
-    c.cost0[((size_t)k * kRows + h) * c.n + j] = ncc_strong_proj<kStage, true>(a, px, py, j + 1, pp, rw);
+    c.cost0[((size_t)k * kRows + h) * c.n + j] = ncc_strong_proj<kStage, true>(a, px, py, c.src[j], pp, rw);
     r += 32;
   }
 }
 
-// Window taps of build_ref_window, split over the lanes.
+// The sources; window taps of build_ref_window, split over the lanes.
+template <int kStage>
 __device__ __forceinline__ void strong_taps(const CoopCtx &c) {
+  load_sources<kStage>(*c.a, c.src, (int)threadIdx.x, kCoopThreads);  // read after the first block barrier
   if (!c.live) return;
   const PMArgs &a = *c.a;
   const int r = a.P.strong_radius, inc = a.P.strong_increment, side = 2 * r / inc + 1;
@@ -1776,7 +1781,7 @@ enum {
 template <int kStage, bool kGN>
 __device__ __forceinline__ void strong_phase(const CoopCtx &c, int phase, int iter) {
   switch (phase) {
-    case kPhTaps: strong_taps(c); break;
+    case kPhTaps: strong_taps<kStage>(c); break;
     case kPhSearch: strong_search(c, iter); break;
     case kPhDistinct: strong_distinct(c); break;
     case kPhList: strong_list(c); break;
@@ -2764,7 +2769,7 @@ __device__ __forceinline__ void lr_eval(const SweepCtx &c, int stage) {
     const int px = px0 + k, si = P.act[q] + 1;
     float4 t = P.pl;
     t.w = dist_to_origin(a.cam[0], px, c.py, pdep, t);
-    const float ncc = ncc_strong_proj<kStage, true>(a, px, c.py, si, plane_projection(a, t, px, c.py), c.window(P));
+    const float ncc = ncc_strong<kStage, true>(a, px, c.py, si, t, c.window(P));
     c.items0[((size_t)k * 12 + h) * n + q] = make_float2(ncc, geom ? geom_cost(a, px, c.py, si, t) : 0.0f);
   }
 }
