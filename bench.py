@@ -312,9 +312,20 @@ def cpu_reference_line(sampler: RefSampler, n_items: int):
     return pix / sched, per, desc, sched
 
 
+def reference_missing():
+    """Why the reference's own code cannot be timed here, or None."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import ref_py as R
+    return None if R.available() else "neither the reference's sources nor a library built from them are here"
+
+
 def run_reference(args):
     rank, world, _ = _env_rank()
     if rank != 0:
+        return 0
+    missing = reference_missing()
+    if missing:
+        print(json.dumps(dict(impl="reference", unavailable=missing)), flush=True)
         return 0
     threads = os.cpu_count() or 1
     sampler = RefSampler(threads)
@@ -558,7 +569,10 @@ def run_ours(args):
             dist.destroy_process_group()
         return 0
     cpu = None
-    if world == 1 and not args.no_cpu_baseline:
+    missing = reference_missing() if world == 1 and not args.no_cpu_baseline else None
+    if missing:
+        cpu = dict(unavailable=missing)
+    elif world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
         sampler = RefSampler(threads)
         cvalue, per, desc, _ = cpu_reference_line(sampler, len(RefSampler.KINDS))
