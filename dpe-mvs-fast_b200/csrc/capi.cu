@@ -61,6 +61,21 @@ void dpe_set_last_error(const char *what, cudaError_t err, const char *file, int
   g_last_error = buf;
 }
 
+cudaError_t dpe_allow_dynamic_smem(const void *func, size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;  // needs no opt-in
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, size_t> limit;  // per device
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t &have = limit[{dev, func}];
+  if (bytes <= have) return cudaSuccess;
+  err = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err == cudaSuccess) have = bytes;
+  return err;
+}
+
 bool dpe_debug_sync() {
   static const bool on = [] {
     const char *v = std::getenv("DPE_DEBUG_SYNC");
@@ -342,17 +357,12 @@ void set_carveout(const void *func, int percent) {
 }
 dim3 shape_grid(int W, int H, dim3 b) { return dim3((W + b.x - 1) / b.x, (H + b.y - 1) / b.y); }
 
-// Dynamic shared bytes above the 48 KB that need no opt-in (many sources).
-template <class K> cudaError_t allow_smem(K *kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 cudaError_t launch_strong_update(int staging, bool gn, dim3 grid, size_t smem, cudaStream_t s, const Launch args, int it,
                                  int parity, int carveout) {
   cudaError_t attr = cudaSuccess;
   with_stage(staging, [&](auto st) {
     auto go = [&](auto *kernel) {
-      if ((attr = allow_smem(kernel, smem)) != cudaSuccess) return;
+      if ((attr = dpe_allow_dynamic_smem((const void *)kernel, smem)) != cudaSuccess) return;
       set_carveout((const void *)kernel, carveout);
       kernel<<<grid, kCoopThreads, smem, s>>>(args, it, parity);
     };
@@ -725,7 +735,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   {
     cudaError_t attr = cudaSuccess;
     with_stage(staging, [&](auto st) {
-      attr = allow_smem(k_local_refine<decltype(st)::value>, g.lr_smem);
+      attr = dpe_allow_dynamic_smem((const void *)k_local_refine<decltype(st)::value>, g.lr_smem);
     });
     DPE_TRY(attr);
   }

@@ -24,6 +24,11 @@ void dpe_set_last_error(const char *what, cudaError_t err, const char *file, int
     }                                                                              \
   } while (0)
 
+// Lets `func` be launched with `bytes` of dynamic shared memory on the current device.  The limit
+// belongs to the function, for the whole process, and a launch above it fails; so it is raised under a
+// lock and never lowered, and what one host thread asked for holds while another's call needs less.
+cudaError_t dpe_allow_dynamic_smem(const void *func, size_t bytes);
+
 // After a kernel launch: report launch-configuration errors with the kernel's name; with
 // DPE_DEBUG_SYNC=1 in the environment also synchronise, so an execution error names its kernel
 // (the reference's DPE_POST_KERNEL, DPE.cu:3-7).

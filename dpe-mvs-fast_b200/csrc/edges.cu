@@ -1014,8 +1014,7 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
     if (!A.ok()) return DPE_ERR_OUT_OF_MEMORY;
     DPE_TRY(cudaMemcpyAsync(tab_d, tab.data(), numangle * sizeof(float2), cudaMemcpyHostToDevice, s));
     const size_t smem = in_shared ? shared(split) : walk_bytes;
-    if (smem > 48 * 1024)
-      DPE_TRY(cudaFuncSetAttribute(k_hough_region, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DPE_TRY(dpe_allow_dynamic_smem((const void *)k_hough_region, smem));
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim = {(unsigned)split, 1, 1};
