@@ -400,9 +400,20 @@ __global__ void k_mark_small(int *labels, int n, const int *__restrict__ counts,
   if (l != 0 && counts[l] <= weak_tex_num) labels[p] = -1;
 }
 
-__global__ void k_list_large(const int *__restrict__ counts, int cap, int weak_tex_num, int *list, int *nlist) {
+// The large regions, each with a share of the border points' scratch: a region's outer border has at most
+// four pixels per pixel of the region (its neighbours), and no more than the map.
+struct LargeRegions {
+  int n;
+  unsigned long long points;
+};
+__global__ void k_list_large(const int *__restrict__ counts, int cap, int weak_tex_num, int *list,
+                             unsigned long long *first_point, LargeRegions *large) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= 1 && k < cap && counts[k] > 0 && counts[k] >= weak_tex_num) list[atomicAdd(nlist, 1)] = k;
+  if (k >= 1 && k < cap && counts[k] > 0 && counts[k] >= weak_tex_num) {
+    const int at = atomicAdd(&large->n, 1);
+    list[at] = k;
+    first_point[at] = atomicAdd(&large->points, (unsigned long long)min((long long)counts[k] * 4, (long long)cap - 1));
+  }
 }
 
 // ---- HoughLinesP on one weak region's outer border, and its segments drawn --------------------
@@ -427,11 +438,13 @@ __global__ void k_list_large(const int *__restrict__ counts, int cap, int weak_t
 // 1100 at its barrier, 2500 of a segment for its walk.
 struct HoughArgs {
   const int *labels;  // first labelling, w x h
-  const int *regions; // region labels, one per CTA
+  const int *regions; // region labels, one per CTA or cluster
+  const unsigned long long *first_point;  // per region: where its points start
   int w, h, threshold, line_length, line_gap, numangle, numrho;
   const float2 *tab;  // (cos, sin) / rho in float, from the host's libm as OpenCV computes it
   unsigned *mask;     // per CTA: w*h bits; null: in shared memory (it is there whenever the counts are)
-  int2 *points;       // per CTA: w*h
+  int2 *points;       // per region and CTA of its cluster: the border, point_cap in all for one CTA each
+  unsigned long long point_cap;
   short *accum;       // per region: numangle*len counts; null: in shared memory
   int first, len;     // the bins that a point of the image can vote for
   int split;          // CTAs of a cluster that share a region's angles
@@ -503,7 +516,7 @@ __global__ void __launch_bounds__(kHoughThreads) k_hough_region(const __grid_con
     const int p = y * w + x;
     return ((mask[p >> 5] >> (p & 31)) & 1u) != 0;
   };
-  int2 *pts = a.points + (size_t)blockIdx.x * n;
+  int2 *pts = a.points + (size_t)rank * a.point_cap + a.first_point[blockIdx.x / split];
   int4 *lines = a.lines + (size_t)(blockIdx.x / split) * a.line_cap;
   // the region's outer border in raster order (DPE.cpp:168-182): not the region, 4-adjacent to it
   if (tid == 0) s_count = 0;
@@ -943,7 +956,8 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
   int *lab0 = A.get<int>("lb_lab0", n2);
   int *counts = A.get<int>("lb_counts", std::max(n2, n_out) + 1);
   int *regions = A.get<int>("lb_regions", n2 + 1);
-  int *nregions = A.get<int>("lb_nregions", 1);
+  unsigned long long *first_point = A.get<unsigned long long>("lb_first_point", n2 + 1);
+  LargeRegions *large = A.get<LargeRegions>("lb_large", 1);
   int *error = A.get<int>("lb_error", 1);
   if (!A.ok()) return DPE_ERR_OUT_OF_MEMORY;
   ConnectScratch cs;
@@ -967,13 +981,15 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
   }
   // first labelling and the large weak regions (DPE.cpp:162-166)
   if ((st = connect_device(ctx, dst, c2, r2, cs, lab0, counts)) != DPE_OK) return st;
-  DPE_TRY(cudaMemsetAsync(nregions, 0, sizeof(int), s));
+  DPE_TRY(cudaMemsetAsync(large, 0, sizeof(LargeRegions), s));
   DPE_TRY(cudaMemsetAsync(error, 0, sizeof(int), s));
-  k_list_large<<<(unsigned)((n2 + 1 + 255) / 256), 256, 0, s>>>(counts, (int)n2 + 1, weak_tex_num, regions, nregions);
+  k_list_large<<<(unsigned)((n2 + 1 + 255) / 256), 256, 0, s>>>(counts, (int)n2 + 1, weak_tex_num, regions, first_point,
+                                                               large);
   DPE_LAUNCHED("k_list_large", s);
-  int nreg = 0;
-  DPE_TRY(cudaMemcpyAsync(&nreg, nregions, sizeof(int), cudaMemcpyDeviceToHost, s));
+  LargeRegions lr{};
+  DPE_TRY(cudaMemcpyAsync(&lr, large, sizeof(lr), cudaMemcpyDeviceToHost, s));
   DPE_TRY(cudaStreamSynchronize(s));
+  const int nreg = lr.n;
   if (nreg > 0) {
     // Hough segments across each region's border, drawn on the Roberts map (DPE.cpp:164-190)
     const int thr = (int)(std::min(c2, r2) / 30.0);
@@ -1005,7 +1021,9 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
     if (!in_shared) split = 1;
     ha.split = split;
     ha.mask = in_shared ? nullptr : A.get<unsigned>("lb_mask", hough_mask_words(n2) * nreg);
-    ha.points = A.get<int2>("lb_points", n2 * nreg * split);
+    ha.first_point = first_point;
+    ha.point_cap = lr.points;
+    ha.points = A.get<int2>("lb_points", lr.points * split);
     ha.accum = in_shared ? nullptr : A.get<short>("lb_accum", (size_t)numangle * ha.len * nreg);
     ha.lines = A.get<int4>("lb_lines", (size_t)line_cap * nreg);
     ha.line_cap = line_cap;
