@@ -426,8 +426,7 @@ __global__ void k_list_large(const int *__restrict__ counts, int cap, int weak_t
 //     the stored ones plus its own earlier votes of the round for the same bin.  Only when some count
 //     reaches the threshold does a point's argmax matter: the votes up to the first such point are
 //     stored, its segment is handled, and the next round starts behind it.  Otherwise all are stored;
-//   * the counts lie in shared memory, 16 bits each (a bin cannot hold more points than its line has
-//     pixels): a vote touches 180 rows, from L2 or L1 180 separate lines.  Where one CTA's shared
+//   * the counts lie in shared memory, 16 bits each (kHoughMaxSide): a vote touches 180 rows, from L2 or L1 180 separate lines.  Where one CTA's shared
 //     memory is too small, 2, 4 or 8 CTAs of a cluster split the angles; each keeps its own copy of the
 //     mask and of the order and makes every walk, and a round exchanges only which points reached the
 //     threshold and with what angle;
@@ -478,7 +477,11 @@ __device__ void draw_line8(uint8_t *img, int width, int x1, int y1, int x2, int 
 constexpr int kHoughThreads = 256, kHoughVotes = 8, kHoughMaxSplit = 8;
 // Shared bytes a CTA may take for the walk, the mask and the counts.
 constexpr size_t kHoughShared = 200 * 1024;
-inline size_t hough_walk_bytes(int w, int h) { return (size_t)2 * (std::max(w, h) + 2) * sizeof(int2); }
+inline size_t hough_walk_bytes(int w, int h) { return (size_t)2 * (std::max(w, h) + 2) * sizeof(short2); }
+// Maps with a longer side than this are refused.  Up to it the 16-bit counts hold: a bin is a strip one
+// pixel wide, which meets each row of a steep line (each column of a flat one) in at most two pixels, so a
+// count stays within twice the longer side, 28890.
+constexpr int kHoughMaxSide = 14445;
 inline size_t hough_mask_words(size_t pixels) { return (pixels + 31) / 32; }
 
 inline size_t hough_acc_bytes(int numangle, int split, int len) {
@@ -486,7 +489,7 @@ inline size_t hough_acc_bytes(int numangle, int split, int len) {
 }
 
 __global__ void __launch_bounds__(kHoughThreads) k_hough_region(const __grid_constant__ HoughArgs a) {
-  extern __shared__ int2 walk[];  // pixels withdrawn by one segment, both directions; then the mask, the counts
+  extern __shared__ short2 walk[];  // pixels withdrawn by one segment, both directions; then the mask, the counts
   typedef cub::BlockScan<int, kHoughThreads> ScanI;
   __shared__ typename ScanI::TempStorage ts_i;
   __shared__ int s_count, s_nwalk, s_nlines;
@@ -730,7 +733,7 @@ __global__ void __launch_bounds__(kHoughThreads) k_hough_region(const __grid_con
           const unsigned take = __ballot_sync(0xffffffffu, m);
           if (m) {
             const int to = nw + __popc(take & ((1u << lane) - 1u));
-            if (to < walk_cap) walk[to] = q;
+            if (to < walk_cap) walk[to] = make_short2((short)q.x, (short)q.y);
             const int p = q.y * w + q.x;
             atomicAnd(&mask[p >> 5], ~(1u << (p & 31)));
           }
@@ -992,6 +995,10 @@ int dpe_edge_labels_device(dpe_ctx *ctx, const uint8_t *gray, int W, int H, int 
   const int nreg = lr.n;
   if (nreg > 0) {
     // Hough segments across each region's border, drawn on the Roberts map (DPE.cpp:164-190)
+    if (std::max(c2, r2) > kHoughMaxSide) {
+      dpe_set_last_error("k_hough_region", cudaErrorInvalidValue, __FILE__, __LINE__);
+      return DPE_ERR_CUDA;
+    }
     const int thr = (int)(std::min(c2, r2) / 30.0);
     const float theta = (float)(3.14159265358979323846 / 180.0);
     int numangle = (int)std::floor(3.14159265358979323846 / theta) + 1;
