@@ -62,17 +62,21 @@ void dpe_set_last_error(const char *what, cudaError_t err, const char *file, int
 }
 
 cudaError_t dpe_allow_dynamic_smem(const void *func, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;  // needs no opt-in
   static std::mutex mu;
   static std::map<std::pair<int, const void *>, size_t> limit;  // per device
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
   std::lock_guard<std::mutex> lock(mu);
-  size_t &have = limit[{dev, func}];
-  if (bytes <= have) return cudaSuccess;
+  auto it = limit.find({dev, func});
+  if (it == limit.end()) {  // without an opt-in: 48 KB less the function's static shared memory
+    cudaFuncAttributes at;
+    if ((err = cudaFuncGetAttributes(&at, func)) != cudaSuccess) return err;
+    it = limit.emplace(std::make_pair(dev, func), (size_t)at.maxDynamicSharedSizeBytes).first;
+  }
+  if (bytes <= it->second) return cudaSuccess;
   err = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err == cudaSuccess) have = bytes;
+  if (err == cudaSuccess) it->second = bytes;
   return err;
 }
 
