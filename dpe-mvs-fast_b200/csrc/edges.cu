@@ -284,7 +284,10 @@ __global__ void k_threshold(uint8_t *d, int n, int thr) {
 // pixels, so a row of up to 2048 is one step of one scan; the step's length is its barriers and the
 // loads behind them, not its pixels.  (With a pixel per thread and a scan each for the count and the
 // minimum, a 1600x1200 map took 5.2 ms more than a 400x300 one; now 1.9 ms.)
-constexpr int kConnectThreads = 512, kConnectItems = 4;
+// Both grow with the warps of the block, so a row takes the smallest block that holds it in one step.
+// Label maps in all, with 512 threads for every row and with 32, 128 or 512: 0.69 -> 0.62 ms at 100x75,
+// 1.03 -> 0.93 at 200x150, 1.97 -> 1.73 at 400x300, 5.16 -> 5.08 at 800x600, 16.8 -> 16.6 at 1600x1200.
+constexpr int kConnectItems = 4;
 
 struct RunScan {
   int start;  // a run starts within the scanned prefix
@@ -297,12 +300,13 @@ struct RunScanOp {
   }
 };
 
-__global__ void __launch_bounds__(kConnectThreads) k_connect_rows(const uint8_t *__restrict__ img, int cols, int rows,
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) k_connect_rows(const uint8_t *__restrict__ img, int cols, int rows,
                                                                  int *__restrict__ lab,
                                                                  unsigned long long *__restrict__ join, int *nlab) {
-  typedef cub::BlockScan<RunScan, kConnectThreads> Scan;
+  typedef cub::BlockScan<RunScan, kThreads> Scan;
   __shared__ typename Scan::TempStorage ts;
-  __shared__ int s_next, s_carry, s_last[kConnectThreads];
+  __shared__ int s_next, s_carry, s_last[kThreads];
   const int tid = threadIdx.x;
   if (tid == 0) {
     s_next = 1;
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(kConnectThreads) k_connect_rows(const uint8_t 
   }
   __syncthreads();
   for (int y = 0; y < rows; ++y) {
-    for (int base = 0; base < cols; base += kConnectThreads * kConnectItems) {
+    for (int base = 0; base < cols; base += kThreads * kConnectItems) {
       const int x0 = base + tid * kConnectItems;
       const size_t p0 = (size_t)y * cols + x0;
       bool in[kConnectItems], leftj[kConnectItems], upj[kConnectItems], labelled[kConnectItems], opens[kConnectItems];
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(kConnectThreads) k_connect_rows(const uint8_t 
         }
         left = run[i];
       }
-      const int end = min(base + kConnectThreads * kConnectItems, cols) - 1;
+      const int end = min(base + kThreads * kConnectItems, cols) - 1;
       if (end >= x0 && end < x0 + kConnectItems) s_carry = last;
       if (tid == 0) s_next = next + total.opens;
       __syncthreads();
@@ -922,7 +926,14 @@ int connect_device(dpe_ctx *ctx, const uint8_t *img, int w, int h, ConnectScratc
   const int n = w * h, cap = n + 1;
   const unsigned bn = (unsigned)((n + 255) / 256), bc = (unsigned)((cap + 255) / 256);
   DPE_TRY(cudaMemsetAsync(c.join, 0, (size_t)cap * sizeof(unsigned long long), s));
-  DPE_TIMED(ctx, KID_EDGE_LABELS, s, k_connect_rows<<<1, kConnectThreads, 0, s>>>(img, w, h, c.lab, c.join, c.nlab));
+  auto rows = [&](auto threads) {  // the smallest block that holds a row in one step
+    constexpr int kThreads = decltype(threads)::value;
+    k_connect_rows<kThreads><<<1, kThreads, 0, s>>>(img, w, h, c.lab, c.join, c.nlab);
+  };
+  DPE_TIMED(ctx, KID_EDGE_LABELS, s,
+            if (w <= 32 * kConnectItems) rows(std::integral_constant<int, 32>());
+            else if (w <= 128 * kConnectItems) rows(std::integral_constant<int, 128>());
+            else rows(std::integral_constant<int, 512>()));
   DPE_LAUNCHED("k_connect_rows", s);
   k_connect_links<<<bc, 256, 0, s>>>(c.join, c.nlab, cap, c.conn_a);
   DPE_LAUNCHED("k_connect_links", s);
