@@ -741,11 +741,13 @@ __device__ __forceinline__ WinClamp window_clamp(const PMArgs &a, const WinProj 
 }
 // True when no tap (|dx|, |dy| <= r) can reach the clamp: the numerators are bounded by r times the sum
 // of their coefficients' magnitudes and the depth from below by |zc| minus the same for Z, so an offset
-// is at most their quotient; 1 % of slack covers the roundings.  The fraction is in [0, 1].
+// is at most their quotient.  The fraction is in [0, 1].  The roundings of a tap's depth and of den are below
+// 1e-6 |zc| together, so where den is above 1e-3 |zc| they are a tenth of the 1 % of slack; windows whose depth
+// nearly vanishes at a tap are clamped.
 __device__ __forceinline__ bool window_inside(const PMArgs &a, const WinProj &wp, float r) {
   const float den = 0.99f * (fabsf(wp.zc) - r * (fabsf(wp.h6) + fabsf(wp.h7)));
   const int mx = min(wp.U0, a.W - 2 - wp.U0), my = min(wp.V0, a.H - 2 - wp.V0);
-  return den > 1e-30f && den < 1e30f && r * (fabsf(wp.g03.x) + fabsf(wp.g14.x)) <= den * (float)mx &&
+  return den > fmaxf(1e-30f, 1e-3f * fabsf(wp.zc)) && den < 1e30f && r * (fabsf(wp.g03.x) + fabsf(wp.g14.x)) <= den * (float)mx &&
          r * (fabsf(wp.g03.y) + fabsf(wp.g14.y)) <= den * (float)my;
 }
 // bilinear_s at (U0 + x, V0 + y): the clamp to [-1, W-1] x [-1, H-1] and the split into texel and
