@@ -2531,7 +2531,8 @@ __global__ void k_filter_strong(const Launch lc, int parity) {
 //     warp's 32 threads: first each against its heaviest source, which alone rules out most (a sample
 //     counts only if its full cost, no less than that part, is 0.1 below the current one), then the
 //     others against the other sources; a source's samples next to each other (they lie along one
-//     line of its image).
+//     line of its image).  With a negative geom_factor costs can be negative: then every sample in the
+//     depth range is evaluated against every source (lr_bounds).
 // LocalRefine on a 1600x1200 view: first call with 10 sources 12.7 -> 3.3 ms, geometric call with 9
 // 14.4 -> 9.8 ms (13.7 without the heaviest source first); 801x603 3.9 -> 0.9 ms.
 struct SweepPixel {
@@ -2773,6 +2774,10 @@ __device__ __forceinline__ void lr_eval(const SweepCtx &c, int stage) {
     c.items0[((size_t)k * 12 + h) * n + q] = make_float2(ncc, geom ? geom_cost(a, px, c.py, si, t) : 0.0f);
   }
 }
+// Whether a sum of a plane's costs bounds it from below: the NCC is in [0, 2], the geometric cost in [0, 3].
+__device__ __forceinline__ bool lr_bounds(const PMArgs &a) {
+  return !(a.P.geom_consistency && a.P.geom_factor < 0.0f);
+}
 // The current cost, summed in the reference's order, and the samples in the depth range; a pixel that
 // no sample can change is closed.
 __device__ __forceinline__ void lr_current(const SweepCtx &c) {
@@ -2794,7 +2799,7 @@ __device__ __forceinline__ void lr_current(const SweepCtx &c) {
   }
   cost_now /= P.weight_normal;
   P.cost_now = cost_now;
-  if (!((double)cost_now > 0.1)) { P.ok = 0; return; }
+  if (lr_bounds(a) && !((double)cost_now > 0.1)) { P.ok = 0; return; }
   uint32_t open = 0;
   for (int pd = -5; pd <= 5; ++pd) {
     const float pdep = sweep_depth(a, P, pd);
@@ -2817,14 +2822,14 @@ __device__ __forceinline__ float lr_cost(const SweepCtx &c, int pd, int q0, int 
   return tc / P.weight_normal;
 }
 __device__ __forceinline__ void lr_drop(const SweepCtx &c) {
-  if (c.lane != 0 || !c.P->ok) return;
+  if (c.lane != 0 || !c.P->ok || !lr_bounds(*c.a)) return;
   SweepPixel &P = *c.P;
   for (int pd = -5; pd <= 5; ++pd)
     if (((P.open >> (pd + 5)) & 1u) && !((double)(P.cost_now - lr_cost(c, pd, P.first, P.first + 1)) > 0.1))
       P.open &= ~(1u << (pd + 5));
   if (!P.open) P.ok = 0;
 }
-// The best open sample.  The ones dropped would not change the outcome: the depth changes only when the
+// The best open sample.  The ones that bounds dropped would not change the outcome: the depth changes only when the
 // smallest cost is more than 0.1 below the current one, and a dropped sample's is not.
 __device__ __forceinline__ void lr_decide(const SweepCtx &c) {
   if (c.lane != 0 || !c.P->ok) return;
