@@ -2901,7 +2901,8 @@ __global__ void __launch_bounds__(kCoopThreads, DPE_LR_MIN_BLOCKS) k_local_refin
     if (stage == 0) lr_current(c);
     else if (stage == 1) lr_drop(c);
     else lr_decide(c);
-    if (!__syncthreads_or(c.P->ok)) return;  // the whole block is done
+    // the whole block is done (a pixel's first lane has just written its ok; the others read it after this)
+    if (!__syncthreads_or(c.lane == 0 && c.P->ok)) return;
   }
 }
 
