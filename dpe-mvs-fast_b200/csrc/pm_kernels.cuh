@@ -260,10 +260,13 @@ __global__ void k_edge_clear_cols(const uint8_t *__restrict__ rows, int w, int h
 
 // BresenhamLine (DPE.cu:162-248); out-of-image linear indices read 0.  A point's part (its place in the
 // low-resolution edge map, and whether it lies on an edge itself) is taken once per point.
-struct LinePoint {
-  short x, y;   // in the low-resolution map
-  uint8_t on;     // on an edge of the full-resolution map
-  uint8_t clear;  // no edge within max_step of it: a walk that starts here meets none
+struct LinePoint {  // 8 bytes: with 12, a block of GenNeighbours takes 3 KB more shared memory
+  unsigned x_on;    // x in the low-resolution map << 1 | on an edge of the full-resolution map
+  unsigned y_clear;  // y << 1 | no edge within max_step of it: a walk that starts here meets none
+  __device__ __forceinline__ int x() const { return (int)(x_on >> 1); }
+  __device__ __forceinline__ int y() const { return (int)(y_clear >> 1); }
+  __device__ __forceinline__ bool on() const { return x_on & 1u; }
+  __device__ __forceinline__ bool clear() const { return y_clear & 1u; }
 };
 struct LineMap {
   float scale_x, scale_y;
@@ -279,15 +282,14 @@ __device__ __forceinline__ LineMap line_map(const PMArgs &a) {
   return m;
 }
 __device__ __forceinline__ LinePoint line_point(const PMArgs &a, const LineMap &m, int x, int y) {
-  LinePoint p;
-  p.x = (short)(int)cvmin(roundf(x * m.scale_x), (float)(m.w - 1));
-  p.y = (short)(int)cvmin(roundf(y * m.scale_y), (float)(m.h - 1));
-  p.on = edge_at(a, (long)x + (long)y * a.W) ? 1 : 0;
+  const int lx = (int)cvmin(roundf(x * m.scale_x), (float)(m.w - 1));
+  const int ly = (int)cvmin(roundf(y * m.scale_y), (float)(m.h - 1));
+  const bool on = edge_at(a, (long)x + (long)y * a.W) != 0;
   // A step moves one place at most in x and in y, so max_step steps stay within that distance.  Near
   // the left and right borders a walk may pass the border by a step, where its linear index reads the
   // neighbouring row: such walks are always made.
-  p.clear = a.edge_dist && p.x >= m.max_step && p.x + m.max_step < m.w && a.edge_dist[p.x + p.y * m.w] ? 1 : 0;
-  return p;
+  const bool clear = a.edge_dist && lx >= m.max_step && lx + m.max_step < m.w && a.edge_dist[lx + (size_t)ly * m.w];
+  return LinePoint{(unsigned)lx << 1 | (on ? 1u : 0u), (unsigned)ly << 1 | (clear ? 1u : 0u)};
 }
 // One walk from (x0, y0) towards (x1, y1).  Out of line: the callers' loops stay in the instruction cache.
 #ifdef __CUDA_ARCH__
@@ -316,10 +318,10 @@ bool line_walk(const uint8_t *edge_low, int w, int h, int max_step, int x0, int 
   return false;
 }
 __device__ __forceinline__ bool line_blocked(const PMArgs &a, const LineMap &m, LinePoint A, LinePoint B) {
-  if (A.on || B.on) return false;
+  if (A.on() || B.on()) return false;
   for (int pass = 0; pass < 2; ++pass) {  // from B to A, then from A to B
     const LinePoint s = pass == 0 ? B : A, t = pass == 0 ? A : B;
-    if (!s.clear && line_walk(a.edge_low, m.w, m.h, m.max_step, s.x, s.y, t.x, t.y)) return true;
+    if (!s.clear() && line_walk(a.edge_low, m.w, m.h, m.max_step, s.x(), s.y(), t.x(), t.y())) return true;
   }
   return false;
 }
@@ -469,7 +471,7 @@ __device__ __forceinline__ void gen_neighbours_pixel(const PMArgs &a, const GnCa
       else if (g.lane == 0) a.complexity[center] = cvmax(0.99f, cv);
     }
   }
-  LinePoint here{0, 0, 0};
+  LinePoint here{0, 0};
   if (edge_limit) here = line_point(a, K.map, px, py);
   for (int odx = -1; odx <= 1; ++odx)
     for (int ody = -1; ody <= 1; ++ody) {
