@@ -1171,12 +1171,19 @@ extern "C" int dpe_kernel_info(char *buf, int len) {
 
 // ------------------------------------------------------------------ allocation-free NCC queries
 namespace {
-// Scratch of dpe_ncc_eval_noalloc: the per-call argument block followed by the clamp-padded
-// images.  Every GPU that loads the library holds these 16 MiB until the process exits.  Nothing
+// Scratch of dpe_ncc_eval_noalloc: the clamp-padded images, and the per-call argument block in an array of
+// its own.  Every GPU that loads the library holds these 16 MiB until the process exits.  Nothing
 // in it needs to start at zero: each call writes the whole argument block and every padded texel
 // it reads before the query kernel runs.
 constexpr size_t kStaticScratchBytes = size_t(16) << 20;
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// What of the 16 MiB no call's images take.  A fixed figure, so that the problems that fit do not change with
+// the argument block.
+constexpr size_t kStaticReserved = 9472;
+struct StaticScratch {
+  unsigned char images[kStaticScratchBytes - kStaticReserved];
+  unsigned char args[sizeof(PMArgs)];
+};
+static __device__ __align__(256) StaticScratch g_static_scratch;
 constexpr int kMaxDevices = 64;
 std::mutex g_static_mu;
 unsigned char *g_static_addr[kMaxDevices] = {};
@@ -1197,7 +1204,7 @@ extern "C" int dpe_ncc_eval_noalloc(const dpe_ncc_query *q, float *costs_out, vo
   if (q->count > 0 && (!q->px || !q->py || !q->src || !q->plane)) return DPE_ERR_INVALID_ARGUMENT;
   const size_t PL = (size_t)(W + 2) * (H + 2);
   const size_t img_bytes = round256(PL * sizeof(float));
-  const size_t need = round256(sizeof(PMArgs)) + (size_t)N * img_bytes;
+  const size_t need = kStaticReserved + (size_t)N * img_bytes;
   if (need > kStaticScratchBytes) {
     char buf[200];
     std::snprintf(buf, sizeof(buf), "dpe_ncc_eval_noalloc: %d padded %dx%d images need %zu bytes of scratch; the "
@@ -1227,15 +1234,15 @@ extern "C" int dpe_ncc_eval_noalloc(const dpe_ncc_query *q, float *costs_out, vo
   a.P.num_images = N;
   for (int i = 0; i < N; ++i) a.cam[i] = q->cameras[i];
   set_homography_bases(a);
-  unsigned char *img_base = base + round256(sizeof(PMArgs));
-  for (int i = 0; i < N; ++i) a.img[i] = reinterpret_cast<const float *>(img_base + (size_t)i * img_bytes);
+  PMArgs *args = reinterpret_cast<PMArgs *>(base + offsetof(StaticScratch, args));
+  for (int i = 0; i < N; ++i) a.img[i] = reinterpret_cast<const float *>(base + (size_t)i * img_bytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   PadSet pads = pad_set(a);
   for (int i = 0; i < N; ++i) pads.src[i] = q->images[i];
-  k_pad_store_args<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads, a, reinterpret_cast<PMArgs *>(base));
+  k_pad_store_args<<<pad_grid(W, H, N), kPadBlock, 0, s>>>(pads, a, args);
   DPE_LAUNCHED("k_pad_store_args", s);
   const int64_t n = q->count;
-  k_ncc_queries<true><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(reinterpret_cast<const PMArgs *>(base), n, q->px,
+  k_ncc_queries<true><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(args, n, q->px,
                                                                     q->py, q->src,
                                                                     reinterpret_cast<const float4 *>(q->plane),
                                                                     costs_out);

@@ -384,9 +384,8 @@ int dpe_ncc_grad_device(dpe_ctx *ctx, const dpe_ncc_query *q, const float *upstr
  *
  * Scratch (the argument block and the clamp-padded images) lives in one statically allocated
  * 16 MiB array in device memory, which every GPU that loads this library holds until the process
- * exits.  A problem is accepted when 256-byte-rounded sizeof(argument block) plus num_images x
- * 256-byte-rounded (width + 2) x (height + 2) x 4 bytes fits in 16 MiB (e.g. up to 12 images of
- * 640x480); larger ones return DPE_ERR_CAPACITY with the sizes in dpe_last_error().  The first
+ * exits.  A problem is accepted when 9472 bytes plus num_images x 256-byte-rounded
+ * (width + 2) x (height + 2) x 4 bytes fit in 16 MiB (e.g. up to 12 images of 640x480); larger ones return DPE_ERR_CAPACITY with the sizes in dpe_last_error().  The first
  * call on a device resolves the array's device address (cudaGetSymbolAddress) with that device
  * current; make that first call before any stream capture.  All calls share the one array and
  * it keeps the previous call's contents, so calls that overlap on the GPU (different streams or
