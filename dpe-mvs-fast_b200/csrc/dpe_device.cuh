@@ -1032,6 +1032,8 @@ __device__ __forceinline__ void weak_window_shape(const PMArgs &a, int center, i
 // first two rows of every column and the third row of the first two, all windows' pairs after each other,
 // then the windows' last taps; so a pair is one aligned 16-byte load.  Windows of another size: plain
 // (w, w * (r - c)) in tap order.
+// The centre window of use_radius can have more taps than the table holds (its step is at least 2 and
+// may be below strong_increment: radius 7 has 8 x 8).  Those past the table are made where they are read.
 __device__ __forceinline__ bool weak_is3(const PMArgs &a) { return a.wtaps == 9; }
 __device__ __forceinline__ const float4 *weak_pairs(const PMArgs &a, const float2 *tab, int k) {
   return reinterpret_cast<const float4 *>(tab) + (k == 0 ? 0 : kWinPairs + 4 * (k - 1));
@@ -1043,7 +1045,7 @@ __device__ __forceinline__ const float2 *weak_plain(const PMArgs &a, const float
 // Stores tap t of window k.
 __device__ __forceinline__ void weak_store(const PMArgs &a, float2 *tab, int k, int t, float w, float wr) {
   if (k == 0) {
-    win_store(reinterpret_cast<float4 *>(tab), t, w, wr);
+    if (t < kWinTaps) win_store(reinterpret_cast<float4 *>(tab), t, w, wr);
   } else if (!weak_is3(a)) {
     tab[kWinTaps + (k - 1) * a.wtaps + t] = make_float2(w, wr);
   } else if (t == 8) {
@@ -1059,6 +1061,19 @@ __device__ __forceinline__ float2 weak_load(const PMArgs &a, const float2 *tab, 
   if (t == 8) return *weak_last(tab, k);
   const int c = t / 3, r = t - 3 * c;
   return win_tap(weak_pairs(a, tab, k), r < 2 ? 2 * c + r : 6 + c);
+}
+
+// Tap t of the centre window of pixel (cx, cy), as weak_prepare makes it.  Out of line: hardly ever taken.
+#ifdef __CUDACC__
+static __device__ __noinline__
+#else
+inline
+#endif
+float2 center_tap(const PMArgs &a, int cx, int cy, int radius, int inc, int t) {
+  const int side = 2 * radius / inc + 1, i = t / side * inc - radius, j = t % side * inc - radius;
+  const float c = texel(a, 0, cx, cy), rp = texel(a, 0, cx + i, cy + j);
+  const float w = bilateral_weight((float)i, (float)j, rp, c, a.P.sigma_spatial, a.P.sigma_color);
+  return make_float2(w, w * (rp - c));
 }
 
 // The hypothesis-dependent sums of a window column: w*s, w*s^2, w*(r-c)*s.
@@ -1172,8 +1187,10 @@ __device__ __forceinline__ float window_ncc_tab(const PMArgs &a, const float H[9
     for (int i = -radius; i <= radius; i += inc, x += finc) {
       WeakSums r = {0, 0, 0};
       float y = y0;
-      for (int j = -radius; j <= radius; j += inc, y += finc)
-        weak_tap(a, H, src, x, y, ref_center, weak_load(a, tab, k, t++), r);
+      for (int j = -radius; j <= radius; j += inc, y += finc, ++t) {
+        const float2 w = k == 0 && t >= kWinTaps ? center_tap(a, cx, cy, radius, inc, t) : weak_load(a, tab, k, t);
+        weak_tap(a, H, src, x, y, ref_center, w, r);
+      }
       s_s += r.s; s_ss += r.ss; s_rs += r.rs;
     }
   }
