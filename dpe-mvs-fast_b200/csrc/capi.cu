@@ -571,17 +571,21 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
     if (!(inexact & 1u)) staging = DPE_STAGE_BF16;
     else if (!(inexact & 2u)) staging = DPE_STAGE_FP16;
   }
+  uint2 *img_quads = staging != DPE_STAGE_FP32 ? get((uint2 *)0, "img_quads", PL * (N - 1)) : nullptr;
+  if (staging != DPE_STAGE_FP32 && !img_quads) {
+    if (ctx->opt.staging != DPE_STAGE_FP32) return DPE_ERR_OUT_OF_MEMORY;
+    A.ok();  // the quads are twice the images: where they do not fit, the FP32 images give the same results
+    staging = DPE_STAGE_FP32;
+  }
   ps->staging = staging;
   a.stage = staging;
-  uint2 *img_quads = staging != DPE_STAGE_FP32 ? get((uint2 *)0, "img_quads", PL * N) : nullptr;
-  if (staging != DPE_STAGE_FP32 && !img_quads) return DPE_ERR_OUT_OF_MEMORY;
   if (staging != DPE_STAGE_FP32) {
-    for (int i = 1; i < N; ++i) a.quad[i] = img_quads + PL * i;
+    for (int i = 1; i < N; ++i) a.quad[i] = img_quads + PL * (i - 1);
     const dim3 grid((unsigned)((PL + 255) / 256), N - 1);
     if (staging == DPE_STAGE_BF16)
-      k_stage_quads<true><<<grid, 256, 0, s>>>(img_pad + PL, img_quads + PL, (long long)PL, W + 2);
+      k_stage_quads<true><<<grid, 256, 0, s>>>(img_pad + PL, img_quads, (long long)PL, W + 2);
     else
-      k_stage_quads<false><<<grid, 256, 0, s>>>(img_pad + PL, img_quads + PL, (long long)PL, W + 2);
+      k_stage_quads<false><<<grid, 256, 0, s>>>(img_pad + PL, img_quads, (long long)PL, W + 2);
     PM_LAUNCHED("k_stage_quads", s);
   }
   return DPE_OK;
