@@ -255,9 +255,6 @@ template <class F> void with_stage(int staging, F &&f) {
 // writes only its own pixel, so the shape changes nothing but speed; all fit __launch_bounds__(128)).
 const dim3 kShapeCands[] = {dim3(16, 8), dim3(32, 4), dim3(8, 16), dim3(64, 2), dim3(8, 8)};
 constexpr int kNumShapes = 5;
-// Shared-memory carveouts (percent; -1 the driver's choice) tried for the cooperative kernels.
-const int kCarveCands[] = {-1, 100, 75, 50};
-constexpr int kNumCarves = 4;
 
 int size_class(long long pixels) {
   int c = 0;
@@ -346,28 +343,14 @@ struct TunedLaunch {
     e->pending.push_back(TuneEntry::Pend{cand, t0, t1});
   }
 };
-// The preferred carveout of a kernel function, set only when it changes (the attribute belongs
-// to the function, process-wide).
-void set_carveout(const void *func, int percent) {
-  static std::mutex mu;
-  static std::map<const void *, int> current;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = current.find(func);
-  if (it != current.end() && it->second == percent) return;
-  if (cudaFuncSetAttribute(func, cudaFuncAttributePreferredSharedMemoryCarveout, percent) == cudaSuccess)
-    current[func] = percent;
-  else
-    cudaGetLastError();
-}
 dim3 shape_grid(int W, int H, dim3 b) { return dim3((W + b.x - 1) / b.x, (H + b.y - 1) / b.y); }
 
 cudaError_t launch_strong_update(int staging, bool gn, dim3 grid, size_t smem, cudaStream_t s, const Launch args, int it,
-                                 int parity, int carveout) {
+                                 int parity) {
   cudaError_t attr = cudaSuccess;
   with_stage(staging, [&](auto st) {
     auto go = [&](auto *kernel) {
       if ((attr = dpe_allow_dynamic_smem((const void *)kernel, smem)) != cudaSuccess) return;
-      set_carveout((const void *)kernel, carveout);
       kernel<<<grid, kCoopThreads, smem, s>>>(args, it, parity);
     };
     if (gn) go(k_strong_update<decltype(st)::value, true>);
@@ -631,12 +614,12 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
       DPE_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, ps[b].weak_flag, a.nmap, L, s));
     }
   }
-  // Launch settings the tuner picks (results do not depend on them): the block shape of the random
-  // initialisation for one problem (a batch keeps the 16 x 8 layout its block table is built for)
-  // and the shared-memory carveout of the strong update.  These two do the same work in every
-  // launch of a size class, so launches with different settings compare; the kernels whose work
-  // follows a view's weak pixels (GenNeighbours, the nearest-strong search, the plane fit,
-  // DepthToWeak, LocalRefine) keep hand-measured settings, since their samples would compare views.
+  // The launch setting the tuner picks (results do not depend on it): the block shape of the random
+  // initialisation for one problem (a batch keeps the 16 x 8 layout its block table is built for), which
+  // does the same work in every launch of a size class, so launches with different settings compare.
+  // The other kernels keep hand-measured settings: the work of GenNeighbours, the nearest-strong search,
+  // the plane fit, DepthToWeak and LocalRefine follows a view's weak pixels, the strong update's the
+  // iteration, and their samples would compare those.
   long long pix_all = 0;
   for (int b = 0; b < n; ++b) pix_all += (long long)ps[b].L;
   auto shaped = [&](int kid, auto launch) {
@@ -647,15 +630,6 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
     TunedLaunch t(ctx, kid, pix_all, kNumShapes, s);
     const dim3 bl = kShapeCands[t.cand];
     launch(shape_grid(ps[0].a.W, ps[0].a.H, bl), bl);
-    t.finish();
-  };
-  auto carved = [&](int kid, auto launch) {
-    if (kid != KID_STRONG_UPDATE) {
-      launch(-1);
-      return;
-    }
-    TunedLaunch t(ctx, kid, pix_all, kNumCarves, s);
-    launch(kCarveCands[t.cand]);
     t.finish();
   };
   // edge distances with edges, label boundaries of WEAK pixels with APD: else nothing to do
@@ -703,9 +677,14 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
           DPE_TRY(cudaMemcpyAsync(a.cost_snap, a.cost, ps[b].L * 4, cudaMemcpyDeviceToDevice, s));
         }
       cudaError_t attr = cudaSuccess;
-      DPE_TIMED(ctx, KID_STRONG_UPDATE, s, carved(KID_STRONG_UPDATE, [&](int cv) {
-                  attr = launch_strong_update(staging, gn, g.cg, g.coop_smem, s, g.coop, it, parity, cv);
-                }));
+      // The driver's split of L1 and shared memory, whichever the size: of 29 calls (160x120 to 1600x1200, 3 to
+      // 21 images, first and geometric) it was the fastest or within 0.2 % of it, where 100 % took 1 to 14 %
+      // longer, 75 % 0 to 2 % and 50 % 9 to 64 %.  One setting, which dpe_ctx_get_tuning lists.
+      DPE_TIMED(ctx, KID_STRONG_UPDATE, s, {
+        TunedLaunch t(ctx, KID_STRONG_UPDATE, pix_all, 1, s);
+        attr = launch_strong_update(staging, gn, g.cg, g.coop_smem, s, g.coop, it, parity);
+        t.finish();
+      });
       DPE_TRY(attr);
       PM_LAUNCHED("k_strong_update", s);
     }
@@ -733,12 +712,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
     DPE_TIMED(ctx, KID_FILTER, s, k_filter_strong<<<g.hg, g.hb, 0, s>>>(g.half, parity));
     PM_LAUNCHED("k_filter_strong", s);
   }
-  DPE_TIMED(ctx, KID_DEPTH_TO_WEAK, s, carved(KID_DEPTH_TO_WEAK, [&](int cv) {
-              with_stage(staging, [&](auto st) {
-                set_carveout((const void *)k_depth_to_weak<decltype(st)::value>, cv);
-                k_depth_to_weak<decltype(st)::value><<<g.sg, kCoopThreads, 0, s>>>(g.sweep);
-              });
-            }));
+  DPE_TIMED(ctx, KID_DEPTH_TO_WEAK, s, with_stage(staging, [&](auto st) { k_depth_to_weak<decltype(st)::value><<<g.sg, kCoopThreads, 0, s>>>(g.sweep); }));
   PM_LAUNCHED("k_depth_to_weak", s);
   {
     cudaError_t attr = cudaSuccess;
@@ -747,12 +721,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
     });
     DPE_TRY(attr);
   }
-  DPE_TIMED(ctx, KID_LOCAL_REFINE, s, carved(KID_LOCAL_REFINE, [&](int cv) {
-              with_stage(staging, [&](auto st) {
-                set_carveout((const void *)k_local_refine<decltype(st)::value>, cv);
-                k_local_refine<decltype(st)::value><<<g.sg, kCoopThreads, g.lr_smem, s>>>(g.sweep);
-              });
-            }));
+  DPE_TIMED(ctx, KID_LOCAL_REFINE, s, with_stage(staging, [&](auto st) { k_local_refine<decltype(st)::value><<<g.sg, kCoopThreads, g.lr_smem, s>>>(g.sweep); }));
   PM_LAUNCHED("k_local_refine", s);
   return DPE_OK;
 }
@@ -1318,9 +1287,8 @@ extern "C" int dpe_ctx_get_tuning(dpe_ctx *ctx, dpe_tuning_entry *out, int capac
       o.size_class = (int)(kv.first % 64);
       o.candidates = e.ncand;
       o.chosen = e.chosen;
-      const bool carve = kid == KID_STRONG_UPDATE || kid == KID_DEPTH_TO_WEAK || kid == KID_LOCAL_REFINE;
       if (e.chosen >= 0) {
-        if (carve) o.carveout = kCarveCands[e.chosen];
+        if (kid == KID_STRONG_UPDATE) o.carveout = -1;
         else { o.block_x = (int)kShapeCands[e.chosen].x; o.block_y = (int)kShapeCands[e.chosen].y; }
       }
       for (int i = 0; i < e.ncand && i < 8; ++i) o.mean_ms[i] = e.count[i] ? (float)(e.sum[i] / e.count[i]) : 0.f;

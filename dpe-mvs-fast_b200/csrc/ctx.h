@@ -93,9 +93,8 @@ class Arena {
 #include "kernel_ids.h"
 
 // ------------------------------------------------------------------ launch tuner
-// Online choice of launch settings that change no result: the block shape of the
-// one-thread-per-pixel kernels and the shared-memory carveout of the cooperative ones.  Per
-// (kernel, size class) the first launches cycle through the candidates, each timed by an event
+// Online choice of launch settings that change no result: the block shape of the random
+// initialisation.  Per (kernel, size class) the first launches cycle through the candidates, each timed by an event
 // pair on its stream; the times are read without synchronising, once the events have completed.
 // When every candidate has kRounds samples, the lowest mean is kept for every later launch.
 struct TuneEntry {

@@ -447,10 +447,10 @@ int dpe_ctx_get_kernel_stats(dpe_ctx *ctx, dpe_kernel_stat *out, int capacity, i
 /* Launch tuner (no reference counterpart; the reference launches fixed 16x16 blocks).  For each
  * (kernel, size class = floor(log2 of the call's pixels)) the context's first launches cycle
  * through candidate settings that change no result -- the block shape of the random
- * initialisation (16x8, 32x4, 8x16, 64x2, 8x8; single-problem calls only) and the shared-memory
- * carveout of the strong update (driver default, 100, 75, 50 %), the two kernels whose launches
- * of one size class do the same work -- each timed by an event pair on the context's stream, and
- * keep the fastest mean after 2 samples each.  On by default; dpe_ctx_set_autotune(ctx, 0) uses
+ * initialisation (16x8, 32x4, 8x16, 64x2, 8x8; single-problem calls only), whose launches of one
+ * size class do the same work -- each timed by an event pair on the context's stream, and
+ * keep the fastest mean after 2 samples each.  The strong update is listed with its one setting,
+ * the driver's shared-memory carveout.  On by default; dpe_ctx_set_autotune(ctx, 0) uses
  * the first candidate throughout. */
 int dpe_ctx_set_autotune(dpe_ctx *ctx, int on);
 typedef struct dpe_tuning_entry {
@@ -460,8 +460,7 @@ typedef struct dpe_tuning_entry {
   int chosen;         /* index of the kept setting; -1 while still measuring                   */
   int block_x;        /* block shape of the kept setting (shape-tuned kernels; else 0)         */
   int block_y;
-  int carveout;       /* carveout of the kept setting in percent, -1 the driver default
-                         (carveout-tuned kernels; else 0)                                      */
+  int carveout;       /* strong update: -1, the driver's shared-memory carveout; else 0        */
   float mean_ms[8];   /* mean measured time per candidate (0: no sample)                       */
 } dpe_tuning_entry;
 int dpe_ctx_get_tuning(dpe_ctx *ctx, dpe_tuning_entry *out, int capacity, int *count);
