@@ -561,7 +561,6 @@ int setup_problem(dpe_ctx *ctx, const dpe_problem *p, int index, ProblemState *p
     staging = DPE_STAGE_FP32;
   }
   ps->staging = staging;
-  a.stage = staging;
   if (staging != DPE_STAGE_FP32) {
     for (int i = 1; i < N; ++i) a.quad[i] = img_quads + PL * (i - 1);
     const dim3 grid((unsigned)((PL + 255) / 256), N - 1);
@@ -616,7 +615,7 @@ int run_sequence(dpe_ctx *ctx, ProblemState *ps, int n, const PMArgs *d_args, co
   }
   // The launch setting the tuner picks (results do not depend on it): the block shape of the random
   // initialisation for one problem (a batch keeps the 16 x 8 layout its block table is built for), which
-  // does the same work in every launch of a size class, so launches with different settings compare.
+  // does the same work in every launch of a stage and size class, so launches with different settings compare.
   // The other kernels keep hand-measured settings: the work of GenNeighbours, the nearest-strong search,
   // the plane fit, DepthToWeak and LocalRefine follows a view's weak pixels, the strong update's the
   // iteration, and their samples would compare those.
@@ -1098,6 +1097,8 @@ extern "C" int dpe_ncc_grad_device(dpe_ctx *ctx, const dpe_ncc_query *q, const f
                                                                reinterpret_cast<float4 *>(grad_depth_normal_out),
                                                                grad_images_out);
   PM_LAUNCHED("k_ncc_grad", s);
+  // The caller's stream is not the context's: the next call of this context, on whichever stream, may write the
+  // padded images and the argument block, or free them where the arena grows.
   DPE_TRY(cudaStreamSynchronize(s));
   return DPE_OK;
 }

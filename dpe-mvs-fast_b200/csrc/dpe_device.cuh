@@ -22,10 +22,12 @@ constexpr int kMaxSrc = DPE_MAX_IMAGES - 1;
 constexpr int kNeighbours = DPE_NEIGHBOUR_NUM;
 constexpr int kMaxWin = 6;  // taps per window side for radius 5 / step 2 (DPE.cu:728-737)
 // Minimum resident blocks per multiprocessor requested for the strong-window cost kernels
-// (__launch_bounds__): bounds their registers, trading spills against occupancy.  Measured on a
-// 1600x1200 view, first call with 10 sources / geometric call with 9 (ms): strong update at 8 blocks
-// 77.9 / 74.2, at 6 64.8 / 61.2, at 5 (96 registers, no spills) 62.7 / 62.1, at 4 59.1 / 61.8, the
-// latter slower at 160x120 (0.59 against 0.52); DepthToWeak at 8, 6 and 5 blocks 50.7, 49.7 and 51.1.
+// (__launch_bounds__): bounds their registers, trading spills against occupancy.  Measured on the
+// present kernels, first call at 1600x1200 with 10 sources / geometric call with 9 / first call at 160x120
+// with 3 (ms): strong update at 6 blocks 54.9 / 51.0 / 0.410, at 5 (96 registers, no spills) 50.2 / 51.0 /
+// 0.392, at 4 47.9 / 50.1 / 0.472: small calls lose what large ones gain (with 20 sources at 640x480, whose
+// shared memory lets four blocks in anyway, 4 would take 12.2 against 14.6).  DepthToWeak at 8, 6 and 5 blocks
+// 48.0 / 54.5 / 0.168, 46.6 / 52.7 / 0.168 and 48.3 / 54.8 / 0.162.
 #ifndef DPE_COST_MIN_BLOCKS
 #define DPE_COST_MIN_BLOCKS 1
 #endif
@@ -35,8 +37,8 @@ constexpr int kMaxWin = 6;  // taps per window side for radius 5 / step 2 (DPE.c
 #ifndef DPE_SWEEP_MIN_BLOCKS
 #define DPE_SWEEP_MIN_BLOCKS 6
 #endif
-// LocalRefine: at 6, 5 blocks and unbounded 3.31, 3.37, 3.38 ms / 14.2, 13.7, 13.4 ms / 0.96, 0.93, 1.15
-// ms (first call, geometric call, 801x603 level)
+// LocalRefine: at 6, 5 blocks and unbounded 3.13, 3.26, 3.27 ms / 9.71, 9.73, 9.80 ms / 0.863, 0.885, 0.891
+// ms (first call, geometric call, 801x603 level), but 1.01, 0.96, 0.87 ms with 20 sources at 640x480
 #ifndef DPE_LR_MIN_BLOCKS
 #define DPE_LR_MIN_BLOCKS 5
 #endif
@@ -65,7 +67,6 @@ struct PMArgs {
   // offset o, the texels P[o], P[o+1], P[o+pw], P[o+pw+1], as four 16-bit values, so a bilinear
   // footprint is one 8-byte load.
   const uint2 *quad[kMaxImages];
-  int stage;  // DPE_STAGE_*: storage the cost kernels sample the source images from
   int gn;     // 1: Gauss-Newton plane hypothesis in the strong update (dpe_options::gn_refine)
   int far;    // 1: byte offsets into a staged image need more than 32 bits (fetch_bytes)
   int six;    // 1: the strong window is the 6 x 6 one (radius 5, step 2) and the image not far
@@ -207,18 +208,6 @@ __device__ __forceinline__ uint32_t philox_word0(uint32_t c0, uint32_t c1, uint3
   }
   return c0;
 }
-__device__ __forceinline__ void philox4(const uint32_t ci[4], const uint32_t ki[2], uint32_t out[4]) {
-  uint32_t c0 = ci[0], c1 = ci[1], c2 = ci[2], c3 = ci[3], k0 = ki[0], k1 = ki[1];
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    if (r > 0) { k0 += 0x9E3779B9u; k1 += 0xBB67AE85u; }
-    const uint32_t lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
-    const uint32_t lo1 = 0xCD9E8D57u * c2, hi1 = __umulhi(0xCD9E8D57u, c2);
-    const uint32_t n0 = hi1 ^ c1 ^ k0, n2 = hi0 ^ c3 ^ k1;
-    c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
-  }
-  out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
-}
 
 // Per-pixel random stream; the counter lives in a register and is written back by the owner.
 struct Rng {
@@ -309,26 +298,10 @@ __device__ __forceinline__ float2 floor_split2(float2 v, int *ix, int *iy) {
 #endif
 }
 
-// tex2D(x+0.5, y+0.5) with linear filtering and clamp-to-edge addressing, exact FP32 weights.
-// The padded border makes the four reads branch-free for x0 in [-1, W-1].
-__device__ __forceinline__ float bilinear(const float *__restrict__ img, int pad_w, int W, int H, float x, float y) {
-  const float xc = fminf(fmaxf(x, -1.0f), (float)(W - 1));
-  const float yc = fminf(fmaxf(y, -1.0f), (float)(H - 1));
-  int ix, iy;
-  const float fx = floor_split(xc, &ix), fy = floor_split(yc, &iy);
-  const float ax = xc - fx, ay = yc - fy;
-  const long long o = (long long)(iy + 1) * pad_w + (ix + 1);
-  const long long n = (long long)pad_w * (H + 2);
-  const float v00 = img_ld(img, o, n, 102), v10 = img_ld(img, o + 1, n, 103);
-  const float v01 = img_ld(img, o + pad_w, n, 104), v11 = img_ld(img, o + pad_w + 1, n, 105);
-  const float top = (1.0f - ax) * v00 + ax * v10;
-  const float bot = (1.0f - ax) * v01 + ax * v11;
-  return (1.0f - ay) * top + ay * bot;
-}
 // ------------------------------------------------------------------ source samplers
 // A source image as the cost kernels sample it.  fetch(o) returns the 2x2 texel footprint of
 // padded offset o, (P[o], P[o+1], P[o+pw], P[o+pw+1]), in FP32; the interpolation is shared, so
-// samplers differ only in storage.  FP32 samples equal bilinear() above exactly.
+// samplers differ only in storage.
 struct SrcF32 {
   static constexpr unsigned kBytes = 4;
   const float *p;
@@ -410,12 +383,11 @@ __device__ __forceinline__ Foot2 fetch2_biased(const Src &src, float2 fu, float2
   return fetch2(src, __float_as_uint(fv.x) * pitch + (__float_as_uint(fu.x) * Src::kBytes + base),
                 __float_as_uint(fv.y) * pitch + (__float_as_uint(fu.y) * Src::kBytes + base));
 }
-// kClamp = false: the caller knows -1 <= x <= W-1 and -1 <= y <= H-1, where the clamp is the
-// identity.
-template <class Src, bool kClamp = true>
+// tex2D(x+0.5, y+0.5) with linear filtering and clamp-to-edge addressing, exact FP32 weights.  The padded
+// border makes the reads branch-free for x0 in [-1, W-1].
+template <class Src>
 __device__ __forceinline__ float bilinear_s(const Src &src, int W, int H, float x, float y) {
-  const float2 c = kClamp ? make_float2(fminf(fmaxf(x, -1.0f), (float)(W - 1)), fminf(fmaxf(y, -1.0f), (float)(H - 1)))
-                          : make_float2(x, y);
+  const float2 c = make_float2(fminf(fmaxf(x, -1.0f), (float)(W - 1)), fminf(fmaxf(y, -1.0f), (float)(H - 1)));
   int ix, iy;
   const float2 f = floor_split2(c, &ix, &iy);
   const float2 a = sub2(c, f);                            // (ax, ay)
@@ -1133,7 +1105,7 @@ __device__ __forceinline__ float window_ncc_tab(const PMArgs &a, const float H[9
   const int side = 2 * radius / inc + 1;
   if (k > 0 && weak_is3(a) && !a.far) {
     const float4 *pairs = weak_pairs(a, tab, k);
-    float2 cX[3], rX[3], rY[3], rZ[3];  // column terms (H0 x, H3 x) and H6 x; row terms H1 y, H4 y, H7 y
+    float2 cX[3];  // column terms (H0 x, H3 x) and H6 x
     float cZ[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {

@@ -419,9 +419,10 @@ typedef struct dpe_options {
    * padded texel's 2x2 footprint as four 16-bit values, one load per bilinear sample; the
    * interpolation, the moments and the NCC stay FP32, as do the reference image and the
    * window weights.  Images of 8-bit integers are exact in both (the finest pyramid level);
-   * interpolated pyramid levels are rounded.  Default DPE_STAGE_FP32: sources sampled as FP32
-   * values, from BF16 footprints when every source texel of the call is exact in BF16 (checked on
-   * the device), which gives the same results with a quarter of the loads. */
+   * interpolated pyramid levels are rounded, except that FP16 holds the halved levels of even-sized
+   * 8-bit images (quarters below 256).  Default DPE_STAGE_FP32: sources sampled as FP32 values, from
+   * BF16 or FP16 footprints when every source texel of the call is exact in that format (checked on
+   * the device) and there is memory for them, which gives the same results with a quarter of the loads. */
   int staging;
   /* 1: every strong-update iteration adds one Gauss-Newton plane hypothesis, built from the
    * adjoint of the strong NCC (dpe_ncc_grad) over the pixel's sampled sources, and keeps it when
