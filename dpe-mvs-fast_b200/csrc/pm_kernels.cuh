@@ -360,10 +360,11 @@ __device__ __forceinline__ void sort_small(float *d, int n) {
 //   * the points' residuals of a round, and the ranks that replace its sorts.
 // Random numbers are made ahead into shared memory, each once; lines that start where no edge is near
 // are not walked (k_edge_clear_*).
-// Bound by instruction issue (0.55 of the slots; 34 k warp instructions per WEAK pixel, half of them the
-// residuals).  Measured, one 1600x1200 view with 403 k WEAK pixels: 126.7 ms one thread per pixel, 43.3
-// with 16 lanes, 29.1 with the numbers ahead and the walks skipped; 32 lanes 35.4, 8 lanes 46.8 (before
-// those two) against 43.1; one 400x300 view 2.0 -> 0.13 ms.
+// Bound by instruction issue (0.60 of the slots; about 45 k warp instructions per WEAK pixel, half of them
+// the residuals, with 15 of 32 threads active).  Measured, one 1600x1200 view with 403 k WEAK pixels: 126.7 ms one thread per pixel, 43.3
+// with 16 lanes, 29.1 with the numbers ahead and the walks skipped, 27.1 with points of 8 bytes; 32 lanes
+// 34.4, 8 lanes do not fit the shared memory (46.8 against 43.3 before the numbers were made ahead); one 400x300
+// view 2.0 -> 0.13 ms.
 // Host builds of this source run it with one lane.
 #ifdef __CUDA_ARCH__
 #ifndef DPE_GN_LANES
@@ -1434,7 +1435,7 @@ __device__ __forceinline__ void strong_probs(const CoopCtx &c, int iter) {
   if (!c.live) return;
   const PMArgs &a = *c.a;
   const int W = a.W, n = c.n, center = c.center;
-  const long long L = (long long)W * a.H;
+  [[maybe_unused]] const long long L = (long long)W * a.H;
   CoopPixel &P = *c.P;
   const uint32_t ctr0 = G(a.rng_ctr, center, L, 106);
 #ifdef __CUDA_ARCH__
