@@ -7,6 +7,7 @@ libdpe_sm100.so; loading fails loudly when it is missing -- there is no CPU fall
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
 from typing import Dict, List, Optional, Sequence
 
@@ -184,6 +185,13 @@ class DPEError(RuntimeError):
         detail = lib.dpe_last_error().decode() if status in (ERR_CUDA, ERR_OUT_OF_MEMORY) else ""
         super().__init__(f"{what}: {lib.dpe_status_string(status).decode()} (status {status}) {detail}".rstrip())
         self.status = status
+
+
+def level_size(n: int, scale_size: int) -> int:
+    """Columns or rows of a pyramid level, as the reference (SceneCache::GetGrayFloatImage) and the
+    library size it: C's round, halves away from zero (Python's and numpy's go to the even neighbour,
+    one less for every other odd size)."""
+    return math.floor(n / float(scale_size) + 0.5)
 
 
 def default_params(lib: Optional[C.CDLL] = None) -> Params:
@@ -462,8 +470,7 @@ class Context:
         int32 labels at the level size of `scale` (0 edges, -1 small regions), as numpy
         (memory=MEM_HOST) or as a CUDA tensor (MEM_DEVICE)."""
         H, W = gray.shape[:2]
-        f = np.float32(1.0) / np.float32(1 << scale)
-        w, h = int(np.round(np.float32(W) * f)), int(np.round(np.float32(H) * f))
+        w, h = level_size(W, 1 << scale), level_size(H, 1 << scale)
         if memory == MEM_HOST:
             img = np.ascontiguousarray(gray, dtype=np.uint8)
             out = np.zeros((h, w), np.int32)

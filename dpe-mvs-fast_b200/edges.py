@@ -14,6 +14,8 @@ import math
 
 import numpy as np
 
+from dpe_b200 import level_size
+
 try:
     import cv2
 except ImportError:  # pragma: no cover - cv2 ships with the image
@@ -173,8 +175,7 @@ def edge_segment(scale: int, src: np.ndarray, mode: int, use_canny: bool, high_r
     if mode == 0:
         dst = cv2.resize(dst, (cols, rows), interpolation=cv2.INTER_LINEAR)
     else:
-        f = 1.0 / float(1 << scale)
-        dst = cv2.resize(dst, (int(round(cols * f)), int(round(rows * f))), interpolation=cv2.INTER_LINEAR)
+        dst = cv2.resize(dst, (level_size(cols, 1 << scale), level_size(rows, 1 << scale)), interpolation=cv2.INTER_LINEAR)
     _, dst = cv2.threshold(dst, robthr, 255, cv2.THRESH_BINARY)
     dst = np.ascontiguousarray(dst)
     _border_fix(dst)
@@ -195,8 +196,7 @@ def level_inputs(gray_full: np.ndarray, scale_size: int, high_res_img: bool = Tr
     while (1 << scale) < scale_size:
         scale += 1
     rows, cols = gray_full.shape
-    f = 1.0 / float(scale_size)
-    new_cols, new_rows = int(round(cols * f)), int(round(rows * f))
+    new_cols, new_rows = level_size(cols, scale_size), level_size(rows, scale_size)
     scaled = cv2.resize(gray_full.astype(np.float32), (new_cols, new_rows), interpolation=cv2.INTER_LINEAR)
     scaled_u8 = np.clip(np.round(scaled), 0, 255).astype(np.uint8)  # convertTo(CV_8UC1)
     edge = edge_segment(scale, scaled_u8, 0, True, high_res_img)

@@ -194,8 +194,7 @@ def edge_labels(gray: np.ndarray, scale: int, high_res_img: bool = True) -> np.n
     map at the level size, 0 on edges and -1 on small regions."""
     gray = np.ascontiguousarray(gray, dtype=np.uint8)
     rows, cols = gray.shape
-    f = np.float32(1.0) / np.float32(1 << scale)
-    w, h = int(np.round(np.float32(cols) * f)), int(np.round(np.float32(rows) * f))
+    w, h = (int(np.floor(n * 0.5 ** scale + 0.5)) for n in (cols, rows))  # C's round
     out = np.zeros((h, w), np.int32)
     if load().oracle_edge_labels(gray.ctypes.data, cols, rows, scale, 1 if high_res_img else 0, out.ctypes.data,
                                  w, h) != 0:
